@@ -45,6 +45,13 @@ namespace px {
 #ifndef PX_FOLD_MINB
 #define PX_FOLD_MINB 3
 #endif
+// the apply pass takes four bricks per warp at a time where it has at least this many for every
+// warp.  Whole passes: the penthouse at 80 voxels per metre (40 bricks per warp) 587 us with
+// four, 700 us with one; at 20 (2 per warp) 712 us with four, 655 us with one; 4, 16 and 64
+// give the same on these, and at 40 (10 per warp, float64 form) 1.60, 1.56 and 1.56 ms
+#ifndef PX_FOLD_FOUR
+#define PX_FOLD_FOUR 16u
+#endif
 #ifndef PX_VSIMPLE_MINB
 #define PX_VSIMPLE_MINB 4
 #endif
@@ -1279,59 +1286,88 @@ __global__ void __launch_bounds__(256, PX_PAINT_MINB) paint_kernel(FoldArgs a) {
 // register j of the warp is the contiguous 128-byte slice pool[64 j .. 64 j + 63].
 // The warp applies its brick's ops in order, as apply() does (shapes.ts:367-412),
 // using the pair classifications.
-// One tile-list entry of a brick, looked up for the apply loop: the op, its
-// (op, brick) pair and that pair's classes, and the op fields the loop needs.
+// One tile-list entry of a brick, looked up for the apply loop: the op's (op, brick)
+// pair (build-local index, below 2^29), the pair's classes and the op fields the loop
+// needs in one word (FE_*), and the paint: the constant's value, or the pair's slot.
+enum : uint32_t { FE_PSC = 0xffffu, FE_CLS = 16, FE_KIND = 18, FE_CONST = 1u << 20, FE_SLOT = 1u << 21 };
 struct FoldEntry {
-  unsigned long long pr;
-  uint32_t oi, meta, pval, pslot, sc;
-  int cls;
+  uint32_t pr, w, val, oi;
 };
+__device__ __forceinline__ uint32_t fe_cls(uint32_t w) { return (w >> FE_CLS) & 3u; }
 
 __device__ __forceinline__ FoldEntry fold_entry(const FoldArgs& a, uint32_t idx, int bx, int by, int bz) {
-  FoldEntry f = {0ull, 0u, 0u, 0u, NO_SLOT, 0u, PC_SKIP};
+  FoldEntry f = {0u, PC_SKIP << FE_CLS, 0u, 0u};
   f.oi = __ldg(a.tile_ops + idx);
   const uint2 bb = __ldg(a.tile_boxes + idx);  // the op's brick box
   const int x0 = bb.x & 1023, y0 = (bb.x >> 10) & 1023, z0 = (bb.x >> 20) & 1023;
   const int x1 = bb.y & 1023, y1 = (bb.y >> 10) & 1023, z1 = (bb.y >> 20) & 1023;
   if (bx >= x0 && bx <= x1 && by >= y0 && by <= y1 && bz >= z0 && bz <= z1) {
     const OpDev* o = a.ops + f.oi;
-    f.pr = o->pair_base + (unsigned long long)(((bz - z0) * (y1 - y0 + 1) + (by - y0)) * (x1 - x0 + 1) + (bx - x0));
-    f.cls = __ldg(a.pcode + f.pr);
-    f.sc = __ldg(a.psub + f.pr);  // meaningful for partial pairs only
-    f.meta = (uint32_t)o->kind | ((uint32_t)o->flags << 8) | ((uint32_t)o->paint_kind << 16);
-    f.pval = o->paint_value;
-    f.pslot = o->paint_slot == NO_SLOT ? NO_SLOT : o->paint_slot + (uint32_t)(f.pr - o->pair_base);
+    const uint32_t local = (uint32_t)(((bz - z0) * (y1 - y0 + 1) + (by - y0)) * (x1 - x0 + 1) + (bx - x0));
+    f.pr = (uint32_t)o->pair_base + local;
+    const uint32_t cls = __ldg(a.pcode + f.pr), sc = __ldg(a.psub + f.pr);  // sc: meaningful for partial pairs only
+    const uint32_t slot = o->paint_slot;
+    f.w = sc | (cls << FE_CLS) | ((uint32_t)o->kind << FE_KIND) | (o->paint_kind == PK_CONST ? FE_CONST : 0u) |
+          (slot != NO_SLOT ? FE_SLOT : 0u);
+    f.val = slot != NO_SLOT ? slot + local : o->paint_value;
   }
   return f;
 }
 
+// The voxel masks of a partial pair's eight sub-blocks, copied to shared memory.
+__device__ __forceinline__ void fetch_masks(const FoldArgs& a, const FoldEntry& f, unsigned long long* dst) {
+  if (fe_cls(f.w) != PC_PARTIAL) return;
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  const unsigned long long* src = a.pmask + (size_t)f.pr * 8;
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d + 16 * k), "l"(src + 2 * k) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
 // INLINE: some painted op has no paint slot (paint values past the slot
 // budget), so paint calls happen here too; otherwise the apply loop calls nothing.
-// A warp takes four bricks at a time; lanes 8j..8j+7 look up the first eight
-// tile-list entries of brick j together (all four bricks' lookups in flight at
-// once), then the bricks are applied one after the other.
+//
+// A warp takes T bricks at a time; the 32 / T lanes of brick j look up the first
+// 32 / T entries of its tile list together (all lookups in flight at once), then the
+// bricks are applied one after the other.  Bound by latency: the ops of a brick
+// follow each other (its alloc / free events need each op's outcome), so a crowded
+// brick is a chain.  T is 4 where there are many bricks for every warp (short
+// lists, the lookups' dependent loads shared by four bricks), else 1: a list of
+// a hundred ops is then one warp's whole work instead of a quarter of it.  The
+// voxel masks of a partial pair and the values of the next painted pair are copied
+// to shared memory ahead of their use (loading both from global memory when the op
+// was applied cost a crowded brick about 1 us per op).  Measured, this against four
+// bricks everywhere and no fetching ahead: the penthouse at 20 voxels per metre
+// (lists up to 160 ops) 175 -> 74 us, at 80 (2 ops a brick) 129 -> 124 us, the
+// apply passes of twelve uneven scenes (100-180 ops a brick in three of them)
+// 1.79 -> 0.58 ms in all.
 template <bool INLINE>
 __global__ void __launch_bounds__(256, PX_FOLD_MINB) fold_kernel(FoldArgs a) {
   pdl_prologue();
-  __shared__ unsigned long long smask[8][8];
   __shared__ __align__(16) unsigned long long spm[8][32][8];  // voxel masks of the looked-up partial pairs
+  __shared__ __align__(16) uint32_t spv[8][BRICK_VOXELS];  // paint values of the next painted pair
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   const int lx0 = (lane & 3) * 2, ly = lane >> 2;
-  const uint32_t grp = (uint32_t)lane >> 3, ent = (uint32_t)lane & 7u;
+  // this lane's voxels in the sub-block masks: sub-blocks s0 (z < 4) and s0 + 4, bits e0 + 16 z and the next
+  const int s0 = (lx0 >> 2) | ((ly >> 2) << 1), e0 = (lx0 & 3) | ((ly & 3) << 2);
   WarpCounters wc = {0, 0, 0, 0, 0};
   uint32_t paint_calls = 0, paint_viol = 0;
   uint32_t st_local = 0;
   const uint32_t n_front = __ldg(a.work_counter + 1), n_work = n_front + __ldg(a.work_counter + 2);
+  const bool four = n_work >= PX_FOLD_FOUR * (gridDim.x * (blockDim.x >> 5));
+  const uint32_t T = four ? 4u : 1u, lsh = four ? 3u : 5u;  // 1 << lsh lanes per brick
+  const uint32_t grp = (uint32_t)lane >> lsh, ent = (uint32_t)lane & ((1u << lsh) - 1u);
 
   for (;;) {
     uint32_t wbase = 0;
-    if (lane == 0) wbase = atomicAdd(a.work_counter, 4u);
+    if (lane == 0) wbase = atomicAdd(a.work_counter, T);
     wbase = __shfl_sync(FULLMASK, wbase, 0);
     if (wbase >= n_work) break;
-    const uint32_t n_here = min(4u, n_work - wbase);
+    const uint32_t n_here = min(T, n_work - wbase);
     uint32_t q_pk = 0, q_g = 0, q_toff = 0, q_tcnt = 0;
-    FoldEntry q = {0ull, 0u, 0u, 0u, NO_SLOT, 0u, PC_SKIP};
+    FoldEntry q = {0u, PC_SKIP << FE_CLS, 0u, 0u};
     if (grp < n_here) {
       const uint32_t wi = wbase + grp;
       q_pk = __ldg(a.work + (wi < n_front ? wi : a.touched_cap - (wi - n_front)));
@@ -1342,27 +1378,19 @@ __global__ void __launch_bounds__(256, PX_FOLD_MINB) fold_kernel(FoldArgs a) {
       q_tcnt = __ldg(a.tile_cnt + tile);
       if (ent < q_tcnt) q = fold_entry(a, q_toff + ent, (int)bx, (int)by, (int)bz);
     }
-    if (q.cls == PC_PARTIAL) {  // its pair's voxel masks, copied to shared memory while the bricks load
-      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&spm[wib][lane][0]);
-      const unsigned long long* srcp = a.pmask + q.pr * 8;
-#pragma unroll
-      for (int k = 0; k < 4; k++)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 16 * k), "l"(srcp + 2 * k) : "memory");
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-    const uint32_t m_all = __ballot_sync(FULLMASK, q.cls != PC_SKIP);  // shapes.ts:364 skips the rest
+    fetch_masks(a, q, spm[wib][lane]);
+    const uint32_t m_all = __ballot_sync(FULLMASK, fe_cls(q.w) != PC_SKIP);  // shapes.ts:364 skips the rest
     uint32_t t_ci = 0, t_tag = 0;  // lane j: brick j's touched-list entry
     bool t_dirty = false;
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    cp_async_wait();
     __syncwarp();
 
     for (uint32_t j = 0; j < n_here; j++) {
-      const uint32_t pk = __shfl_sync(FULLMASK, q_pk, 8 * j);
-      const uint32_t g = __shfl_sync(FULLMASK, q_g, 8 * j);
-      const uint32_t toff = __shfl_sync(FULLMASK, q_toff, 8 * j), tcnt = __shfl_sync(FULLMASK, q_tcnt, 8 * j);
+      const uint32_t pk = __shfl_sync(FULLMASK, q_pk, j << lsh);
+      const uint32_t g = __shfl_sync(FULLMASK, q_g, j << lsh);
+      const uint32_t toff = __shfl_sync(FULLMASK, q_toff, j << lsh), tcnt = __shfl_sync(FULLMASK, q_tcnt, j << lsh);
       const int bx = (int)(pk & 1023u), by = (int)((pk >> 10) & 1023u), bz = (int)(pk >> 20);
       const uint32_t ci = (uint32_t)bx + (uint32_t)a.BX * ((uint32_t)by + (uint32_t)a.BY * (uint32_t)bz);
-      const int ox = bx * 8, oy = by * 8, oz = bz * 8;
 
       // current brick contents (VoxelWorld.ts:55-61)
       int state = ST_EMPTY;
@@ -1384,26 +1412,23 @@ __global__ void __launch_bounds__(256, PX_FOLD_MINB) fold_kernel(FoldArgs a) {
         for (int k = 0; k < 8; k++) vox[k] = pb[32 * k + lane];
       }
 
-      // apply the op whose entry lane `b` holds (`pm`: its voxel masks are in spm[wib][b])
+      // apply the op whose entry lane `b` holds (`pm`: its voxel masks are in spm[wib][b]);
+      // a painted pair's values are in spv[wib]
       auto apply = [&](const FoldEntry& f, int b, bool pm) {
-        const unsigned long long pair = __shfl_sync(FULLMASK, f.pr, b);
-        const int cls = __shfl_sync(FULLMASK, f.cls, b);
-        const uint32_t mt = __shfl_sync(FULLMASK, f.meta, b);
-        const uint32_t pv = __shfl_sync(FULLMASK, f.pval, b);
-        const uint32_t slot = __shfl_sync(FULLMASK, f.pslot, b);
-        const uint32_t o_idx = __shfl_sync(FULLMASK, f.oi, b);
-        const uint32_t psc = __shfl_sync(FULLMASK, f.sc, b);
-        const bool full = cls == PC_FULL;
-        const int kind = (int)(mt & 0xffu);
-        const uint32_t pk_ = mt >> 16;
-        const bool constPaint = pk_ == PK_CONST;
+        const uint32_t fw = __shfl_sync(FULLMASK, f.w, b);
+        const uint32_t fv = __shfl_sync(FULLMASK, f.val, b);
+        const uint32_t pair = __shfl_sync(FULLMASK, f.pr, b);
+        const uint32_t psc = fw & FE_PSC;
+        const bool full = fe_cls(fw) == PC_FULL;
+        const int kind = (int)((fw >> FE_KIND) & 3u);
+        const bool constPaint = fw & FE_CONST;
         // uniform shortcuts (shapes.ts:367-374)
         int set_u = -1;
         if (full) {
-          if (kind == KIND_ADD && constPaint) set_u = (int)pv;
+          if (kind == KIND_ADD && constPaint) set_u = (int)fv;
           else if (kind == KIND_CARVE) set_u = 0;
           else if (kind == KIND_PAINT && state == ST_EMPTY) return;
-          else if (kind == KIND_PAINT && constPaint && state == ST_UNIF) set_u = (int)pv;
+          else if (kind == KIND_PAINT && constPaint && state == ST_UNIF) set_u = (int)fv;
         }
         if (set_u >= 0) {  // setBrickUniform (VoxelWorld.ts:89-97)
           if (state == ST_MIXED) {
@@ -1420,86 +1445,79 @@ __global__ void __launch_bounds__(256, PX_FOLD_MINB) fold_kernel(FoldArgs a) {
         }
         if (kind == KIND_PAINT && state == ST_EMPTY) return;
 
-        // sub-block and voxel classes (shapes.ts:382-394), computed by classify_kernel
+        // the covered voxels of this lane (shapes.ts:382-394): bit 2 k + h of lb is voxel
+        // (x0 + h, y, k), from the sub-block classes and the partial ones' masks
+        uint32_t lb = 0xffffu;
         if (!full) {
-          if (lane < 8) {
-            const uint32_t c = (psc >> (2 * lane)) & 3u;
-            smask[wib][lane] = c == PC_FULL      ? ~0ull
-                               : c != PC_PARTIAL ? 0ull
-                               : pm              ? spm[wib][b][lane]
-                                                 : __ldg(a.pmask + pair * 8 + lane);
+          const uint32_t c0 = (psc >> (2 * s0)) & 3u, c1 = (psc >> (2 * s0 + 8)) & 3u;
+          auto mask = [&](uint32_t c, int s) -> unsigned long long {
+            return c == PC_FULL ? ~0ull : c != PC_PARTIAL ? 0ull : pm ? spm[wib][b][s] : __ldg(a.pmask + (size_t)pair * 8 + s);
+          };
+          const unsigned long long m0 = mask(c0, s0), m1 = mask(c1, s0 + 4);
+          lb = 0;
+#pragma unroll
+          for (int jj = 0; jj < 4; jj++) {
+            lb |= (uint32_t)((m0 >> (e0 + 16 * jj)) & 3ull) << (2 * jj);
+            lb |= (uint32_t)((m1 >> (e0 + 16 * jj)) & 3ull) << (2 * jj + 8);
           }
           wc.sub += 8;
           wc.vox += 64 * __popc(psc & ~(psc >> 1) & 0x5555u);  // sub-blocks of class PC_PARTIAL (01)
-        } else if (lane < 8) {
-          smask[wib][lane] = ~0ull;
         }
-        __syncwarp();
 
-        // write voxels (shapes.ts:395-405)
+        // write voxels (shapes.ts:395-405), whole voxel pairs at a time: a value for every
+        // covered voxel (carve: air; a const paint; a painted pair's values), all u16, so
+        // the stored value equals the compared one
         bool changed = false;
+        auto covered = [&](int k) -> uint32_t {  // the voxels of pair k the op writes, a half word each
+          const uint32_t two = (lb >> (2 * k)) & 3u;
+          uint32_t keep = ((two & 1u) ? 0xffffu : 0u) | ((two & 2u) ? 0xffff0000u : 0u);
+          if (kind == KIND_PAINT)  // Paint recolours non-air voxels only
+            keep &= ((vox[k] & 0xffffu) ? 0xffffu : 0u) | ((vox[k] & 0xffff0000u) ? 0xffff0000u : 0u);
+          return keep;
+        };
+        auto store = [&](int k, uint32_t keep, uint32_t val) {
+          const uint32_t nv = (vox[k] & ~keep) | (val & keep);
+          changed = changed || nv != vox[k];
+          vox[k] = nv;
+        };
         if (constPaint || kind == KIND_CARVE) {
-          // one value for every covered voxel (carve: air; a const paint is a u16, so the
-          // unstored value equals the stored one): whole voxel pairs at a time.  Bit 2j + h
-          // of lb is voxel (x0 + h, y, j) of this lane.
-          const int base = (lx0 & 3) | ((ly & 3) << 2);
-          const int s0 = (lx0 >> 2) | ((ly >> 2) << 1);
-          const unsigned long long m0 = smask[wib][s0], m1 = smask[wib][s0 + 4];
-          uint32_t lb = 0;
-#pragma unroll
-          for (int jj = 0; jj < 4; jj++) {
-            lb |= (uint32_t)((m0 >> (base + 16 * jj)) & 3ull) << (2 * jj);
-            lb |= (uint32_t)((m1 >> (base + 16 * jj)) & 3ull) << (2 * jj + 8);
-          }
-          const uint32_t v = kind == KIND_CARVE ? 0u : pv;
+          const uint32_t v = kind == KIND_CARVE ? 0u : fv;
           const uint32_t vv = v | (v << 16);
 #pragma unroll
-          for (int k = 0; k < 8; k++) {
-            const uint32_t two = (lb >> (2 * k)) & 3u;
-            uint32_t keep = ((two & 1u) ? 0xffffu : 0u) | ((two & 2u) ? 0xffff0000u : 0u);
-            if (kind == KIND_PAINT)  // Paint recolours non-air voxels only
-              keep &= ((vox[k] & 0xffffu) ? 0xffffu : 0u) | ((vox[k] & 0xffff0000u) ? 0xffff0000u : 0u);
-            const uint32_t nv = (vox[k] & ~keep) | (vv & keep);
-            changed = changed || nv != vox[k];
-            vox[k] = nv;
-          }
-        } else {
+          for (int k = 0; k < 8; k++) store(k, covered(k), vv);
+        } else if (fw & FE_SLOT) {  // evaluated by paint_kernel
 #pragma unroll
           for (int k = 0; k < 8; k++) {
-            const int s = (lx0 >> 2) | ((ly >> 2) << 1) | ((k >> 2) << 2);
-            const int e0 = (lx0 & 3) | ((ly & 3) << 2) | ((k & 3) << 4);
-            const unsigned long long ms = smask[wib][s];
+            const uint32_t keep = covered(k);
+            const uint2 pv = *reinterpret_cast<const uint2*>(&spv[wib][64 * k + 2 * lane]);
+            if (((pv.x & PV_RANGE) && (keep & 0xffffu)) || ((pv.y & PV_RANGE) && (keep >> 16))) st_local |= ST_RANGE;
+            paint_calls += (keep & 1u) + (keep >> 31);
+            store(k, keep, (pv.x & 0xffffu) | (pv.y << 16));
+          }
+        } else if constexpr (INLINE) {  // a painted op without a slot: its paint calls here
+          const OpDev* O = a.ops + __shfl_sync(FULLMASK, f.oi, b);
+#pragma unroll
+          for (int k = 0; k < 8; k++) {
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-              if (!((ms >> (e0 + h)) & 1ull)) continue;
+              if (!((lb >> (2 * k + h)) & 1u)) continue;
               const uint32_t cur = (vox[k] >> (16 * h)) & 0xffffu;
-              uint32_t next;
               if (kind == KIND_PAINT && cur == 0) continue;
-              else if (slot != NO_SLOT) {  // evaluated by paint_kernel
-                const uint32_t pvv = __ldg(a.pvals + (size_t)slot * 512 + (uint32_t)((lx0 + h) | (ly << 3) | (k << 6)));
-                if (pvv & PV_RANGE) st_local |= ST_RANGE;
-                next = pvv & 0xffffu;
-                paint_calls++;
-              } else {
-                if constexpr (INLINE) {
-                  const uint32_t pv2 = paint_at_voxel(a.params, a.vs, a.validate, a.ops + o_idx, ox + lx0 + h, oy + ly, oz + k);
-                  if (pv2 & PV_RANGE) st_local |= ST_RANGE;
-                  if (pv2 & PV_VIOL) paint_viol++;
-                  next = pv2 & 0xffffu;
-                  paint_calls++;
-                } else {  // every painted op has a slot in this build
-                  st_local |= ST_CHAIN;
-                  next = cur;
-                }
-              }
-              if (next != cur) {  // Uint16Array store; the comparison uses the unstored value
-                vox[k] = (vox[k] & ~(0xffffu << (16 * h))) | ((next & 0xffffu) << (16 * h));
+              const uint32_t pv2 = paint_at_voxel(a.params, a.vs, a.validate, O, bx * 8 + lx0 + h, by * 8 + ly, bz * 8 + k);
+              if (pv2 & PV_RANGE) st_local |= ST_RANGE;
+              if (pv2 & PV_VIOL) paint_viol++;
+              const uint32_t next = pv2 & 0xffffu;
+              paint_calls++;
+              if (next != cur) {
+                vox[k] = (vox[k] & ~(0xffffu << (16 * h))) | (next << (16 * h));
                 changed = true;
               }
             }
           }
+          __syncwarp();
+        } else {  // every painted op has a slot in this build
+          st_local |= ST_CHAIN;
         }
-        __syncwarp();
         if (!__any_sync(FULLMASK, changed)) return;
         dirty = true;
         uint8_t ev = 0;
@@ -1507,12 +1525,11 @@ __global__ void __launch_bounds__(256, PX_FOLD_MINB) fold_kernel(FoldArgs a) {
           ev = 1; src = (long long)pair; state = ST_MIXED;
           wc.alloc++;
         }
-        // compactCell (VoxelWorld.ts:147-156)
-        const uint32_t v0 = __shfl_sync(FULLMASK, vox[0] & 0xffffu, 0);
-        const uint32_t vv = v0 | (v0 << 16);
+        // compactCell (VoxelWorld.ts:147-156): are all voxels equal?
+        const uint32_t v0 = __shfl_sync(FULLMASK, vox[0] & 0xffffu, 0), vv0 = v0 | (v0 << 16);
         bool eq = true;
 #pragma unroll
-        for (int k = 0; k < 8; k++) eq = eq && vox[k] == vv;
+        for (int k = 0; k < 8; k++) eq = eq && vox[k] == vv0;
         if (__all_sync(FULLMASK, eq)) {
           if (lane == 0) a.fsrc[pair] = src;
           ev |= 2;
@@ -1523,13 +1540,50 @@ __global__ void __launch_bounds__(256, PX_FOLD_MINB) fold_kernel(FoldArgs a) {
         if (lane == 0) a.evt[pair] = ev;
       };
 
-      // entries 0..7 of the tile list, looked up above by lanes 8j..8j+7
-      for (uint32_t m = (m_all >> (8 * j)) & 0xffu; m; m &= m - 1) apply(q, (int)(8 * j) + __ffs(m) - 1, true);
+      // apply the entries `m` (lane bits) of f in order; the next painted pair's values are
+      // on their way while the entries before it are applied
+      auto apply_all = [&](const FoldEntry& f, uint32_t m, bool pm) {
+        uint32_t painted = m & __ballot_sync(FULLMASK, (f.w & FE_SLOT) != 0u);
+        auto fetch_paint = [&]() {
+          const uint32_t slot = __shfl_sync(FULLMASK, f.val, __ffs(painted) - 1);
+          const uint32_t d = (uint32_t)__cvta_generic_to_shared(&spv[wib][4 * lane]);
+          const uint32_t* sv = a.pvals + (size_t)slot * BRICK_VOXELS + 4 * lane;
+#pragma unroll
+          for (int k = 0; k < 4; k++)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d + 512 * k), "l"(sv + 128 * k) : "memory");
+        };
+        if (painted) fetch_paint();
+        for (; m; m &= m - 1) {
+          const int b = __ffs(m) - 1;
+          const bool now = painted & (m & (0u - m));
+          if (now) {
+            cp_async_wait();
+            __syncwarp();
+          }
+          apply(f, b, pm);
+          if (now) {
+            painted &= painted - 1;
+            __syncwarp();  // every lane has read its values
+            if (painted) fetch_paint();
+          }
+        }
+      };
+
+      // the first entries of the tile list, looked up above by this brick's lanes
+      apply_all(q, m_all & ((four ? 0xffu : 0xffffffffu) << (j << lsh)), true);
       // the rest of a longer list, 32 entries per pass
-      for (uint32_t c0 = 8; c0 < tcnt; c0 += 32) {
-        FoldEntry f = {0ull, 0u, 0u, 0u, NO_SLOT, 0u, PC_SKIP};
+      for (uint32_t c0 = 1u << lsh; c0 < tcnt; c0 += 32) {
+        FoldEntry f = {0u, PC_SKIP << FE_CLS, 0u, 0u};
         if (c0 + lane < tcnt) f = fold_entry(a, toff + c0 + lane, bx, by, bz);
-        for (uint32_t m = __ballot_sync(FULLMASK, f.cls != PC_SKIP); m; m &= m - 1) apply(f, __ffs(m) - 1, false);
+        const uint32_t m = __ballot_sync(FULLMASK, fe_cls(f.w) != PC_SKIP);
+        if (!m) continue;
+        if (!four) {  // one brick: its first entries' masks have been read
+          __syncwarp();
+          fetch_masks(a, f, spm[wib][lane]);
+          cp_async_wait();
+          __syncwarp();
+        }
+        apply_all(f, m, !four);
       }
 
       if (!dirty) continue;
@@ -1568,6 +1622,7 @@ __global__ void __launch_bounds__(256, PX_FOLD_MINB) fold_kernel(FoldArgs a) {
         else st_local |= ST_STAGE_OVERFLOW;
       }
     }
+    __syncwarp();  // the shared masks and values have been read
   }
   if (lane == 0) {
     if (wc.sub) atomicAdd(&a.res->c.sub_evals, (unsigned long long)wc.sub);
