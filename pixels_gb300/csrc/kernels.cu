@@ -22,6 +22,7 @@
 #include "px_internal.cuh"
 #include "sdf64.cuh"
 #include "sdf32.cuh"
+#include "sdf32p.cuh"
 #include "paint.cuh"
 #include "paint32.cuh"
 
@@ -44,6 +45,15 @@ namespace px {
 #endif
 #ifndef PX_FOLD_MINB
 #define PX_FOLD_MINB 3
+#endif
+// items per ticket of the lean voxel kernels, at most, and tickets per warp, at least.  Sum of
+// these kernels, penthouse at 80 / 256 edits at 160 / synthetic: 1 item 165 / 182 / 620 us,
+// 4 items 92 / 73 / 284, 8 items 98 / 72 / 289, 16 items (2 tickets) 106 / 74 / 317
+#ifndef PX_VOXEL_TICKET
+#define PX_VOXEL_TICKET 4u
+#endif
+#ifndef PX_VOXEL_TICKETS
+#define PX_VOXEL_TICKETS 4u
 #endif
 // the apply pass takes four bricks per warp at a time where it has at least this many for every
 // warp.  Whole passes: the penthouse at 80 voxels per metre (40 bricks per warp) 587 us with
@@ -477,58 +487,19 @@ __device__ __forceinline__ void brick_bases(const FoldArgs& a, const OpDev* O, i
   bo[2] = {b2.x, b2.y};
 }
 
-// The point through a rotation of the shape's frame (shapes.ts:263-320 on
-// intervals, in the centre-radius form of lin2): p holds the pivot's two
-// coordinates, cos and sin.
-__device__ __forceinline__ void rot32(uint32_t op, const Iv* __restrict__ p, Iv& x, Iv& y, Iv& z) {
-  const Iv p0 = ldp(p, 0), p1 = ldp(p, 1), c = ldp(p, 2), sn = ldp(p, 3), nsn = ineg(sn);
-  if (op == OP_ROT_Y) {
-    const Iv dx = isub(x, p0), dz = isub(z, p1);
-    x = lin2(p0, c, dx, sn, dz);
-    z = lin2(p1, nsn, dx, c, dz);
-  } else if (op == OP_ROT_X) {
-    const Iv dy = isub(y, p0), dz = isub(z, p1);
-    y = lin2(p0, c, dy, sn, dz);
-    z = lin2(p1, nsn, dy, c, dz);
-  } else {
-    const Iv dx = isub(x, p0), dy = isub(y, p1);
-    x = lin2(p0, c, dx, sn, dy);
-    y = lin2(p1, nsn, dx, c, dy);
-  }
+// The same offsets' lower ends, and a voxel's coordinate from one: the float32 points
+// of the lean programs.
+__device__ __forceinline__ void brick_bases_f(const FoldArgs& a, const OpDev* O, int bx, int by, int bz, float* bo) {
+  const float2* bt = a.bases + O->base_off;
+  bo[0] = __ldg(&bt[bx - O->bx0].x);
+  bo[1] = __ldg(&bt[O->nx + (by - O->by0)].x);
+  bo[2] = __ldg(&bt[O->nx + O->ny + (bz - O->bz0)].x);
 }
+__device__ __forceinline__ float coord_f(float base, float k, float vs_lo) { return base + k * vs_lo; }
 
-// Apply a lean program's stage (LP_* kinds): one rotation, or (AFF) a composed run.
-template <bool AFF>
-__device__ __forceinline__ void stage32(uint32_t kind, const Iv* __restrict__ p, Iv& x, Iv& y, Iv& z) {
-  if (AFF && kind == LP_AFFINE) aff32(p, x, y, z);
-  else if (kind) rot32(OP_ROT_X - 1 + kind, p, x, y, z);
-}
-
-// A lean program (LP_* forms) at one point in float32 intervals, without the
-// interpreter's value stack and rotation frames; amb: a polygon crossing test
-// the intervals could not settle.  One copy of the primitive and stage code
-// serves both primitives of forms 2 and 3.
-__device__ __forceinline__ Iv lean_point(const FoldArgs& a, const OpDev* V, Iv x, Iv y, Iv z, float M, bool& amb) {
-  const Iv* __restrict__ P = reinterpret_cast<const Iv*>(a.p32);
-  const uint32_t l0 = *reinterpret_cast<const uint32_t*>(V->lp), l1 = *reinterpret_cast<const uint32_t*>(V->lp + 4);
-  const uint32_t form = l0 & 0xffu, comb = (l0 >> 8) & 0xffu, ioff = l1 >> 24, kinds = (l1 >> 16) & 0xffu;
-  const uint32_t* c32 = a.code32 + V->code_off;
-  const uint2* cw = a.code + V->code_off;
-  Iv v = {0.f, 0.f}, xs = x, ys = y, zs = z;
-#pragma unroll 1
-  for (uint32_t k = 0; k < (form > 1 ? 2u : 1u); k++) {
-    const uint32_t ip = k ? l0 >> 24 : (l0 >> 16) & 0xffu;
-    if (k == 0 || form == 3) {  // the stage: instruction 0, or the second primitive's own
-      xs = x; ys = y; zs = z;
-      const uint32_t ks = k ? kinds >> 4 : kinds & 15u, is = k ? (l1 >> 8) & 0xffu : 0u;
-      if (ks) stage32<true>(ks, P + (__ldg(c32 + is) & C32_OFF), xs, ys, zs);
-    }
-    const uint32_t w = __ldg(&cw[ip].x);
-    const Iv u = prim32(w & 0xffu, (int)(w >> 8), P + (__ldg(c32 + ip) & C32_OFF), xs, ys, zs, M, amb);
-    v = k == 0 ? u : comb == LP_NEGMAX ? imax(v, ineg(u)) : comb == LP_MAX ? imax(v, u) : imin(v, u);
-  }
-  if (ioff != LP_NONE) v = iadd(v, ldp(P + (__ldg(c32 + ioff) & C32_OFF), 0));  // offset (penthouse.ts:250)
-  return v;
+// The (op, brick) pair of op O at brick (bx, by, bz).
+__device__ __forceinline__ uint32_t pair_of_brick(const OpDev* O, int bx, int by, int bz) {
+  return (uint32_t)O->pair_base + (uint32_t)(((bz - O->bz0) * O->ny + (by - O->by0)) * O->nx + (bx - O->bx0));
 }
 
 // The rest of the brick pass for one pair per lane (`valid`), its class cls
@@ -660,18 +631,20 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_CLASSIFY_MINB : PX_CLASSIF
         cls = PC_FULL;
       } else {
         const bool use32 = MODE == 1 && !(flags & OPF_FP64_ONLY);
-        Iv bo[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-        if (use32) brick_bases(a, O, bx, by, bz, bo);
         cls = 3;
-        if (MODE == 1 && use32 && O->lp[LP_FORM] && !a.validate) {  // a lean program: no interpreter
-          bool amb = false;
-          const Iv k = koff(3.5f, a.vs_lo, a.vs_hi);
-          const Iv d = lean_point(a, O, iadd(bo[0], k), iadd(bo[1], k), iadd(bo[2], k), O->thr[T_M], amb);
-          if (!amb) cls = classify32(d, O->thr, T_BSK_HI);
+        if (MODE == 1 && use32 && O->lw[0] && !a.validate) {  // a lean program: no interpreter
+          float b[3], lo[1], hi[1];
+          brick_bases_f(a, O, bx, by, bz, b);
+          const float z[1] = {coord_f(b[2], 3.5f, a.vs_lo)};
+          lean_f<1, 3, true, true>(a, O, coord_f(b[0], 3.5f, a.vs_lo), coord_f(b[1], 3.5f, a.vs_lo), z, lo, hi);
+          cls = classify32({lo[0], hi[0]}, O->thr, T_BSK_HI);
         }
-        if (cls == 3)  // the interpreter, with the float64 rescue
+        if (cls == 3) {  // the interpreter, with the float64 rescue
+          Iv bo[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+          if (use32) brick_bases(a, O, bx, by, bz, bo);
           cls = eval_decide<MODE>(a, O, a.code + O->code_off, (int)O->code_len, use32, bo, 3.5f, 3.5f, 3.5f,
                                   (float)(bx * 8 + 4), (float)(by * 8 + 4), (float)(bz * 8 + 4), 1, ls);
+        }
         n_brick++;
       }
     }
@@ -744,7 +717,8 @@ __device__ __forceinline__ void sub_finish(const FoldArgs& a, bool have, uint32_
     const uint32_t slot = vb + __popc(grp & ((1u << lane) - 1u));
     if (slot < a.vq_cap[k])
       a.vitems[a.vq_base[k] + slot] =
-          make_uint4(oo, (uint32_t)(pp << 3) | (uint32_t)s, __float_as_uint(dc.lo), __float_as_uint(dc.hi));
+          make_uint4(oo | ((uint32_t)s << 24), (uint32_t)pbx | ((uint32_t)pby << 10) | ((uint32_t)pbz << 20),
+                     __float_as_uint(dc.lo), __float_as_uint(dc.hi));
     else st_local |= ST_STAGE_OVERFLOW;
   }
 }
@@ -799,22 +773,25 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_SUB_MINB : PX_CLASSIFY64_M
       brick_of_pair(Q, pp, pbx, pby, pbz);
       boxr = (Q->flags & OPF_BOX_RANGES) && !a.validate;
       const bool use32 = MODE == 1 && !(Q->flags & OPF_FP64_ONLY);
-      Iv bo[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-      if (use32) brick_bases(a, Q, pbx, pby, pbz, bo);
       const int sxb = s & 1, syb = (s >> 1) & 1, szb = (s >> 2) & 1;
       scls = 3;
-      if (MODE == 1 && use32 && Q->lp[LP_FORM] && !a.validate) {  // a lean program: no interpreter
-        bool amb = false;
-        dc = lean_point(a, Q, iadd(bo[0], koff(4.f * sxb + 1.5f, a.vs_lo, a.vs_hi)),
-                        iadd(bo[1], koff(4.f * syb + 1.5f, a.vs_lo, a.vs_hi)),
-                        iadd(bo[2], koff(4.f * szb + 1.5f, a.vs_lo, a.vs_hi)), Q->thr[T_M], amb);
-        if (!amb) scls = classify32(dc, Q->thr, T_SSK_HI);
+      if (MODE == 1 && use32 && Q->lw[0] && !a.validate) {  // a lean program: no interpreter
+        float b[3], lo[1], hi[1];
+        brick_bases_f(a, Q, pbx, pby, pbz, b);
+        const float z[1] = {coord_f(b[2], 4.f * szb + 1.5f, a.vs_lo)};
+        lean_f<1, 3, true, true>(a, Q, coord_f(b[0], 4.f * sxb + 1.5f, a.vs_lo), coord_f(b[1], 4.f * syb + 1.5f, a.vs_lo),
+                                 z, lo, hi);
+        dc = {lo[0], hi[0]};
+        scls = classify32(dc, Q->thr, T_SSK_HI);
       }
-      if (scls == 3)  // the interpreter, with the float64 rescue
+      if (scls == 3) {  // the interpreter, with the float64 rescue
+        Iv bo[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+        if (use32) brick_bases(a, Q, pbx, pby, pbz, bo);
         scls = eval_decide<MODE>(a, Q, a.code + Q->code_off, (int)Q->code_len, use32, bo, 4.f * sxb + 1.5f,
                                  4.f * syb + 1.5f, 4.f * szb + 1.5f, (float)(pbx * 8 + sxb * 4 + 2),
                                  (float)(pby * 8 + syb * 4 + 2), (float)(pbz * 8 + szb * 4 + 2), 2, ls, true,
                                  MODE == 1 && use32 ? &dc : nullptr);
+      }
     }
     uint32_t code16 = (uint32_t)scls << (2 * s);
     code16 |= __shfl_xor_sync(FULLMASK, code16, 1);
@@ -872,11 +849,10 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_VOXEL_MINB : PX_CLASSIFY64
     const uint32_t first = __shfl_sync(FULLMASK, incl - own, k);
     const uint4 item = __ldg(a.vitems + a.vq_base[a.vclass_order[32 * g + k]] + (it - first));
     const Iv dcen = {__uint_as_float(item.z), __uint_as_float(item.w)};  // the sub-block centre's value
-    const OpDev* V = a.ops + item.x;
-    const unsigned long long vp = item.y >> 3;
-    const int ss = item.y & 7;
-    int vbx, vby, vbz;
-    brick_of_pair(V, vp, vbx, vby, vbz);
+    const OpDev* V = a.ops + (item.x & 0xffffffu);
+    const int ss = (int)(item.x >> 24);
+    const int vbx = (int)(item.y & 1023u), vby = (int)((item.y >> 10) & 1023u), vbz = (int)(item.y >> 20);
+    const unsigned long long vp = pair_of_brick(V, vbx, vby, vbz);
     const bool use32 = MODE == 1 && !(V->flags & OPF_FP64_ONLY);
     Iv bo[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
     if (use32) brick_bases(a, V, vbx, vby, vbz, bo);
@@ -950,25 +926,24 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_VOXEL_MINB : PX_CLASSIFY64
 // one or two primitives under a rotation, a composed run of rotations or none
 // (LP_* forms): 88% of the penthouse's non-box voxel work, all of the
 // rotated synthetic scenes' -- in the mixed form: the same decisions as
-// voxel_kernel (shapes.ts:390-394), without the interpreters' value stack and
-// rotation frames.  Lane = voxel column (x, z) of the sub-block and a pair of
-// y rows; unrotated primitives extruded along y (or rotated about y) share
-// their x/z work between the two voxels.
+// voxel_kernel (shapes.ts:390-394) from float32 points and the op's error bound
+// (sdf32p.cuh).  A warp takes one sub-block; lane = x | y << 2 | (z & 1) << 4 evaluates
+// voxels z and z + 2, so that two ballots are the mask.
 // VALIDATE (validation mode) evaluates every voxel in float64 too, in line.
-// Otherwise a voxel the interval cannot decide goes to the rescue list, which
-// voxel_kernel<1, ...> resolves in float64 first, and counts as outside until
-// then (no call in this kernel: every value live across one would be saved to
-// local memory).
+// Otherwise a voxel nearer to the surface than the bound goes to the rescue list,
+// which paint_kernel<1> resolves in float64 first, and counts as outside until then
+// (no call in this kernel: every value live across one would be saved to local
+// memory).
 // G: the group of the voxel queue (VQ_NARROW, VQ_AFFINE or VQ_WIDE), each
 // compiled with only its forms' live values.
 template <bool VALIDATE, int G>
 __global__ void __launch_bounds__(256, G == VQ_WIDE ? PX_VWIDE_MINB : G == VQ_AFFINE ? PX_VAFF_MINB : PX_VSIMPLE_MINB)
     voxel_lean_kernel(FoldArgs a) {
-  constexpr bool WIDE = G == VQ_WIDE, AFF = G != VQ_NARROW;
   pdl_prologue();
   const int lane = threadIdx.x & 31;
   LaneStats ls = {a.res};
   uint32_t* const taken = &a.vitem_counter[VQ_TAKEN + G];
+  // the group's classes' item counts in the order they are taken, as an inclusive prefix over lanes
   const int my_cls = a.vclass_order[32 * G + lane];
   uint32_t incl = min(__ldg(&a.vitem_counter[1 + my_cls]), a.vq_cap[my_cls]);
   const uint32_t own = incl;
@@ -978,156 +953,108 @@ __global__ void __launch_bounds__(256, G == VQ_WIDE ? PX_VWIDE_MINB : G == VQ_AF
     if (lane >= o) incl += t;
   }
   const uint32_t n_items = __shfl_sync(FULLMASK, incl, 31);
-  const int col = lane & 15, yh = lane >> 4;
-  const Iv* __restrict__ P = reinterpret_cast<const Iv*>(a.p32);
+  const uint32_t at0 = a.vq_base[my_cls] - (incl - own);  // queue position of item `it` of this class: at0 + it
+  const int lx = lane & 3, lyv = (lane >> 2) & 3, lz = lane >> 4;  // and lz + 2
+  // distance classes of the two voxels (OpDev::lip: axes at 1.5 voxels from the centre)
+  const int kxy = (lx == 0 || lx == 3) + (lyv == 0 || lyv == 3);
+  const int kc[2] = {kxy + (lz == 0), kxy + (lz == 1)};
+  // items per ticket: one counter serves the whole grid, and with a ticket per item its
+  // atomics, some 0.65 ns each, were the kernel's bound (1.5 items per ns whatever the
+  // shapes); few where the items are few, so that the warps end together
+  const uint32_t B = max(1u, min(PX_VOXEL_TICKET, n_items / (PX_VOXEL_TICKETS * gridDim.x * (blockDim.x >> 5))));
   NextTicket tk;
-  tk.issue(taken, 1, lane);
+  tk.issue(taken, B, lane);
   for (;;) {
-    const uint32_t it = tk.get();
-    if (it >= n_items) break;
-    tk.issue(taken, 1, lane);
-    const int k = __popc(__ballot_sync(FULLMASK, incl <= it));  // class of item `it`
-    const uint32_t first = __shfl_sync(FULLMASK, incl - own, k);
-    const uint4 item = __ldg(a.vitems + a.vq_base[a.vclass_order[32 * G + k]] + (it - first));
-    const Iv dcen = {__uint_as_float(item.z), __uint_as_float(item.w)};  // the sub-block centre's value
-    const OpDev* V = a.ops + item.x;
-    const unsigned long long vp = item.y >> 3;
-    const int ss = item.y & 7;
-    int vbx, vby, vbz;
-    brick_of_pair(V, vp, vbx, vby, vbz);
-    Iv bo[3];
-    brick_bases(a, V, vbx, vby, vbz, bo);
-    const int sxo = (ss & 1) * 4, syo = ((ss >> 1) & 1) * 4, szo = ((ss >> 2) & 1) * 4;
-    const int lx = sxo + (col & 3), lz = szo + (col >> 2), ly0 = syo + 2 * yh;
-    const int lip0 = lip_decide(V, dcen, col & 3, 2 * yh, col >> 2), lip1 = lip_decide(V, dcen, col & 3, 2 * yh + 1, col >> 2);
-    const float M = V->thr[T_M];
-    bool amb0 = false, amb1 = false;  // a polygon crossing test the interval could not settle, per voxel
-    Iv2 d = {{0.f, 0.f}, {0.f, 0.f}};
-    if (lip0 == 3 || lip1 == 3 || VALIDATE) {
-      const uint2 lpw = make_uint2(*reinterpret_cast<const uint32_t*>(V->lp), *reinterpret_cast<const uint32_t*>(V->lp + 4));
-      const uint32_t form = WIDE ? lpw.x & 0xffu : 1u, comb = (lpw.x >> 8) & 0xffu, ip1 = (lpw.x >> 16) & 0xffu,
-                     ip2 = lpw.x >> 24, is2 = (lpw.y >> 8) & 0xffu, kinds = (lpw.y >> 16) & 0xffu,
-                     ioff = lpw.y >> 24;
-      const uint32_t k1 = kinds & 15u, k2 = WIDE ? kinds >> 4 : 0u;
-      const uint32_t* c32 = a.code32 + V->code_off;
-      const uint2* cw = a.code + V->code_off;
-      const uint32_t w1 = __ldg(&cw[ip1].x), w2 = form > 1 ? __ldg(&cw[ip2].x) : 0u;
-      const uint32_t p1 = w1 & 0xffu, p2 = w2 & 0xffu;
-      const Iv* pr1 = P + (__ldg(c32 + ip1) & C32_OFF);
-      const Iv* pr2 = P + (__ldg(c32 + (form > 1 ? ip2 : ip1)) & C32_OFF);
-      const Iv* ps1 = P + (__ldg(c32) & C32_OFF);  // the first stage is instruction 0
-      const Iv* ps2 = P + (__ldg(c32 + (k2 ? is2 : 0u)) & C32_OFF);
-      const Iv x = iadd(bo[0], koff((float)lx, a.vs_lo, a.vs_hi)), z = iadd(bo[2], koff((float)lz, a.vs_lo, a.vs_hi));
-      const Iv y0 = iadd(bo[1], koff((float)ly0, a.vs_lo, a.vs_hi)), y1 = iadd(bo[1], koff((float)(ly0 + 1), a.vs_lo, a.vs_hi));
-      auto combine = [&](Iv u, Iv v) -> Iv {
-        return comb == LP_NEGMAX ? imax(u, ineg(v)) : comb == LP_MAX ? imax(u, v) : imin(u, v);
-      };
-      // y-extruded primitives, unrotated or rotated about y: x and z are shared by both voxels
-      const bool ysep = (k1 == 0 || k1 == 2) && (k2 == 0 || k2 == 2) && op_is_y_separable(p1) &&
-                        (form == 1 || op_is_y_separable(p2));
-      if (ysep) {
-        bool amb = false;  // the column's polygon work is shared by both voxels
-        Iv x1 = x, z1 = z, yd = y0;
-        if (k1) rot32(OP_ROT_Y, ps1, x1, yd, z1);
-        d = prim32_y2(p1, (int)(w1 >> 8), pr1, x1, y0, y1, z1, M, amb);
-        if (form > 1) {
-          Iv x2 = x1, z2 = z1;
-          if (form == 3) {
-            x2 = x; z2 = z;
-            if (k2) rot32(OP_ROT_Y, ps2, x2, yd, z2);
-          }
-          const Iv2 e = prim32_y2(p2, (int)(w2 >> 8), pr2, x2, y0, y1, z2, M, amb);
-          d = {combine(d.a, e.a), combine(d.b, e.b)};
-        }
-        amb0 = amb1 = amb;
-      } else {
+    const uint32_t it0 = tk.get();
+    if (it0 >= n_items) break;
+    tk.issue(taken, B, lane);
+    // lane j's item: its class (the classes' counts before it: a binary search over the
+    // lanes), its queue position, loaded by all lanes at once
+    const uint32_t n_here = min(B, n_items - it0);
+    const uint32_t mine = min(it0 + (uint32_t)lane, n_items - 1);
+    int kl = 0;
+#pragma unroll
+    for (int o = 16; o; o >>= 1)
+      if (__shfl_sync(FULLMASK, incl, kl + o - 1) <= mine) kl += o;
+    const uint32_t at = __shfl_sync(FULLMASK, at0, kl) + mine;
+    uint4 items = make_uint4(0u, 0u, 0u, 0u);
+    if ((uint32_t)lane < n_here) items = __ldg(a.vitems + at);
 #pragma unroll 1
-        for (int q = 0; q < 2; q++) {
-          bool ambq = false;  // each voxel's own crossing tests
-          Iv x1 = x, y1q = q ? y1 : y0, z1 = z;
-          stage32<AFF>(k1, ps1, x1, y1q, z1);
-          Iv v = prim32(p1, (int)(w1 >> 8), pr1, x1, y1q, z1, M, ambq);
-          if (form == 2) {
-            v = combine(v, prim32(p2, (int)(w2 >> 8), pr2, x1, y1q, z1, M, ambq));
-          } else if (form == 3) {
-            Iv x2 = x, y2q = q ? y1 : y0, z2 = z;
-            stage32<AFF>(k2, ps2, x2, y2q, z2);
-            v = combine(v, prim32(p2, (int)(w2 >> 8), pr2, x2, y2q, z2, M, ambq));
-          }
-          if (q) { d.b = v; amb1 = ambq; } else { d.a = v; amb0 = ambq; }
-        }
-      }
-      if (ioff != LP_NONE) {  // offset (penthouse.ts:250)
-        const Iv o = ldp(P + (__ldg(c32 + ioff) & C32_OFF), 0);
-        d = {iadd(d.a, o), iadd(d.b, o)};
-      }
-    }
-    const uint2* code = a.code + V->code_off;
-    const int clen = (int)V->code_len;
-    uint32_t lo = 0, hi = 0, resc = 0;  // resc: bit q, voxel q of this lane left to float64
+    for (uint32_t j = 0; j < n_here; j++) {
+      const uint4 item = make_uint4(__shfl_sync(FULLMASK, items.x, j), __shfl_sync(FULLMASK, items.y, j),
+                                    __shfl_sync(FULLMASK, items.z, j), __shfl_sync(FULLMASK, items.w, j));
+      const Iv dcen = {__uint_as_float(item.z), __uint_as_float(item.w)};  // the sub-block centre's value
+      const OpDev* V = a.ops + (item.x & 0xffffffu);
+      const int ss = (int)(item.x >> 24);
+      const int vbx = (int)(item.y & 1023u), vby = (int)((item.y >> 10) & 1023u), vbz = (int)(item.y >> 20);
+      float bo[3];
+      brick_bases_f(a, V, vbx, vby, vbz, bo);
+      const int x = (ss & 1) * 4 + lx, y = ((ss >> 1) & 1) * 4 + lyv, z = ((ss >> 2) & 1) * 4 + lz;
+      const float zp[2] = {coord_f(bo[2], (float)z, a.vs_lo), coord_f(bo[2], (float)(z + 2), a.vs_lo)};
+      float lo[2], hi[2];
+      lean_f<2, G == VQ_WIDE ? 3 : 1, G != VQ_AFFINE, G != VQ_NARROW>(a, V, coord_f(bo[0], (float)x, a.vs_lo),
+                                                                      coord_f(bo[1], (float)y, a.vs_lo), zp, lo, hi);
+      uint32_t bal[2], resc[2];
 #pragma unroll
-    for (int q = 0; q < 2; q++) {
-      const Iv dk = q ? d.b : d.a;
-      const bool amb = q ? amb1 : amb0;
-      const int lipk = q ? lip1 : lip0;
-      int inside = lipk;
-      if (lipk == 3 || VALIDATE) {
-        inside = amb ? 3 : (dk.lo > V->thr[T_V_HI] ? 0 : (dk.hi <= V->thr[T_V_LO] ? 1 : 3));
+      for (int q = 0; q < 2; q++) {
+        const float t = V->lip[kc[q]];  // settled by the centre's value, or by the voxel's own
+        const int lip = dcen.lo > t ? 0 : dcen.hi < -t ? 1 : 3;
+        const int own_r = lo[q] > 0.f ? 0 : hi[q] < 0.f ? 1 : 3;
+        int inside = lip != 3 ? lip : own_r;
         if constexpr (VALIDATE) {
-          const VoxelF64 f = voxel_f64(a.params, a.vs, 1, code, clen, dk, amb, inside,
-                                       (float)(vbx * 8 + lx) + 0.5f, (float)(vby * 8 + ly0 + q) + 0.5f,
-                                       (float)(vbz * 8 + lz) + 0.5f);
-          if (f.viol) ls.viol();
-          if (inside == 3) ls.rescue(0, amb, f.err);
+          const VoxelF64 f = voxel_f64(a.params, a.vs, 1, a.code + V->code_off, (int)V->code_len, {lo[q], hi[q]}, false,
+                                       own_r, (float)(vbx * 8 + x) + 0.5f, (float)(vby * 8 + y) + 0.5f,
+                                       (float)(vbz * 8 + z + 2 * q) + 0.5f);
+          if (f.viol || (own_r != 3 && own_r != f.inside)) ls.viol();
+          if (own_r == 3) ls.rescue(0, false, f.err);
+          if (lip != 3 && f.inside != lip) ls.viol();  // the centre's bound disagreed with the evaluation
           inside = f.inside;
-          if (lipk != 3 && inside != lipk) ls.viol();  // the bound disagreed with the evaluation
-        } else if (inside == 3) {  // resolved in float64 after the work loop; outside until then
-          resc |= 1u << q;
-          inside = 0;
         }
+        bal[q] = __ballot_sync(FULLMASK, inside == 1);
+        resc[q] = __ballot_sync(FULLMASK, inside == 3);  // resolved by paint_kernel; outside until then
       }
-      const int bit = (col & 3) | ((2 * yh + q) << 2) | ((col >> 2) << 4);  // voxel index in the sub-block
-      if (inside == 1) {
-        if (bit < 32) lo |= 1u << bit;
-        else hi |= 1u << (bit - 32);
-      }
-    }
-    const unsigned long long m =
-        (unsigned long long)__reduce_or_sync(FULLMASK, lo) | ((unsigned long long)__reduce_or_sync(FULLMASK, hi) << 32);
-    // a lone box's sub-block is queued only in validation mode: check its runs
-    if (VALIDATE && (V->flags & OPF_BOX_RANGES) && lane == 0 &&
-        box_mask(V, vbx * 8 + sxo, vby * 8 + syo, vbz * 8 + szo) != m)
-      ls.viol();
-    if (lane == 0) a.pmask[vp * 8 + ss] = m;
-    if (!VALIDATE) {  // undecided voxels to the rescue list, one atomic per warp
-      const uint32_t nr = __popc(resc);
-      const uint32_t tot = __reduce_add_sync(FULLMASK, nr);
-      if (tot) {
-        uint32_t at = nr;  // this lane's first entry: an exclusive prefix over the lanes
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t t = __shfl_up_sync(FULLMASK, at, o);
-          if (lane >= o) at += t;
-        }
-        at -= nr;
+      const uint32_t pair = pair_of_brick(V, vbx, vby, vbz);
+      const unsigned long long m = (unsigned long long)bal[0] | ((unsigned long long)bal[1] << 32);
+      // a lone box's sub-block is queued only in validation mode: check its runs
+      if (VALIDATE && (V->flags & OPF_BOX_RANGES) && lane == 0 &&
+          box_mask(V, vbx * 8 + (ss & 1) * 4, vby * 8 + ((ss >> 1) & 1) * 4, vbz * 8 + ((ss >> 2) & 1) * 4) != m)
+        ls.viol();
+      if (lane == 0) a.pmask[(size_t)pair * 8 + ss] = m;
+      if (!VALIDATE && (resc[0] | resc[1])) {  // undecided voxels to the rescue list, one atomic per warp
         uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(&a.res->n_rescue, tot);
+        if (lane == 0) base = atomicAdd(&a.res->n_rescue, (uint32_t)(__popc(resc[0]) + __popc(resc[1])));
         base = __shfl_sync(FULLMASK, base, 0);
 #pragma unroll
         for (int q = 0; q < 2; q++) {
-          if (!((resc >> q) & 1u)) continue;
-          const Iv dk = q ? d.b : d.a;
-          const bool amb = q ? amb1 : amb0;
-          const int bit = (col & 3) | ((2 * yh + q) << 2) | ((col >> 2) << 4);
-          const uint4 e = make_uint4(item.x | ((uint32_t)bit << 24) | (amb ? 1u << 30 : 0u), item.y,
-                                     __float_as_uint(dk.lo), __float_as_uint(dk.hi));
-          const uint32_t r = base + at++;
-          if (r < a.rescue_cap) a.rescue[r] = e;
+          if (!((resc[q] >> lane) & 1u)) continue;
+          const uint32_t r = base + (q ? __popc(resc[0]) : 0) + __popc(resc[q] & ((1u << lane) - 1u));
+          if (r < a.rescue_cap)
+            a.rescue[r] = make_uint4((item.x & 0xffffffu) | ((uint32_t)(lane | (q << 5)) << 24),
+                                     (pair << 3) | (uint32_t)ss, __float_as_uint(lo[q]), __float_as_uint(hi[q]));
           else atomicOr(&a.res->status, (uint32_t)ST_RESCUE_OVERFLOW);
         }
       }
     }
   }
+}
+
+// A voxel the float32 points left undecided ([lo, hi]: its enclosure): float32 intervals,
+// which follow this voxel's magnitudes instead of the op's largest, then float64.  Returns
+// the decision.  Out of line: a few voxels in a build.
+__device__ __noinline__ int rescue_voxel(const FoldArgs& a, const OpDev* R, int bx, int by, int bz, int lx, int ly, int lz,
+                                         Iv dk, LaneStats& ls) {
+  Iv bo[3];
+  brick_bases(a, R, bx, by, bz, bo);
+  bool amb = false;
+  const Iv d = sdf32i(a.code + R->code_off, a.code32 + R->code_off, (int)R->code_len, reinterpret_cast<const Iv*>(a.p32),
+                      iadd(bo[0], koff((float)lx, a.vs_lo, a.vs_hi)), iadd(bo[1], koff((float)ly, a.vs_lo, a.vs_hi)),
+                      iadd(bo[2], koff((float)lz, a.vs_lo, a.vs_hi)), R->thr[T_M], amb);
+  if (!amb && d.lo > R->thr[T_V_HI]) return 0;
+  if (!amb && d.hi <= R->thr[T_V_LO]) return 1;
+  const VoxelF64 f = voxel_f64(a.params, a.vs, 0, a.code + R->code_off, (int)R->code_len, dk, false, 3,
+                               (float)(bx * 8 + lx) + 0.5f, (float)(by * 8 + ly) + 0.5f, (float)(bz * 8 + lz) + 0.5f);
+  ls.rescue(0, amb, f.err);
+  return f.inside;
 }
 
 // One paint call at voxel (x, y, z) of the world, in float64 (the paint kinds
@@ -1191,13 +1118,16 @@ __device__ __forceinline__ uint32_t paint_voxel(const FoldArgs& a, const OpDev* 
 // warp from evaluating a painted brick's 512 calls alone.  Mixed mode tries the
 // certified float32 evaluation first (paint32.cuh).
 // Mixed form: first the voxels the lean voxel kernels left undecided (the rescue
-// list), one per thread, in float64 (shapes.ts:393): the inside ones are ORed
-// into their sub-block masks, and a painted op's paint value is stored for them
-// here.  Entry r goes to block r mod gridDim.x, so a warp holds few (an FP64
-// instruction of a sparse warp is far quicker than a full one: FP64 runs at 1/64
-// of the float32 rate) and the float64 chains overlap the paint work.  A paint
-// item of the same sub-block may read its mask before or after the OR: it then
-// paints the voxel too or leaves it out, and either way stores the same value.
+// list), one per thread, in intervals, then float64 (shapes.ts:393): the inside ones
+// are ORed into their sub-block masks, and a painted op's paint value is stored for
+// them here.  Bound by instruction fetch: long programs run once by few lanes.  So two
+// warps per SM take them, neighbouring entries (mostly of one shape) in one warp, beside
+// the paint work of the others.  Paint pass of the synthetic scene (7,672 entries, 410 of
+// them left to float64; 129 us without any): two warps per SM 149 us, one 156, four 201,
+// every warp 189 to 211, and float64 at once in two 153; the penthouse at 80 voxels per
+// metre (870 entries, 37 us without): 41, 40, 42, 41 to 44, and 57 us.  A paint item of the
+// same sub-block may read its mask before or after the OR: it then paints the voxel too
+// or leaves it out, and either way stores the same value.
 template <int MODE>
 __global__ void __launch_bounds__(256, PX_PAINT_MINB) paint_kernel(FoldArgs a) {
   pdl_prologue();
@@ -1206,21 +1136,20 @@ __global__ void __launch_bounds__(256, PX_PAINT_MINB) paint_kernel(FoldArgs a) {
   if (MODE == 1) {
     LaneStats ls = {a.res};
     const uint32_t n_resc = min(__ldcg(&a.res->n_rescue), a.rescue_cap);
-    for (uint32_t r = blockIdx.x + gridDim.x * threadIdx.x; r < n_resc; r += gridDim.x * blockDim.x) {
+    // one warp of each of half the blocks takes consecutive entries
+    const uint32_t nb = (gridDim.x + 1) / 2, per = (n_resc + nb - 1) / nb;
+    const uint32_t end = threadIdx.x < 32 && blockIdx.x < nb ? min(n_resc, (blockIdx.x + 1) * per) : 0u;
+    for (uint32_t r = blockIdx.x * per + (uint32_t)lane; r < end; r += 32) {
       const uint4 ri = __ldcg(a.rescue + r);
       const OpDev* R = a.ops + (ri.x & 0xffffffu);
       const int bit = (int)((ri.x >> 24) & 63u);
-      const bool ramb = (ri.x >> 30) & 1u;
       const unsigned long long rp = ri.y >> 3;
       const int rs = ri.y & 7;
       int rbx, rby, rbz;
       brick_of_pair(R, rp, rbx, rby, rbz);
       const int lx = (rs & 1) * 4 + (bit & 3), ly = ((rs >> 1) & 1) * 4 + ((bit >> 2) & 3), lz = ((rs >> 2) & 1) * 4 + (bit >> 4);
       const Iv dk = {__uint_as_float(ri.z), __uint_as_float(ri.w)};
-      const VoxelF64 f = voxel_f64(a.params, a.vs, 0, a.code + R->code_off, (int)R->code_len, dk, ramb, 3,
-                                   (float)(rbx * 8 + lx) + 0.5f, (float)(rby * 8 + ly) + 0.5f, (float)(rbz * 8 + lz) + 0.5f);
-      ls.rescue(0, ramb, f.err);
-      if (!f.inside) continue;
+      if (!rescue_voxel(a, R, rbx, rby, rbz, lx, ly, lz, dk, ls)) continue;
       atomicOr(a.pmask + rp * 8 + rs, 1ull << bit);
       if (R->paint_slot == NO_SLOT) continue;
       Iv bo[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
@@ -1662,7 +1591,8 @@ void launch_fold(const FoldArgs& a, int mode, int n_sms, cudaStream_t s, cudaEve
       if (a.validate) launch_pdl(voxel_lean_kernel<true, VQ_WIDE>, dim3(grid(PX_VWIDE_MINB)), dim3(256), 0, s, a);
       else launch_pdl(voxel_lean_kernel<false, VQ_WIDE>, dim3(grid(PX_VWIDE_MINB)), dim3(256), 0, s, a);
     }
-    launch_pdl(voxel_kernel<1, VQ_GENERIC, VQ_GENERIC>, dim3(grid(PX_VOXEL_MINB)), dim3(256), 0, s, a);
+    if (a.vq_nonempty & (1u << VQ_GENERIC))
+      launch_pdl(voxel_kernel<1, VQ_GENERIC, VQ_GENERIC>, dim3(grid(PX_VOXEL_MINB)), dim3(256), 0, s, a);
   } else {
     launch_pdl(classify_kernel<0>, dim3(grid(PX_CLASSIFY64_MINB)), dim3(256), 0, s, a);
     launch_pdl(sub_kernel<0>, dim3(grid(PX_CLASSIFY64_MINB)), dim3(256), 0, s, a);

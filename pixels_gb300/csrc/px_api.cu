@@ -326,7 +326,7 @@ bool compose_rotations(const uint32_t* code, uint32_t i, uint32_t k, const doubl
   return ok;
 }
 
-// The lean voxel kernel's reading of a program (LP_* forms in px_internal.cuh), or
+// The reading of a lean program (LP_* forms in px_internal.cuh), or
 // lp[LP_FORM] = 0.  A stage is one rotation, or a run composed by rotation_runs.
 void lean_program(const uint32_t* code, uint32_t n, uint8_t lp[8]) {
   if (n > 40) return;
@@ -484,6 +484,161 @@ bool convert32(const uint32_t* code, uint32_t n, const double* P, const double A
     }
   }
   return ok;
+}
+
+// ---------------------------------------------------------------------------
+// Error bound of a lean program's float32 point value (sdf32p.cuh).
+//
+// Each quantity carries m, a bound of its exact magnitude, and e, a bound of
+// |float32 value - exact value|, where "exact" is the expression on the exact
+// inputs.  The functions below repeat the device's operations: an operation's
+// error is the first- and second-order effect of its operands' errors plus half
+// a unit in the last place, 2^-24 of the magnitude computed.
+struct EB {
+  double m, e;
+};
+constexpr double U32 = 0x1p-24;
+static inline EB eb_round(EB a) { return {a.m, a.e + U32 * (a.m + a.e)}; }
+static inline EB eb_add(EB a, EB b) { return eb_round({a.m + b.m, a.e + b.e}); }
+static inline EB eb_mul(EB a, EB b) { return eb_round({a.m * b.m, a.m * b.e + a.e * b.m + a.e * b.e}); }
+static inline EB eb_fma(EB a, EB b, EB c) {
+  return eb_round({a.m * b.m + c.m, a.m * b.e + a.e * b.m + a.e * b.e + c.e});
+}
+static inline EB eb_sat(EB a) { return {std::min(a.m, 1.0), std::min(a.e, 1.0)}; }  // clamped to [0, 1]
+static inline EB eb_max(EB a, EB b) { return {std::max(a.m, b.m), std::max(a.e, b.e)}; }  // minima and maxima
+// A length: 1-Lipschitz in its components; the squares, sums (2^-24 each, of
+// positive terms), the reciprocal root (2^-22.9) and the product come to less
+// than 8 * 2^-24 of the length, and the floor of the root's argument to 2^-50.
+static inline EB eb_len(EB a, EB b, EB c = {0, 0}) {
+  const double m = std::sqrt(a.m * a.m + b.m * b.m + c.m * c.m), e = std::sqrt(a.e * a.e + b.e * b.e + c.e * c.e);
+  return {m, e + 8 * U32 * (m + e) + 0x1p-49};
+}
+static inline EB eb_extrude(EB d, EB h) { return eb_add(eb_max(d, h), eb_len(d, h)); }
+// a constant: the device takes the lower end of its interval
+static inline EB eb_param(const float2& v) {
+  return {std::max(std::fabs((double)v.x), std::fabs((double)v.y)), (double)v.y - (double)v.x};
+}
+
+// polygon_f's signed distance.  Unsigned, the worst edge's.  The sign can differ
+// from the exact polygon's only near the boundary: moving the point and the vertices
+// linearly from their exact to their float32 places crosses no edge unless the point
+// lies within those moves (dp, dv) of the boundary; and on the float32 polygon an edge
+// whose ends straddle the point's height is taken on the wrong side only if the two
+// products compared differ by less than their own errors (3 * 2^-24 each), which
+// leaves the crossing, on the edge, within 9 * 2^-24 of the edge's width (at most
+// twice the vertices' magnitude) from the point.  There the distance is off by
+// at most twice that, added to the bound.
+static EB eb_polygon(EB px, EB py, const float2* r, uint32_t n) {
+  EB bx = {0, 0}, by = {0, 0};
+  double dv = 0, V = 0;
+  for (uint32_t i = 0; i < n; i++, r += 6) {
+    const EB vx = eb_param(r[0]), vy = eb_param(r[1]), ex = eb_param(r[3]), ey = eb_param(r[4]), inv = eb_param(r[5]);
+    const EB wx = eb_add(px, vx), wy = eb_add(py, vy);
+    const EB t = eb_sat(eb_mul(eb_fma(wx, ex, eb_mul(wy, ey)), inv));
+    bx = eb_max(bx, eb_fma(ex, t, wx));  // (at least w's: the first distance is to a vertex)
+    by = eb_max(by, eb_fma(ey, t, wy));
+    dv = std::max(dv, vx.e + vy.e);
+    V = std::max(V, std::max(vx.m, vy.m));
+  }
+  const EB d = eb_len(bx, by);
+  const double near = px.e + py.e + dv + 20 * U32 * V;
+  return {d.m, d.e + 2 * near};
+}
+
+static EB eb_polyline(EB px, EB py, const float2* r, uint32_t n) {
+  EB bx = {0, 0}, by = {0, 0};
+  for (uint32_t i = 0; i < n; i++, r += 5) {
+    const EB ex = eb_param(r[2]), ey = eb_param(r[3]), inv = eb_param(r[4]);
+    const EB wx = eb_add(px, eb_param(r[0])), wy = eb_add(py, eb_param(r[1]));
+    const EB t = eb_sat(eb_mul(eb_fma(wx, ex, eb_mul(wy, ey)), inv));
+    bx = eb_max(bx, eb_fma(ex, t, wx));
+    by = eb_max(by, eb_fma(ey, t, wy));
+  }
+  return eb_len(bx, by);
+}
+
+// prim_f
+static EB eb_prim(uint32_t w, const float2* p, const EB x[3]) {
+  const uint32_t op = w & 0xffu, cnt = w >> 8;
+  auto c = [&](int k) { return eb_param(p[k]); };
+  switch (op) {
+    case OP_BOX: case OP_ROUNDBOX: {
+      const EB q0 = eb_add(eb_add(x[0], c(0)), c(3)), q1 = eb_add(eb_add(x[1], c(1)), c(4)),
+               q2 = eb_add(eb_add(x[2], c(2)), c(5));
+      const EB d = eb_add(eb_len(q0, q1, q2), eb_max(eb_max(q0, q1), q2));
+      return eb_add(d, op == OP_ROUNDBOX ? c(6) : EB{0, 0});
+    }
+    case OP_SPHERE: return eb_add(eb_len(eb_add(x[0], c(0)), eb_add(x[1], c(1)), eb_add(x[2], c(2))), c(3));
+    case OP_ELLIPSOID:
+      return eb_mul(eb_add(eb_len(eb_mul(eb_add(x[0], c(0)), c(3)), eb_mul(eb_add(x[1], c(1)), c(4)),
+                                  eb_mul(eb_add(x[2], c(2)), c(5))), {1, 0}), c(6));
+    case OP_CAPSULE: {
+      const EB a0 = eb_add(x[0], c(0)), a1 = eb_add(x[1], c(1)), a2 = eb_add(x[2], c(2));
+      const EB t = eb_sat(eb_mul(eb_fma(a2, c(5), eb_fma(a1, c(4), eb_mul(a0, c(3)))), c(6)));
+      return eb_add(eb_len(eb_fma(c(3), t, a0), eb_fma(c(4), t, a1), eb_fma(c(5), t, a2)), c(7));
+    }
+    case OP_CYL_X: case OP_CYL_Y: case OP_CYL_Z: case OP_TORUS_X: case OP_TORUS_Y: case OP_TORUS_Z: {
+      const int axis = (int)(op >= OP_TORUS_X ? op - OP_TORUS_X : op - OP_CYL_X);
+      const EB a = eb_add(x[(axis + 1) % 3], c((axis + 1) % 3)), b = eb_add(x[(axis + 2) % 3], c((axis + 2) % 3)),
+               h = eb_add(x[axis], c(axis));
+      const EB dr = eb_add(eb_len(a, b), c(3));
+      return op >= OP_TORUS_X ? eb_add(eb_len(dr, h), c(4)) : eb_extrude(dr, eb_add(h, c(4)));
+    }
+    case OP_LATHE_SOLID: case OP_LATHE_SHELL: {
+      const EB r = eb_len(eb_add(x[0], c(0)), eb_add(x[2], c(2))), h = eb_add(x[1], c(1));
+      return op == OP_LATHE_SOLID ? eb_polygon(r, h, p + 3, cnt) : eb_add(eb_polyline(r, h, p + 4, cnt - 1), c(3));
+    }
+    case OP_PRISM:
+      return eb_extrude(eb_polygon(eb_add(x[0], c(0)), eb_add(x[2], c(1)), p + 4, cnt),
+                        eb_add(eb_add(x[1], c(2)), c(3)));
+    case OP_STADIUM:
+      return eb_extrude(eb_add(eb_len(eb_add(eb_add(x[0], c(0)), c(2)), eb_add(x[2], c(1))), c(3)),
+                        eb_add(eb_add(x[1], c(4)), c(5)));
+  }
+  return {0, std::numeric_limits<double>::infinity()};
+}
+
+// stage_f
+static void eb_stage(uint32_t kind, const float2* p, const EB in[3], EB out[3]) {
+  auto c = [&](int k) { return eb_param(p[k]); };
+  if (kind == LP_AFFINE) {
+    for (int r = 0; r < 3; r++)
+      out[r] = eb_fma(c(3 * r + 2), in[2], eb_fma(c(3 * r + 1), in[1], eb_fma(c(3 * r), in[0], c(9 + r))));
+    return;
+  }
+  for (int k = 0; k < 3; k++) out[k] = in[k];
+  if (!kind) return;
+  const int iu = kind == 1 ? 1 : 0, iv = kind == 3 ? 1 : 2;
+  const EB u = eb_add(in[iu], c(0)), v = eb_add(in[iv], c(1));
+  out[iu] = eb_fma(c(2), u, eb_fma(c(3), v, c(0)));
+  out[iv] = eb_fma(c(2), v, eb_fma(c(3), u, c(1)));
+}
+
+// The error bounds of the op's lean program (d.lw), per primitive, over the points of its
+// bricks (bases: their first voxel centres as float32 intervals, per axis; up to 7 voxels
+// on), with the margin between the exact value and the reference's float64 one.
+static void lean_error(const OpDev& d, const float2* p32, const float2* bases, const int n[3], float vs_lo, float vs_hi,
+                       double E[2]) {
+  EB x[3];
+  for (int k = 0; k < 3; k++) {
+    double m = 0, w = 0;
+    for (int i = 0; i < n[k]; i++, bases++) {
+      m = std::max(m, std::max(std::fabs((double)bases->x), std::fabs((double)bases->y)));
+      w = std::max(w, (double)bases->y - (double)bases->x);
+    }
+    const EB step = eb_round({8.0 * vs_hi, 8.0 * ((double)vs_hi - vs_lo)});
+    x[k] = eb_add({m, w}, step);
+  }
+  EB y[3];
+  const uint32_t form = d.lw[0] & 0xffu;
+  eb_stage((d.lw[0] >> 16) & 15u, p32 + d.lw[3], x, y);
+  // (the factor: this arithmetic's own rounding)
+  E[0] = eb_prim(d.lw[1], p32 + d.lw[2], y).e * (1 + 0x1p-20) + MIXED_MARGIN;
+  E[1] = 0;
+  if (form > 1) {
+    if (form == 3) eb_stage((d.lw[0] >> 20) & 15u, p32 + d.lw[6], x, y);
+    E[1] = eb_prim(d.lw[4], p32 + d.lw[5], y).e * (1 + 0x1p-20) + MIXED_MARGIN;
+  }
 }
 
 // Validate one op's SDF bytecode: opcodes, parameter ranges, finite values,
@@ -909,7 +1064,6 @@ int convert_ops(const px_world* w, const IrOp* iops, size_t i0, size_t i1, const
       if (opk >= OP_BOX && opk < OP_ROT_X) first_prim = opk;
     }
     d.paint_off = (uint32_t)(param_base + o.paint_param);
-    for (int k = 0; k < 3; k++) { d.mn[k] = o.mn[k]; d.mx[k] = o.mx[k]; }
     for (int k = 0; k < 4; k++) d.frame[k] = o.frame[k];
     // shapes.ts:341-347: voxel range of the op, clamped to the world
     double vx0 = js_max(0, std::floor(o.mn[0] / vs - 0.5)), vy0 = js_max(0, std::floor(o.mn[1] / vs - 0.5)),
@@ -1012,7 +1166,7 @@ int convert_ops(const px_world* w, const IrOp* iops, size_t i0, size_t i1, const
         for (int k = 0; k < 3; k++)
           for (int b = b0[k]; b <= b1[k]; b++) out.bases.push_back(enc((b * 8 + 0.5) * vs - d.anchor[k], 0x1p-38));
       }
-      size_t c32_before = out.code32.size(), p32_before = out.p32.size();
+      const size_t c32_before = out.code32.size();
       bool ok32 = convert32(code + 2 * (size_t)o.code_begin, o.code_len, P, d.anchor, out.code32, out.p32);
       double ext = (double)w->dx * vs;
       if ((double)w->dy * vs > ext) ext = (double)w->dy * vs;
@@ -1024,17 +1178,44 @@ int convert_ops(const px_world* w, const IrOp* iops, size_t i0, size_t i1, const
           ysep = ysep && op_is_y_separable(code[2 * ((size_t)o.code_begin + k)] & 0xffu);
         if (ysep) d.flags |= OPF_Y_SEPARABLE;
         d.vclass = (first_prim & 15u) | (ysep && !(d.flags & OPF_FP64_ONLY) ? 16u : 0u);
-        // a program of the lean voxel kernel (LP_* forms)
-        for (int k = 0; k < 8; k++) d.lp[k] = 0;
-        if (!(d.flags & (OPF_FP64_ONLY | OPF_DEEP))) lean_program(code + 2 * (size_t)o.code_begin, o.code_len, d.lp);
+        // a lean program (LP_* forms), where its float32 points decide all but a few voxels: an
+        // error bound of up to 1/128 voxel leaves at most about one in 300 near the surface
+        // undecided (shapes of some 50 m at 80 voxels per metre; larger ones take the
+        // interpreter).  A second primitive may be far away, and its bound larger
+        uint8_t lp[8] = {0};
+        const uint32_t* oc = code + 2 * (size_t)o.code_begin;
+        if (!(d.flags & (OPF_FP64_ONLY | OPF_DEEP)) && d.bx0 <= d.bx1) lean_program(oc, o.code_len, lp);
+        for (int k = 0; k < 8; k++) d.lw[k] = 0;
+        d.err[0] = d.err[1] = 0.f;
+        if (lp[LP_FORM]) {
+          auto par = [&](uint32_t i) { return out.code32[c32_before + i] & C32_OFF; };  // range-local (merge)
+          const uint32_t k1 = lp[LP_KINDS] & 15u, k2 = lp[LP_KINDS] >> 4;
+          d.lw[0] = lp[LP_FORM] | ((uint32_t)lp[LP_COMB] << 8) | (k1 << 16) | (k2 << 20) |
+                    (lp[LP_OFF] != LP_NONE ? 1u << 24 : 0u);
+          d.lw[1] = oc[2 * lp[LP_P1]];
+          d.lw[2] = par(lp[LP_P1]);
+          d.lw[3] = par(0);  // the first stage is instruction 0
+          d.lw[4] = lp[LP_FORM] > 1 ? oc[2 * lp[LP_P2]] : 0u;
+          d.lw[5] = lp[LP_FORM] > 1 ? par(lp[LP_P2]) : 0u;
+          d.lw[6] = k2 ? par(lp[LP_S2]) : 0u;
+          d.lw[7] = lp[LP_OFF] != LP_NONE ? par(lp[LP_OFF]) : 0u;
+          const int nb[3] = {d.bx1 - d.bx0 + 1, d.by1 - d.by0 + 1, d.bz1 - d.bz0 + 1};
+          double E[2];
+          lean_error(d, out.p32.data(), out.bases.data() + d.base_off, nb, rd32(vs), ru32(vs), E);
+          if (E[0] <= vs / 128 && E[1] <= vs / 32) {
+            d.err[0] = ru32(E[0]);
+            d.err[1] = ru32(E[1]);
+          } else {
+            for (int k = 0; k < 8; k++) { d.lw[k] = 0; lp[k] = 0; }
+          }
+        }
         // the voxel queue's group and class: one primitive under at most one rotation
         // (by primitive and rotation), the other lean forms (by first primitive and
         // form), the interpreter's programs (by sub-block class)
-        const uint32_t p1op = d.lp[LP_FORM] ? code[2 * ((size_t)o.code_begin + d.lp[LP_P1])] & 15u : 0u;
-        const uint32_t k1 = d.lp[LP_KINDS] & 15u;
-        if (d.lp[LP_FORM] == 1 && k1 != LP_AFFINE) d.vq_class = 32u * VQ_NARROW + (p1op | (k1 ? 16u : 0u));
-        else if (d.lp[LP_FORM] == 1) d.vq_class = 32u * VQ_AFFINE + p1op;
-        else if (d.lp[LP_FORM]) d.vq_class = 32u * VQ_WIDE + (p1op | (d.lp[LP_FORM] == 3 ? 16u : 0u));
+        const uint32_t p1op = d.lw[1] & 15u, k1 = lp[LP_KINDS] & 15u;
+        if (lp[LP_FORM] == 1 && k1 != LP_AFFINE) d.vq_class = 32u * VQ_NARROW + (p1op | (k1 ? 16u : 0u));
+        else if (lp[LP_FORM] == 1) d.vq_class = 32u * VQ_AFFINE + p1op;
+        else if (lp[LP_FORM]) d.vq_class = 32u * VQ_WIDE + (p1op | (lp[LP_FORM] == 3 ? 16u : 0u));
         else d.vq_class = 32u * VQ_GENERIC + d.vclass;
       }
       d.paint_slot = NO_SLOT;
@@ -1047,8 +1228,6 @@ int convert_ops(const px_world* w, const IrOp* iops, size_t i0, size_t i1, const
         else
           out.p32.resize(at);
       }
-      (void)c32_before;
-      (void)p32_before;
     }
     d.cost = op_cost(code + 2 * (size_t)o.code_begin, o.code_len, d.flags);
     // the op's first (op, brick) pair (range-local; rebased when the ranges merge), its
@@ -1352,7 +1531,9 @@ static int submit_ops_impl(px_world* w, const void* ir, size_t bytes) {
   // convert the ops in contiguous ranges on the host pool, then append the
   // ranges in order (offsets rebased)
   HostPool& pool = HostPool::get();
-  const int n_chunks = n_ops < 512 ? 1 : (int)std::min<size_t>((size_t)pool.size() * 4, n_ops / 32);
+  // (few short programs -- a serving step's edits -- are not worth waking the pool for)
+  const bool few = n_ops < 64 || (n_ops < 512 && n_code < 1024);
+  const int n_chunks = few ? 1 : (int)std::min<size_t>((size_t)pool.size() * 4, n_ops / 32);
   std::vector<SubmitChunk> chunks(n_chunks);
   pool.run(n_chunks, [&](int k) {
     const size_t i0 = n_ops * k / n_chunks, i1 = n_ops * (k + 1) / n_chunks;
@@ -1403,6 +1584,8 @@ static int submit_ops_impl(px_world* w, const void* ir, size_t bytes) {
       d.base_off += (uint32_t)pl.bases;
       d.pair_base += pl.pairs;
       if (d.paint32_off != NO_SLOT) d.paint32_off += (uint32_t)pl.p32;
+      if (d.lw[0])
+        for (int k : {2, 3, 5, 6, 7}) d.lw[k] += (uint32_t)pl.p32;
     }
     auto put = [](auto& dst, size_t pos, const auto& src) {
       if (!src.empty()) std::memcpy(dst.data() + pos, src.data(), src.size() * sizeof(src[0]));

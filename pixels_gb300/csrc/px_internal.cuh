@@ -1,5 +1,6 @@
 // Shared definitions of the voxeliser's host runtime and kernels.
 #pragma once
+#include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -69,45 +70,55 @@ struct IrOp {
 };
 static_assert(sizeof(IrOp) == 128, "PXIR op is 128 bytes");
 
-// An op as the kernels see it.
-struct OpDev {
-  int32_t bx0, by0, bz0, bx1, by1, bz1;  // brick box (inclusive), from apply()'s voxel range
-  int32_t nx, ny;                        // box extent in bricks (x, y)
+// An op as the kernels see it.  Grouped by the passes that read it, in 32-byte sectors of
+// whole 128-byte lines: the apply pass reads the first sector, the lean programs' passes the
+// first line (laid out by subject instead, over 400 bytes: sub-block pass of the penthouse at
+// 80 voxels per metre 61 us, apply 124; so 54 and 117).
+struct alignas(128) OpDev {
   uint64_t pair_base;                    // index of the op's first (op, brick) pair
-  // ceil(2^64 / nx) and ceil(2^64 / (nx ny)) (0 for a divisor of 1): a pair's brick
-  // row and slab by one 64-bit high multiply instead of a division (brick_of_pair)
-  uint64_t inv_nx, inv_nxy;
-  uint32_t code_off, code_len;           // SDF bytecode (uint2 records)
-  uint32_t paint_off;                    // paint parameters (doubles)
   uint8_t kind, flags;
   uint16_t paint_kind;
   uint32_t paint_value;
-  uint32_t vclass;                       // sub-block work class (VCLASSES): first primitive, y-extruded
-  uint32_t vq_class;                     // voxel work class (VQ_CLASSES): 32 per VQ_* group
-  // a program of the lean voxel kernel (LP_* forms; lp[LP_FORM] == 0: not one): instruction
-  // indices within the op of its primitives, stages and offset, and the stages' kinds
-  uint8_t lp[8];
-  double bhd, shd;                       // brickHalfDiag, subHalfDiag (shapes.ts:349-350)
-  double mn[3], mx[3];                   // contains box (boxes only)
-  double frame[4];                       // paint frame px, pz, cos, sin
-  double anchor[3];                      // mixed mode: origin of the op's float32 coordinates
-  float thr[12];                         // mixed mode thresholds (T_*)
-  int32_t cbx0, cby0, cbz0, cbx1, cby1, cbz1;  // bricks the box fully contains (contains(), shapes.ts:47-48,360)
-  uint32_t base_off;                     // mixed mode: float32 first-voxel-centre offsets per brick row
-  float cost;                            // relative cost of one evaluation (work order only)
-  // OPF_BOX_RANGES (a lone axis-aligned box): per axis, the first and last voxel
-  // whose centre the reference's float64 box SDF puts inside on that axis
-  int32_t vr[6];                         // x lo, x hi, y lo, y hi, z lo, z hi (empty: lo > hi)
   // paints evaluated ahead of the apply pass (paint_kernel): the op's first
   // paint slot (one slot of 512 values per (op, brick) pair), or NO_SLOT
   uint32_t paint_slot;
   // mixed mode: float32 parameters of the certified paint evaluation (p32 index), or NO_SLOT
   uint32_t paint32_off;
+  uint32_t base_off;                     // mixed mode: float32 first-voxel-centre offsets per brick row
+  uint32_t vq_class;                     // voxel work class (VQ_CLASSES): 32 per VQ_* group
+
+  int32_t bx0, by0, bz0, bx1, by1, bz1;  // brick box (inclusive), from apply()'s voxel range
+  int32_t nx, ny;                        // box extent in bricks (x, y)
+
+  // a lean program (LP_* forms; lw[0] == 0: not one), all a kernel needs of it in two
+  // 16-byte loads: form | combinator << 8 | first stage's kind << 16 | second's << 20 |
+  // has an offset << 24; first primitive (opcode | count << 8), its parameters and its
+  // stage's (p32 indices); the second primitive's three; the offset's parameter
+  uint32_t lw[8];
+
   // mixed mode: a voxel of a partial sub-block is outside if the sub-block centre's
   // value exceeds lip[k], inside if it is below -lip[k] (k: the voxel's distance class
   // from the centre; every shape's SDF is Lipschitz with constant <= its slack)
   float lip[4];
+  float err[2];                          // error bounds of a lean program's float32 points, per primitive (plus the margin)
+  uint32_t vclass;                       // sub-block work class (VCLASSES): first primitive, y-extruded
+  float cost;                            // relative cost of one evaluation (work order only)
+
+  // ceil(2^64 / nx) and ceil(2^64 / (nx ny)) (0 for a divisor of 1): a pair's brick
+  // row and slab by one 64-bit high multiply instead of a division (brick_of_pair)
+  uint64_t inv_nx, inv_nxy;
+  uint32_t code_off, code_len;           // SDF bytecode (uint2 records)
+  uint32_t paint_off;                    // paint parameters (doubles)
+  float thr[T_COUNT];                    // mixed mode thresholds (T_*)
+  int32_t cbx0, cby0, cbz0, cbx1, cby1, cbz1;  // bricks the box fully contains (contains(), shapes.ts:47-48,360)
+  // OPF_BOX_RANGES (a lone axis-aligned box): per axis, the first and last voxel
+  // whose centre the reference's float64 box SDF puts inside on that axis
+  int32_t vr[6];                         // x lo, x hi, y lo, y hi, z lo, z hi (empty: lo > hi)
+  double bhd, shd;                       // brickHalfDiag, subHalfDiag (shapes.ts:349-350)
+  double frame[4];                       // paint frame px, pz, cos, sin
+  double anchor[3];                      // mixed mode: origin of the op's float32 coordinates
 };
+static_assert(sizeof(OpDev) == 384 && offsetof(OpDev, lw) == 64 && offsetof(OpDev, inv_nx) == 128, "lines as laid out");
 constexpr uint32_t NO_SLOT = 0xffffffffu;
 // paint kinds whose calls are the most expensive (transcendentals, Math.hypot):
 // chip stack, tufted, vase, painting.  Their calls are evaluated ahead of the
@@ -150,7 +161,7 @@ struct BuildResult {
   BuildCounters c;
   unsigned long long max_err_bits;  // max |mid(d32) - d64| over rescued evaluations (double bits, >= 0)
   uint32_t free_len;     // derive: length of the GPU free list (GpuWorld.ts:103-111, C_FREE_TOP)
-  uint32_t n_rescue;     // voxels the float32 pass left to float64 (voxel_lean_kernel), pushed
+  uint32_t n_rescue;     // voxels the float32 points left undecided (voxel_lean_kernel), pushed
   uint32_t h_before;     // holes before the build (from the WorldState)
   uint32_t u_before;     // poolUsed before the build
   uint32_t pad2;
@@ -175,14 +186,14 @@ constexpr int VQ_CLASSES = 128;
 constexpr int VQ_TAKEN = 1 + VQ_CLASSES;  // vitem_counter[VQ_TAKEN + group]: items the group's kernel took
 constexpr int CULL_COUNTER = 200;         // chunk_counter[CULL_COUNTER]: tile-list entries reserved by cull_kernel
 
-// Programs of the lean voxel kernels, by form:
+// Lean programs (lean_f, sdf32p.cuh), by form:
 //   1  [stage] prim [stage end] [offset]
 //   2  [stage] prim prim comb [stage end] [offset]           (one stage for both)
 //   3  [stage] prim [stage end] [stage] prim [stage end] comb [offset]
 // A stage is one rotation (kind 1-3: about x, y, z) or a run of rotations the
 // float32 parameters hold composed into one affine map (kind 4); comb is a
 // subtract step, an intersection or a union.
-enum { LP_FORM, LP_COMB, LP_P1, LP_P2, LP_S1, LP_S2, LP_KINDS, LP_OFF };
+enum { LP_FORM, LP_COMB, LP_P1, LP_P2, LP_S1, LP_S2, LP_KINDS, LP_OFF };  // lean_program's reading (host)
 enum : uint8_t { LP_NEGMAX = 1, LP_MAX = 2, LP_MIN = 3, LP_NONE = 0xff, LP_AFFINE = 4 };
 // code32 flags of the float32 path: a run of rotations (not all about y) composed
 // into an affine map on its first rotation; its other rotations and all but the
@@ -202,13 +213,13 @@ struct FoldArgs {
   uint16_t* psub;             // per partial pair: 2 bits per sub-block (PC_*)
   unsigned long long* pmask;  // per partial pair: 8 inside-masks (bit = x&3 | (y&3)<<2 | (z&3)<<4)
   uint32_t* chunk_counter;
-  // voxels whose float32 interval cannot decide them, left by voxel_lean_kernel to
-  // paint_kernel<1> (which resolves them in float64 first): (op | voxel bit << 24 |
-  // undecided-crossing-test << 30, pair << 3 | sub-block, interval lo, hi bits)
+  // voxels whose float32 point cannot decide them, left by voxel_lean_kernel to
+  // paint_kernel<1> (which resolves them first): (op | voxel bit << 24, pair << 3 |
+  // sub-block, the point's enclosure lo, hi bits)
   uint4* rescue;
   uint32_t rescue_cap;
-  uint4* vitems;              // partial sub-blocks to classify voxel by voxel: (op, pair << 3 | sub,
-                              // bits of the centre value's enclosure lo, hi)
+  uint4* vitems;              // partial sub-blocks to classify voxel by voxel: (op | sub-block << 24, brick
+                              // x | y << 10 | z << 20, bits of the centre value's enclosure lo, hi)
   uint32_t vitems_cap;
   uint32_t* vitem_counter;    // [1 + k] items pushed to class k, [VQ_TAKEN + g] items taken from group g
   uint32_t vq_base[VQ_CLASSES], vq_cap[VQ_CLASSES];  // per-class regions of vitems
