@@ -421,6 +421,8 @@ __device__ __forceinline__ int eval_decide(const FoldArgs& a, const OpDev* O, co
   const double vs = a.vs;
   const double X = (double)tx * vs, Y = (double)ty * vs, Z = (double)tz * vs;
   const double d = (O->flags & OPF_DEEP) ? sdf64_deep(code, clen, a.params, X, Y, Z) : sdf64(code, clen, a.params, X, Y, Z);
+  // the exact value lies within the margin of this one, where the op's range is certified
+  if (dout && !(O->flags & OPF_FP64_ONLY)) *dout = {__double2float_rd(d - MIXED_MARGIN), __double2float_ru(d + MIXED_MARGIN)};
   if (what == 0) return d > 0.0 ? 0 : 1;
   return classify64(d, what == 1 ? O->bhd : O->shd);
 }
@@ -665,7 +667,7 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_CLASSIFY_MINB : PX_CLASSIF
 // The rest of the sub-block pass for one sub-block per lane (`have`), its class
 // scls known: the voxel mask of a lone box's partial sub-block (per-axis runs),
 // the paint items of a covered sub-block of a painted op, the Lipschitz decision
-// of a partial sub-block (mixed form) and its voxel work item.  Warp-collective.
+// of a partial sub-block and its voxel work item.  Warp-collective.
 template <int MODE>
 __device__ __forceinline__ void sub_finish(const FoldArgs& a, bool have, uint32_t oo, unsigned long long pp, int pbx,
                                            int pby, int pbz, int s, int scls, Iv dc, bool boxr, int lane,
@@ -695,10 +697,10 @@ __device__ __forceinline__ void sub_finish(const FoldArgs& a, bool have, uint32_
       }
     }
   }
-  // mixed form: a partial sub-block whose centre value is farther from 0 than
-  // every voxel's distance bound (Lipschitz) has all its voxels decided
+  // a partial sub-block whose centre value is farther from 0 than every voxel's
+  // distance bound (Lipschitz) has all its voxels decided
   bool lipd = false;
-  if (MODE == 1 && have && scls == PC_PARTIAL && !boxr && !a.validate) {
+  if (have && scls == PC_PARTIAL && !boxr && !a.validate) {
     const float l3 = a.ops[oo].lip[3];
     if (dc.lo > l3 || dc.hi < -l3) {
       a.pmask[pp * 8 + s] = dc.lo > l3 ? 0ull : ~0ull;
@@ -764,7 +766,7 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_SUB_MINB : PX_CLASSIFY64_M
     unsigned long long pp = 0;
     int pbx = 0, pby = 0, pbz = 0, scls = PC_SKIP;
     bool boxr = false;
-    Iv dc = {-INFINITY, INFINITY};  // enclosure of the sub-block centre's value (mixed form)
+    Iv dc = {-INFINITY, INFINITY};  // enclosure of the sub-block centre's value
     if (have) {
       const uint2 item = __ldg(a.pitems + a.pq_base[a.class_order[my_k]] + (it - my_first));
       oo = item.x;
@@ -790,7 +792,7 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_SUB_MINB : PX_CLASSIFY64_M
         scls = eval_decide<MODE>(a, Q, a.code + Q->code_off, (int)Q->code_len, use32, bo, 4.f * sxb + 1.5f,
                                  4.f * syb + 1.5f, 4.f * szb + 1.5f, (float)(pbx * 8 + sxb * 4 + 2),
                                  (float)(pby * 8 + syb * 4 + 2), (float)(pbz * 8 + szb * 4 + 2), 2, ls, true,
-                                 MODE == 1 && use32 ? &dc : nullptr);
+                                 MODE == 0 || use32 ? &dc : nullptr);
       }
     }
     uint32_t code16 = (uint32_t)scls << (2 * s);
@@ -806,8 +808,8 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_SUB_MINB : PX_CLASSIFY64_M
   if (lane == 0 && stw) atomicOr(&a.res->status, stw);
 }
 
-// Mixed form: a voxel's decision from its sub-block centre's value dc, when the
-// SDF's Lipschitz bound settles it (0 outside, 1 inside, 3 undecided); (ox, oy,
+// A voxel's decision from its sub-block centre's value dc, when the SDF's Lipschitz
+// bound settles it (0 outside, 1 inside, 3 undecided); (ox, oy,
 // oz) is the voxel's offset in the sub-block, 0..3 per axis.
 __device__ __forceinline__ int lip_decide(const OpDev* O, Iv dc, int ox, int oy, int oz) {
   const int k = (ox == 0 || ox == 3) + (oy == 0 || oy == 3) + (oz == 0 || oz == 3);  // axes at 1.5 voxels
@@ -824,6 +826,7 @@ __device__ __forceinline__ int lip_decide(const OpDev* O, Iv dc, int ox, int oy,
 template <int MODE, int G0, int G1>
 __global__ void __launch_bounds__(256, MODE == 1 ? PX_VOXEL_MINB : PX_CLASSIFY64_MINB) voxel_kernel(FoldArgs a) {
   pdl_prologue();
+  __shared__ uint8_t s_open[MODE == 0 ? 8 : 1][64];  // float64 form: the voxels of a warp's sub-block to evaluate
   const int lane = threadIdx.x & 31;
   LaneStats ls = {a.res};
 #pragma unroll 1
@@ -896,13 +899,42 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_VOXEL_MINB : PX_CLASSIFY64
         }
       }
       m = (unsigned long long)__reduce_or_sync(FULLMASK, lo) | ((unsigned long long)__reduce_or_sync(FULLMASK, hi) << 32);
+    } else if (MODE == 0) {
+      // the float64 form, bound by the FP64 pipe (1/64 of the FP32 rate): the voxels the centre's
+      // value leaves undecided (47 of 64 on average), gathered so that half a sub-block or less
+      // takes one evaluation instead of two.  Penthouse at 40 voxels per metre: every voxel
+      // 890 us, undecided ones in place 731, gathered 634
+      uint32_t in[2], open[2];
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        const int lip = a.validate ? 3 : lip_decide(V, dcen, lane & 3, (lane >> 2) & 3, 2 * r + (lane >> 4));
+        in[r] = __ballot_sync(FULLMASK, lip == 1);
+        open[r] = __ballot_sync(FULLMASK, lip == 3);
+        if (lip == 3) s_open[threadIdx.x >> 5][(r ? __popc(open[0]) : 0) + __popc(open[r] & ((1u << lane) - 1u))] = (uint8_t)(r * 32 + lane);
+      }
+      __syncwarp();
+      const int n_open = __popc(open[0]) + __popc(open[1]);
+      uint32_t lo = 0, hi = 0;
+#pragma unroll 1
+      for (int i = lane; i < n_open; i += 32) {
+        const int e = s_open[threadIdx.x >> 5][i];
+        const int lx = sxo + (e & 3), lyv = syo + ((e >> 2) & 3), lz = szo + (e >> 4);
+        if (eval_decide<MODE>(a, V, code, clen, use32, bo, (float)lx, (float)lyv, (float)lz, (float)(vbx * 8 + lx) + 0.5f,
+                              (float)(vby * 8 + lyv) + 0.5f, (float)(vbz * 8 + lz) + 0.5f, 0, ls) == 1) {
+          if (e < 32) lo |= 1u << e;
+          else hi |= 1u << (e - 32);
+        }
+      }
+      __syncwarp();
+      m = (unsigned long long)(in[0] | __reduce_or_sync(FULLMASK, lo)) |
+          ((unsigned long long)(in[1] | __reduce_or_sync(FULLMASK, hi)) << 32);
     } else {
       uint32_t bal[2];
 #pragma unroll
       for (int r = 0; r < 2; r++) {
         const int e = r * 32 + lane;
         const int lx = sxo + (e & 3), lyv = syo + ((e >> 2) & 3), lz = szo + (e >> 4);
-        const int lipd = MODE == 1 && use32 ? lip_decide(V, dcen, e & 3, (e >> 2) & 3, e >> 4) : 3;
+        const int lipd = use32 ? lip_decide(V, dcen, e & 3, (e >> 2) & 3, e >> 4) : 3;
         int inside = lipd;
         if (lipd == 3 || a.validate) {
           inside = eval_decide<MODE>(a, V, code, clen, use32, bo, (float)lx, (float)lyv, (float)lz,
