@@ -134,7 +134,7 @@ int px_set_derive_on_build(px_world* w, uint32_t max_bricks);
    the reference (GpuWorld.ts:90-101 computes these with its world); this entry
    point exists for callers that must not allocate device memory once they run
    (fixed device budgets, frame loops): it allocates nothing and uses a fixed
-   scratch area of 2 MiB + 256 bytes inside the library, which limits
+   scratch area of 2 MiB inside the library, which limits
    n_pool_bricks to PX_NOALLOC_MAX_POOL_BRICKS (larger: PX_E_TOO_LARGE, no GPU
    work).  The first call on each device looks up that area, with the device
    current; make it before any stream capture on that device, and do not call
