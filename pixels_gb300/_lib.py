@@ -149,8 +149,9 @@ def world_destroy(h):
 
 
 def submit_ops(h, ir: bytes):
-    buf = ctypes.create_string_buffer(ir, len(ir))
-    _check(h, load().px_submit_ops(h, buf, len(ir)))
+    if not isinstance(ir, bytes):  # read in place when immutable
+        ir = bytes(ir)
+    _check(h, load().px_submit_ops(h, ir, len(ir)))
 
 
 def build(h, mode: int, stream: int = 0):

@@ -136,6 +136,20 @@ __device__ __forceinline__ bool box_overlaps_tile(uint2 b, int tx, int ty, int t
   return x0 <= tx * 4 + 3 && x1 >= tx * 4 && y0 <= ty * 4 + 3 && y1 >= ty * 4 && z0 <= tz * 4 + 3 && z1 >= tz * 4;
 }
 
+// The chunk order's entries (ChunkFill), one op per warp, by the blocks of a cull launch
+// after its first n_tile_blocks.
+__device__ __forceinline__ void fill_chunks(const ChunkFill& f, int n_ops, int block) {
+  const int i = block * 8 + (int)(threadIdx.x >> 5);
+  if (i >= n_ops) return;
+  const unsigned long long base = f.ops[i].pair_base, end = i + 1 < n_ops ? f.ops[i + 1].pair_base : f.n_pairs;
+  const uint32_t c0 = (uint32_t)((base + 31) / 32), c1 = (uint32_t)((end + 31) / 32);
+  uint2* dst = f.order + f.dst[i];
+  for (uint32_t c = c0 + (threadIdx.x & 31u); c < c1; c += 32) {
+    const bool whole = (unsigned long long)c * 32 + 32 <= end || end >= f.n_pairs;
+    dst[c - c0] = make_uint2(c, (uint32_t)i | (whole ? 0x80000000u : 0u));
+  }
+}
+
 // The op boxes are followed by one union box per 32 consecutive ops: a warp
 // tests the 32-op groups first and only the ops of groups that overlap its
 // tile (a two-level culling hierarchy; scene ops come object by object, so
@@ -146,8 +160,13 @@ __device__ __forceinline__ bool box_overlaps_tile(uint2 b, int tx, int ty, int t
 // order; tile_off / tile_cnt locate them.
 __global__ void __launch_bounds__(256) cull_kernel(const uint2* __restrict__ boxes, int n_ops, int TX, int TY, int TZ,
                                                    uint32_t* tile_cnt, uint32_t* tile_off, uint32_t* tile_ops,
-                                                   uint2* tile_boxes, uint32_t* counter) {
+                                                   uint2* tile_boxes, uint32_t* counter, int n_tile_blocks,
+                                                   ChunkFill fill) {
   pdl_prologue();
+  if ((int)blockIdx.x >= n_tile_blocks) {
+    fill_chunks(fill, n_ops, (int)blockIdx.x - n_tile_blocks);
+    return;
+  }
   __shared__ uint32_t s_cnt[8], s_base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n_tiles = TX * TY * TZ;
@@ -218,8 +237,13 @@ __global__ void __launch_bounds__(256) cull_kernel(const uint2* __restrict__ box
 // order from it.  W: words of the bit set (ops / 32, rounded up).
 __global__ void __launch_bounds__(256) cull_sorted_kernel(const uint2* __restrict__ boxes, int n_ops, int TX, int TY,
                                                           int TZ, int W, uint32_t* tile_cnt, uint32_t* tile_off,
-                                                          uint32_t* tile_ops, uint2* tile_boxes, uint32_t* counter) {
+                                                          uint32_t* tile_ops, uint2* tile_boxes, uint32_t* counter,
+                                                          int n_tile_blocks, ChunkFill fill) {
   pdl_prologue();
+  if ((int)blockIdx.x >= n_tile_blocks) {
+    fill_chunks(fill, n_ops, (int)blockIdx.x - n_tile_blocks);
+    return;
+  }
   extern __shared__ uint32_t s_bits[];  // [8][W]
   __shared__ uint32_t s_cnt[8], s_base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -295,15 +319,17 @@ __global__ void __launch_bounds__(256) cull_sorted_kernel(const uint2* __restric
 }
 
 void launch_cull(const uint2* boxes, int n_ops, int TX, int TY, int TZ, uint32_t* tile_cnt, uint32_t* tile_off,
-                 uint32_t* tile_ops, uint2* tile_boxes, uint32_t* counter, bool sorted, cudaStream_t s) {
-  const int n_tiles = TX * TY * TZ;
+                 uint32_t* tile_ops, uint2* tile_boxes, uint32_t* counter, bool sorted, const ChunkFill& fill,
+                 cudaStream_t s) {
+  const int n_tiles = TX * TY * TZ, n_tile_blocks = (n_tiles + 7) / 8;
   const int W = (n_ops + 31) / 32;
+  const dim3 grid(n_tile_blocks + (fill.dst ? (n_ops + 7) / 8 : 0));
   if (sorted)
-    launch_pdl(cull_sorted_kernel, dim3((n_tiles + 7) / 8), dim3(256), (size_t)8 * W * 4, s, boxes, n_ops, TX, TY, TZ,
-               W, tile_cnt, tile_off, tile_ops, tile_boxes, counter);
+    launch_pdl(cull_sorted_kernel, grid, dim3(256), (size_t)8 * W * 4, s, boxes, n_ops, TX, TY, TZ, W, tile_cnt, tile_off,
+               tile_ops, tile_boxes, counter, n_tile_blocks, fill);
   else
-    launch_pdl(cull_kernel, dim3((n_tiles + 7) / 8), dim3(256), 0, s, boxes, n_ops, TX, TY, TZ, tile_cnt, tile_off,
-               tile_ops, tile_boxes, counter);
+    launch_pdl(cull_kernel, grid, dim3(256), 0, s, boxes, n_ops, TX, TY, TZ, tile_cnt, tile_off, tile_ops, tile_boxes,
+               counter, n_tile_blocks, fill);
 }
 
 // ---------------------------------------------------------------------------

@@ -58,6 +58,37 @@ struct DefaultInitAlloc : std::allocator<T> {
 template <class T>
 using hvec = std::vector<T, DefaultInitAlloc<T>>;
 
+// What the host needs of each op to lay out a build, apart from its 384-byte record: its
+// (op, brick) pairs, relative cost and work classes (a pass over these stays in cache).
+struct OpLite {
+  uint32_t n_pairs;
+  float cost;
+  uint8_t vclass, vq_class;
+};
+
+// One contiguous range of a submitted op list, converted by one host thread:
+// offsets into its own arrays, rebased when the ranges are merged in order.
+struct SubmitChunk {
+  std::vector<OpDev> ops;
+  std::vector<OpLite> lite;
+  std::vector<uint2> boxes, code;
+  std::vector<double> xparams;     // expanded polygon records (device float64 layout)
+  std::vector<uint32_t> code32;    // float32 parameter offset per instruction
+  std::vector<float2> bases, p32;
+  std::vector<uint32_t> xfix;      // instructions whose parameter offset is a polygon record
+  uint64_t n_pairs = 0, n_tile_pairs = 0;        // the range's (op, brick) pairs and tile-list entries
+  std::vector<uint32_t> painted64, painted32;    // its painted ops (range-local indices)
+  int rc = PX_OK;
+  std::string err;
+  void clear() {  // (the arrays keep their room for the next list)
+    ops.clear(); lite.clear(); boxes.clear(); code.clear(); xparams.clear(); code32.clear(); bases.clear(); p32.clear();
+    xfix.clear(); painted64.clear(); painted32.clear();
+    n_pairs = n_tile_pairs = 0;
+    rc = PX_OK;
+    err.clear();
+  }
+};
+
 // one host-to-device copy of a build's op tables
 struct Upload {
   void* dst;
@@ -94,7 +125,13 @@ struct px_world {
   hvec<double> last_params;
   bool ops_resident = false;   // the device op tables already hold `ops`
   hvec<uint2> boxes;
-  std::vector<uint2> h_boxes;  // boxes + 32-op group boxes as uploaded
+  hvec<OpLite> lite, last_lite;
+  std::vector<SubmitChunk> chunks;  // conversion workspace of px_submit_ops, kept between lists
+  // the cull kernels' table as uploaded (cull_tables) and its scratch
+  hvec<uint2> h_boxes, h_groups;
+  hvec<uint32_t> h_sort[4];
+  size_t n_cull = 0;            // its entries
+  bool cull_ready = false;      // it holds the queued ops
   hvec<uint2> code;
   hvec<double> params;
   hvec<uint32_t> code32, last_code32;   // per instruction: float32 parameter offset
@@ -105,7 +142,6 @@ struct px_world {
 
   // per-build device scratch
   DevBuf d_ops, d_boxes, d_code, d_params, d_code32, d_p32, d_bases;
-  std::vector<uint32_t> h_cull_order;  // the ops along a Morton curve of their boxes (cull_sorted_kernel)
   bool cull_sorted = false;
   DevBuf tile_cnt, tile_off, tile_ops, tile_boxes;
   DevBuf evt, fsrc, pos, etype, ew, depth, tree, replay_tmp;
@@ -114,7 +150,8 @@ struct px_world {
   uint32_t rescue_cap = 1u << 16;  // voxels a build may leave to float64 (grown on overflow)
   DevBuf rescue;
   DevBuf chunk_op, pcode, psub, pmask, chunk_counter, vitems, pitems;
-  std::vector<uint32_t> h_chunk_op;  // the chunks in classify order: (chunk, op of its first pair | single-op bit)
+  DevBuf chunk_dst;                  // per op: where its chunks begin in the classify order
+  hvec<uint32_t> h_chunk_dst;
   std::vector<Upload> h_uploads;     // the op-table copies of the build being enqueued
   std::vector<uint32_t> h_painted;  // the build's painted ops, float64-only ones first
   // totals of the queued op list, summed as it is converted: (op, brick) pairs,
@@ -124,7 +161,6 @@ struct px_world {
     std::vector<uint32_t> painted64, painted32;
     void clear() { pairs = tile_pairs = 0; painted64.clear(); painted32.clear(); }
   } q, last_q;
-  std::vector<uint8_t> h_op_bucket;  // per op: cost bucket (0..63) of one evaluation
   uint8_t class_order[VCLASSES] = {0};  // sub-block class order of the resident ops
   uint8_t vclass_order[VQ_CLASSES] = {0};  // voxel class order (each group on its own)
   uint32_t vq_nonempty = 0;                // bit g: voxel group g has ops
@@ -253,7 +289,9 @@ inline float2 enc(double v, double pad = 0.0) { return make_float2(rd32(v - pad)
 // but the first, C32_SKIP.
 void rotation_runs(const uint32_t* code, uint32_t n, std::vector<uint32_t>& flag) {
   auto is_rot = [](uint32_t op) { return op == OP_ROT_X || op == OP_ROT_Y || op == OP_ROT_Z; };
-  std::vector<int> close(n, -1), stack;
+  static thread_local std::vector<int> close, stack;  // (no allocation per op)
+  close.assign(n, -1);
+  stack.clear();
   for (uint32_t i = 0; i < n; i++) {
     const uint32_t op = code[2 * i] & 0xffu;
     if (is_rot(op)) stack.push_back((int)i);
@@ -330,7 +368,8 @@ bool compose_rotations(const uint32_t* code, uint32_t i, uint32_t k, const doubl
 // lp[LP_FORM] = 0.  A stage is one rotation, or a run composed by rotation_runs.
 void lean_program(const uint32_t* code, uint32_t n, uint8_t lp[8]) {
   if (n > 40) return;
-  std::vector<uint32_t> flag(n, 0u);
+  static thread_local std::vector<uint32_t> flag;
+  flag.assign(n, 0u);
   rotation_runs(code, n, flag);
   auto op_at = [&](uint32_t i) { return code[2 * i] & 0xffu; };
   auto is_prim = [&](uint32_t i) { return i < n && op_at(i) >= OP_BOX && op_at(i) < OP_ROT_X; };
@@ -427,7 +466,8 @@ bool convert32(const uint32_t* code, uint32_t n, const double* P, const double A
     }
   };
   // runs of rotations whose ends follow each other: composed into one affine map
-  std::vector<uint32_t> flag(n, 0u);
+  static thread_local std::vector<uint32_t> flag;
+  flag.assign(n, 0u);
   rotation_runs(code, n, flag);
   for (uint32_t i = 0; i < n; i++) {
     uint32_t op = code[2 * i] & 0xffu, cnt = code[2 * i] >> 8;
@@ -849,7 +889,7 @@ void px_world_destroy(px_world* w) {
                     &w->d_p32, &w->d_bases, &w->tile_cnt,
                     &w->tile_off, &w->tile_ops, &w->evt, &w->fsrc, &w->pos, &w->etype,
                     &w->ew, &w->replay_tmp, &w->depth, &w->tree, &w->staging, &w->touched,
-                    &w->stage_cell, &w->stage_src, &w->chunk_op, &w->pcode, &w->psub, &w->pmask,
+                    &w->stage_cell, &w->stage_src, &w->chunk_op, &w->chunk_dst, &w->pcode, &w->psub, &w->pmask,
                     &w->chunk_counter, &w->vitems, &w->work_counter, &w->res, &w->opaque,
                     &w->udens, &w->super_counts, &w->density, &w->paint_items, &w->pvals, &w->tile_boxes, &w->bmark, &w->work, &w->pitems,
                     &w->free_list, &w->rescue};
@@ -955,21 +995,6 @@ float op_cost(const uint32_t* code, uint32_t code_len, uint32_t flags) {
   if (flags & OPF_CONTAINS) c *= 0.5f;
   return c;
 }
-
-// One contiguous range of a submitted op list, converted by one host thread:
-// offsets into its own arrays, rebased when the ranges are merged in order.
-struct SubmitChunk {
-  std::vector<OpDev> ops;
-  std::vector<uint2> boxes, code;
-  std::vector<double> xparams;     // expanded polygon records (device float64 layout)
-  std::vector<uint32_t> code32;    // float32 parameter offset per instruction
-  std::vector<float2> bases, p32;
-  std::vector<uint32_t> xfix;      // instructions whose parameter offset is a polygon record
-  uint64_t n_pairs = 0, n_tile_pairs = 0;        // the range's (op, brick) pairs and tile-list entries
-  std::vector<uint32_t> painted64, painted32;    // its painted ops (range-local indices)
-  int rc = PX_OK;
-  std::string err;
-};
 
 int chunk_fail(SubmitChunk& out, int code, const char* fmt, ...) {
   char buf[512];
@@ -1241,6 +1266,7 @@ int convert_ops(const px_world* w, const IrOp* iops, size_t i0, size_t i1, const
       if (d.kind != KIND_CARVE && d.paint_kind != PK_CONST)
         (d.paint32_off == NO_SLOT ? out.painted64 : out.painted32).push_back((uint32_t)out.ops.size());
     }
+    out.lite.push_back({(uint32_t)(out.n_pairs - d.pair_base), d.cost, (uint8_t)(d.vclass & (VCLASSES - 1)), (uint8_t)d.vq_class});
     out.ops.push_back(d);
     out.boxes.push_back(box);
   }
@@ -1257,81 +1283,169 @@ class HostPool {
     return *p;
   }
   int size() const { return (int)workers_.size() + 1; }
-  // run f(k) for k in [0, n) on the pool and the calling thread
+  // run f(k) for k in [0, n) on the pool and the calling thread; returns once every f(k)
+  // has, without waiting for workers that woke too late to take one
   void run(int n, const std::function<void(int)>& f) {
     if (n <= 1 || workers_.empty()) {
       for (int k = 0; k < n; k++) f(k);
       return;
     }
     std::lock_guard<std::mutex> one_job(run_mu_);  // callers on other threads wait their turn
-    job_ = &f;
-    n_ = n;
-    next_.store(0);
-    done_.store(0);
+    const uint32_t gen = (uint32_t)(ticket_.load(std::memory_order_relaxed) >> 32) + 1;
+    Job& j = job_[gen & 1];  // (the last job's slot stays as it was for a worker that still looks at it)
+    j.f.store(&f, std::memory_order_relaxed);
+    j.n.store((uint32_t)n, std::memory_order_relaxed);
+    done_.store(0, std::memory_order_relaxed);
     {
       std::lock_guard<std::mutex> g(mu_);
-      gen_.fetch_add(1, std::memory_order_release);
+      ticket_.store((uint64_t)gen << 32, std::memory_order_release);
     }
     cv_.notify_all();
     work();
-    // the workers' part: spin briefly, then sleep until the last one reports
-    const int want = (int)workers_.size();
+    // jobs still running on the workers: spin briefly, then sleep until the last one reports
     const auto t0 = std::chrono::steady_clock::now();
-    while (done_.load(std::memory_order_acquire) != want) {
+    while (done_.load(std::memory_order_acquire) != (uint32_t)n) {
       if (std::chrono::steady_clock::now() - t0 > std::chrono::microseconds(200)) {
         std::unique_lock<std::mutex> g(mu_);
-        done_cv_.wait(g, [&] { return done_.load(std::memory_order_acquire) == want; });
+        done_cv_.wait(g, [&] { return done_.load(std::memory_order_acquire) == (uint32_t)n; });
         break;
       }
     }
-    job_ = nullptr;
   }
 
  private:
+  struct Job {
+    std::atomic<const std::function<void(int)>*> f{nullptr};
+    std::atomic<uint32_t> n{0};
+  };
   HostPool() {
     unsigned hc = std::thread::hardware_concurrency();
     int n = (int)std::min<unsigned>(hc > 1 ? hc - 1 : 0, 15);
     for (int i = 0; i < n; i++) workers_.emplace_back([this] { loop(); });
     for (auto& t : workers_) t.detach();
   }
+  // Take the current job's indices one by one.  ticket_ holds (generation, next index): an
+  // index is taken by compare-and-swap, so one of a job that has ended is never run, and a job
+  // whose index was taken cannot end before it is done.
   void work() {
     for (;;) {
-      const int k = next_.fetch_add(1);
-      if (k >= n_) break;
-      (*job_)(k);
+      uint64_t t = ticket_.load(std::memory_order_acquire);
+      Job& j = job_[(t >> 32) & 1];
+      const std::function<void(int)>* f = j.f.load(std::memory_order_relaxed);
+      const uint32_t n = j.n.load(std::memory_order_relaxed), k = (uint32_t)t;
+      if (k >= n) {
+        if (ticket_.load(std::memory_order_acquire) == t) break;
+        continue;  // the next job began meanwhile
+      }
+      if (!ticket_.compare_exchange_weak(t, t + 1, std::memory_order_acq_rel)) continue;
+      (*f)((int)k);
+      if (done_.fetch_add(1, std::memory_order_acq_rel) + 1 == n) {
+        std::lock_guard<std::mutex> g(mu_);
+        done_cv_.notify_one();
+      }
     }
   }
   void loop() {
-    uint64_t seen = 0;
+    uint64_t seen = 0;  // the generation last worked on
     for (;;) {
       // spin up to 50 us for the next job (the jobs of one submit follow each
       // other within microseconds), then sleep: longer spinning would take the
       // cores from the caller's other threads between submits
       const auto t0 = std::chrono::steady_clock::now();
       uint32_t i = 0;
-      while (gen_.load(std::memory_order_acquire) == seen) {
+      while ((ticket_.load(std::memory_order_acquire) >> 32) == seen) {
         if ((++i & 255u) == 0 && std::chrono::steady_clock::now() - t0 > std::chrono::microseconds(50)) {
           std::unique_lock<std::mutex> g(mu_);
-          cv_.wait(g, [&] { return gen_.load(std::memory_order_acquire) != seen; });
+          cv_.wait(g, [&] { return (ticket_.load(std::memory_order_acquire) >> 32) != seen; });
           break;
         }
       }
-      seen = gen_.load(std::memory_order_acquire);
+      seen = ticket_.load(std::memory_order_acquire) >> 32;
       work();
-      if (done_.fetch_add(1, std::memory_order_acq_rel) + 1 == (int)workers_.size()) {
-        std::lock_guard<std::mutex> g(mu_);
-        done_cv_.notify_one();
-      }
     }
   }
   std::vector<std::thread> workers_;
   std::mutex run_mu_, mu_;
   std::condition_variable cv_, done_cv_;
-  const std::function<void(int)>* job_ = nullptr;
-  int n_ = 0;
-  std::atomic<int> next_{0}, done_{0};
-  std::atomic<uint64_t> gen_{0};
+  Job job_[2];
+  std::atomic<uint64_t> ticket_{0};  // generation << 32 | next index
+  std::atomic<uint32_t> done_{0};    // indices of the current job that have returned
 };
+
+// The cull kernels' table from the op boxes in h_boxes[0 .. n_ops): after them the union box of
+// every 32 ops of the culling order, then that order, two per entry, where it is not the op
+// order: along a Morton curve of the boxes' centres (in 4-brick tiles), taken where its groups
+// cover less than half the tiles the op order's do -- scattered ops (cull_sorted_kernel's bit
+// set costs more on compact scenes).
+void cull_tables(px_world* w, int n_ops) {
+  const int n_groups = (n_ops + 31) / 32;
+  w->h_boxes.resize((size_t)n_ops + n_groups + (n_ops + 1) / 2);
+  const uint2* B = w->h_boxes.data();
+  // the union boxes of 32 ops of an order (none: the op order), and the tiles they cover in all
+  // (the group tests a tile passes grow with it)
+  auto group_boxes = [&](const uint32_t* ord, uint2* gb) {
+    uint64_t vol = 0;
+    for (int g = 0; g < n_groups; g++) {
+      uint32_t lo[3] = {1023, 1023, 1023}, hi[3] = {0, 0, 0};
+      bool any = false;
+      for (int k = g * 32; k < n_ops && k < g * 32 + 32; k++) {
+        const uint2 b = B[ord ? ord[k] : (uint32_t)k];
+        if (b.x >> 30) continue;
+        any = true;
+        for (int a = 0; a < 3; a++) {
+          lo[a] = std::min(lo[a], (b.x >> (10 * a)) & 1023u);
+          hi[a] = std::max(hi[a], (b.y >> (10 * a)) & 1023u);
+        }
+      }
+      gb[g] = any ? make_uint2(lo[0] | (lo[1] << 10) | (lo[2] << 20), hi[0] | (hi[1] << 10) | (hi[2] << 20))
+                  : make_uint2(3u << 30, 0u);
+      if (any) vol += (uint64_t)(hi[0] / 4 - lo[0] / 4 + 1) * (hi[1] / 4 - lo[1] / 4 + 1) * (hi[2] / 4 - lo[2] / 4 + 1);
+    }
+    return vol;
+  };
+  uint2* const groups = w->h_boxes.data() + n_ops;
+  const uint64_t vol_seq = group_boxes(nullptr, groups);
+  w->cull_sorted = false;
+  w->n_cull = (size_t)n_ops + n_groups;
+  if (n_ops > CULL_SORTED_MAX_OPS || n_groups <= 1) return;
+  auto spread = [](uint32_t v) {  // 8 bits -> every third bit
+    v = (v | (v << 8)) & 0x00f00fu;
+    v = (v | (v << 4)) & 0x0c30c3u;
+    return (v | (v << 2)) & 0x249249u;
+  };
+  for (auto& v : w->h_sort) v.resize(n_ops);
+  uint32_t *key = w->h_sort[0].data(), *ord = w->h_sort[1].data(), *key2 = w->h_sort[2].data(), *ord2 = w->h_sort[3].data();
+  for (int i = 0; i < n_ops; i++) {
+    const uint2 b = B[i];
+    ord[i] = (uint32_t)i;
+    key[i] = 0xffffffu;  // no bricks: last (the far corner's key is the same: the order stays stable)
+    if (b.x >> 30) continue;
+    uint32_t c[3];
+    for (int a = 0; a < 3; a++) c[a] = ((((b.x >> (10 * a)) & 1023u) + ((b.y >> (10 * a)) & 1023u)) >> 3) & 255u;
+    key[i] = spread(c[0]) | (spread(c[1]) << 1) | (spread(c[2]) << 2);
+  }
+  for (int shift = 0; shift < 24; shift += 8) {  // a stable radix sort on the 24-bit keys
+    uint32_t at[256] = {0};
+    for (int i = 0; i < n_ops; i++) at[(key[i] >> shift) & 255u]++;
+    for (uint32_t d = 0, sum = 0; d < 256; d++) {
+      const uint32_t c = at[d];
+      at[d] = sum;
+      sum += c;
+    }
+    for (int i = 0; i < n_ops; i++) {
+      const uint32_t t = at[(key[i] >> shift) & 255u]++;
+      key2[t] = key[i];
+      ord2[t] = ord[i];
+    }
+    std::swap(key, key2);
+    std::swap(ord, ord2);
+  }
+  w->h_groups.resize(n_groups);
+  if (2 * group_boxes(ord, w->h_groups.data()) >= vol_seq) return;
+  w->cull_sorted = true;
+  std::memcpy(groups, w->h_groups.data(), sizeof(uint2) * n_groups);
+  for (int k = 0; k < n_ops; k += 2) w->h_boxes[w->n_cull++] = make_uint2(ord[k], k + 1 < n_ops ? ord[k + 1] : 0u);
+}
 
 // The build scratch that scales with the (op, brick) pairs P, the tile-list
 // entries, the paint slots, the touched bricks, the allocator events E_max and
@@ -1381,7 +1495,7 @@ int reserve_build_scratch(px_world* w, uint64_t P, uint32_t max_ops) {
     if ((rc0 = ensure(w, w->d_ops, sizeof(OpDev) * n)) || (rc0 = ensure(w, w->d_boxes, sizeof(uint2) * (n + (n + 31) / 32 + (n + 1) / 2))) ||
         (rc0 = ensure(w, w->d_code, sizeof(uint2) * n)) || (rc0 = ensure(w, w->d_params, sizeof(double) * 16 * n)) ||
         (rc0 = ensure(w, w->d_code32, sizeof(uint32_t) * n)) || (rc0 = ensure(w, w->d_p32, sizeof(float2) * 16 * n)) ||
-        (rc0 = ensure(w, w->d_bases, sizeof(float2) * 192 * n)))
+        (rc0 = ensure(w, w->d_bases, sizeof(float2) * 192 * n)) || (rc0 = ensure(w, w->chunk_dst, 4 * n)))
       return rc0;
     const void* after[7] = {w->d_ops.p, w->d_boxes.p, w->d_code.p, w->d_params.p, w->d_code32.p, w->d_p32.p, w->d_bases.p};
     for (int k = 0; k < 7; k++)
@@ -1534,13 +1648,17 @@ static int submit_ops_impl(px_world* w, const void* ir, size_t bytes) {
   // (few short programs -- a serving step's edits -- are not worth waking the pool for)
   const bool few = n_ops < 64 || (n_ops < 512 && n_code < 1024);
   const int n_chunks = few ? 1 : (int)std::min<size_t>((size_t)pool.size() * 4, n_ops / 32);
-  std::vector<SubmitChunk> chunks(n_chunks);
+  std::vector<SubmitChunk>& chunks = w->chunks;
+  if (chunks.size() < (size_t)n_chunks) chunks.resize(n_chunks);
+  const bool first_list = w->ops.empty();
+  w->cull_ready = false;
   pool.run(n_chunks, [&](int k) {
     const size_t i0 = n_ops * k / n_chunks, i1 = n_ops * (k + 1) / n_chunks;
+    chunks[k].clear();
     convert_ops(w, iops, i0, i1, code, n_code, Pp, n_params, param_base, chunks[k]);
   });
-  for (auto& c : chunks)
-    if (c.rc != PX_OK) return fail(w, c.rc, "%s", c.err.c_str());
+  for (int k = 0; k < n_chunks; k++)
+    if (chunks[k].rc != PX_OK) return fail(w, chunks[k].rc, "%s", chunks[k].err.c_str());
   // every range's place in the world's arrays, then all ranges rebased and
   // copied at once (the IR's own parameters as one more job)
   struct Place {
@@ -1568,13 +1686,27 @@ static int submit_ops_impl(px_world* w, const void* ir, size_t bytes) {
   w->p32.resize(end.p32);
   w->bases.resize(end.bases);
   w->ops.resize(end.ops);
+  w->lite.resize(end.ops);
   w->boxes.resize(end.ops);
   w->params.resize(end.xp);
   auto merge = [&](int k) {
-    if (k == n_chunks) {
+    if (k == 0) {  // the cull kernels' table, the longest of these jobs (a list appended to another: at the build)
+      if (!first_list) return;
+      w->h_boxes.resize(n_ops);
+      size_t at0 = 0;
+      for (int q = 0; q < n_chunks; q++) {
+        const auto& b = chunks[q].boxes;
+        if (!b.empty()) std::memcpy(w->h_boxes.data() + at0, b.data(), b.size() * sizeof(uint2));
+        at0 += b.size();
+      }
+      cull_tables(w, (int)n_ops);
+      return;
+    }
+    if (k == 1) {
       if (n_params) std::memcpy(w->params.data() + param_base, Pp, n_params * sizeof(double));
       return;
     }
+    k -= 2;
     SubmitChunk& c = chunks[k];
     const Place& pl = at[k];
     for (uint32_t i : c.xfix) c.code[i].y += (uint32_t)pl.xp;
@@ -1595,15 +1727,16 @@ static int submit_ops_impl(px_world* w, const void* ir, size_t bytes) {
     put(w->p32, pl.p32, c.p32);
     put(w->bases, pl.bases, c.bases);
     put(w->ops, pl.ops, c.ops);
+    put(w->lite, pl.ops, c.lite);
     put(w->boxes, pl.ops, c.boxes);
     put(w->params, pl.xp, c.xparams);
   };
   if (n_chunks > 1) {
-    pool.run(n_chunks + 1, merge);
+    pool.run(n_chunks + 2, merge);
   } else {  // a small list: no threads
-    merge(0);
-    merge(1);
+    for (int k = 0; k < 3; k++) merge(k);
   }
+  w->cull_ready = first_list;
   return PX_OK;
 }
 
@@ -1723,20 +1856,20 @@ static int build_enqueue_impl(px_world* w, int mode, void* stream) {
 
   // scratch (a reallocated op table loses its resident copy)
   const void* op_bufs_before[9] = {w->d_ops.p, w->d_boxes.p, w->d_code.p, w->d_params.p, w->d_code32.p,
-                                   w->d_p32.p, w->d_bases.p, w->chunk_op.p, w->chunk_op.p};
+                                   w->d_p32.p, w->d_bases.p, w->chunk_op.p, w->chunk_dst.p};
   if ((rc = ensure(w, w->d_ops, sizeof(OpDev) * (size_t)n_ops)) ||
       (rc = ensure(w, w->d_boxes, sizeof(uint2) * ((size_t)n_ops + (n_ops + 31) / 32 + (n_ops + 1) / 2))) ||
       (rc = ensure(w, w->d_code, sizeof(uint2) * w->code.size())) ||
       (rc = ensure(w, w->d_params, sizeof(double) * w->params.size())) ||
       (rc = ensure(w, w->d_code32, sizeof(uint32_t) * w->code32.size())) ||
       (rc = ensure(w, w->d_p32, sizeof(float2) * w->p32.size())) ||
-      (rc = ensure(w, w->d_bases, sizeof(float2) * w->bases.size())) ||
+      (rc = ensure(w, w->d_bases, sizeof(float2) * w->bases.size())) || (rc = ensure(w, w->chunk_dst, 4 * (size_t)n_ops)) ||
       (rc = ensure_pair_scratch(w, P, tile_pairs, n_slots, touched_bound, E_max, stage_cap)))
     return rc;
   const uint32_t H_max = H;
   {
     const void* after[9] = {w->d_ops.p, w->d_boxes.p, w->d_code.p, w->d_params.p, w->d_code32.p,
-                            w->d_p32.p, w->d_bases.p, w->chunk_op.p, w->chunk_op.p};
+                            w->d_p32.p, w->d_bases.p, w->chunk_op.p, w->chunk_dst.p};
     for (int k = 0; k < 9; k++)
       if (after[k] != op_bufs_before[k]) w->ops_resident = false;
   }
@@ -1752,113 +1885,40 @@ static int build_enqueue_impl(px_world* w, int mode, void* stream) {
   ups.clear();
   if (upload) {
     ups.push_back({w->d_ops.p, w->ops.data(), sizeof(OpDev) * (size_t)n_ops});
-    {  // op boxes, then the union box of every 32 ops of the culling order (cull_kernel /
-       // cull_sorted_kernel), then that order: along a Morton curve of the boxes' centres
-       // (in 4-brick tiles) when the sorted kernel is used, else the op order itself
-      const int n_groups = (n_ops + 31) / 32;
-      // the union boxes of 32 ops of an order, and the tiles they cover in all (the
-      // group tests a tile passes grow with it)
-      auto group_boxes = [&](const std::vector<uint32_t>& ord, std::vector<uint2>& gb) {
-        uint64_t vol = 0;
-        gb.clear();
-        for (int g = 0; g < n_groups; g++) {
-          uint32_t lo[3] = {1023, 1023, 1023}, hi[3] = {0, 0, 0};
-          bool any = false;
-          for (int k = g * 32; k < n_ops && k < g * 32 + 32; k++) {
-            const uint2 b = w->boxes[ord[k]];
-            if (b.x >> 30) continue;
-            any = true;
-            for (int a = 0; a < 3; a++) {
-              lo[a] = std::min(lo[a], (b.x >> (10 * a)) & 1023u);
-              hi[a] = std::max(hi[a], (b.y >> (10 * a)) & 1023u);
-            }
-          }
-          gb.push_back(any ? make_uint2(lo[0] | (lo[1] << 10) | (lo[2] << 20), hi[0] | (hi[1] << 10) | (hi[2] << 20))
-                           : make_uint2(3u << 30, 0u));
-          if (any) vol += (uint64_t)(hi[0] / 4 - lo[0] / 4 + 1) * (hi[1] / 4 - lo[1] / 4 + 1) * (hi[2] / 4 - lo[2] / 4 + 1);
-        }
-        return vol;
-      };
-      std::vector<uint32_t>& ord = w->h_cull_order;
-      ord.resize(n_ops);
-      for (int i = 0; i < n_ops; i++) ord[i] = (uint32_t)i;
-      std::vector<uint2> gb_seq, gb_mc;
-      const uint64_t vol_seq = group_boxes(ord, gb_seq);
-      bool sorted = false;
-      if (n_ops <= CULL_SORTED_MAX_OPS && n_groups > 1) {
-        auto spread = [](uint32_t v) {  // 8 bits -> every third bit
-          uint32_t r = 0;
-          for (int k = 0; k < 8; k++) r |= ((v >> k) & 1u) << (3 * k);
-          return r;
-        };
-        std::vector<uint32_t> key(n_ops), mc(ord);
-        for (int i = 0; i < n_ops; i++) {
-          const uint2 b = w->boxes[i];
-          if (b.x >> 30) { key[i] = 0xffffffffu; continue; }  // no bricks: last
-          uint32_t c[3];
-          for (int a = 0; a < 3; a++) c[a] = ((((b.x >> (10 * a)) & 1023u) + ((b.y >> (10 * a)) & 1023u)) >> 3) & 255u;
-          key[i] = spread(c[0]) | (spread(c[1]) << 1) | (spread(c[2]) << 2);
-        }
-        std::stable_sort(mc.begin(), mc.end(), [&](uint32_t x, uint32_t y) { return key[x] < key[y]; });
-        // the spatial order where its groups cover less than half the tiles the op order's
-        // do: scattered ops (the sorted kernel's bit set costs more on compact scenes)
-        if (2 * group_boxes(mc, gb_mc) < vol_seq) {
-          sorted = true;
-          ord.swap(mc);
-        }
-      }
-      w->cull_sorted = sorted;
+    if (!w->cull_ready) {  // several lists were queued
       w->h_boxes.assign(w->boxes.begin(), w->boxes.end());
-      const std::vector<uint2>& gb = sorted ? gb_mc : gb_seq;
-      w->h_boxes.insert(w->h_boxes.end(), gb.begin(), gb.end());
-      if (sorted)  // the order, two per uint2
-        for (int k = 0; k < n_ops; k += 2)
-          w->h_boxes.push_back(make_uint2(ord[k], k + 1 < n_ops ? ord[k + 1] : 0u));
-      ups.push_back({w->d_boxes.p, w->h_boxes.data(), sizeof(uint2) * w->h_boxes.size()});
+      cull_tables(w, n_ops);
+      w->cull_ready = true;
     }
+    ups.push_back({w->d_boxes.p, w->h_boxes.data(), sizeof(uint2) * w->n_cull});
     ups.push_back({w->d_code.p, w->code.data(), sizeof(uint2) * w->code.size()});
     ups.push_back({w->d_params.p, w->params.data(), sizeof(double) * w->params.size()});
     ups.push_back({w->d_code32.p, w->code32.data(), sizeof(uint32_t) * w->code32.size()});
     ups.push_back({w->d_p32.p, w->p32.data(), sizeof(float2) * w->p32.size()});
     ups.push_back({w->d_bases.p, w->bases.data(), sizeof(float2) * w->bases.size()});
   }
-  // the build's counters and flags start at zero
-  ups.push_back({w->res.p, nullptr, sizeof(BuildResult)});
-  ups.push_back({w->work_counter.p, nullptr, 16});
-  ups.push_back({w->chunk_counter.p, nullptr, 1024});
-  ups.push_back({w->evt.p, nullptr, P});
-  ups.push_back({w->bmark.p, nullptr, 4 * ((w->ncells + 31) / 32)});
-  ups.push_back({w->replay_tmp.p, nullptr, replay_clear_bytes(P)});  // the replay's tickets and look-back flags
-  ups.push_back({w->tree.p, nullptr, tree_clear_bytes(E_max), 0x7f});  // min-tree levels 1 and 2, above every depth
-  if ((rc = issue_uploads(w, ups, s))) return rc;  // the op tables; the chunk order follows the cull launches
-
-  BuildResult* res = (BuildResult*)w->res.p;
-  launch_cull((const uint2*)w->d_boxes.p, n_ops, w->TX, w->TY, w->TZ, (uint32_t*)w->tile_cnt.p,
-              (uint32_t*)w->tile_off.p, (uint32_t*)w->tile_ops.p, (uint2*)w->tile_boxes.p,
-              (uint32_t*)w->chunk_counter.p + CULL_COUNTER, w->cull_sorted, s);
-  // the classify pass's chunk order, computed while the cull kernels run
+  // per class: the (op, brick) pairs (the queues' regions) and the costliest op
+  uint64_t per[VCLASSES] = {0}, vper[VQ_CLASSES] = {0};
+  float cc[VCLASSES] = {0.f}, cv[VQ_CLASSES] = {0.f};
+  for (const OpLite& o : w->lite) {
+    per[o.vclass] += o.n_pairs;
+    vper[o.vq_class] += o.n_pairs;
+    if (!o.n_pairs) continue;
+    cc[o.vclass] = std::max(cc[o.vclass], o.cost);
+    cv[o.vq_class] = std::max(cv[o.vq_class], o.cost);
+  }
   const size_t n_chunks = (P + 31) / 32;
   if (upload) {
-    // op of the first pair of every 32-pair chunk, then the order classify_kernel
-    // takes the chunks in: costliest ops first (a bucket sort, stable within a bucket)
-    w->h_chunk_op.resize(2 * n_chunks);
-    w->h_op_bucket.resize(n_ops);
-    float cc[VCLASSES] = {0.f}, cv[VQ_CLASSES] = {0.f};
-    for (int i = 0; i < n_ops; i++) {
-      const float c = w->ops[i].cost;
-      w->h_op_bucket[i] = (uint8_t)cost_bucket(c);
-      if (w->ops[i].bx0 <= w->ops[i].bx1) {
-        cc[w->ops[i].vclass] = std::max(cc[w->ops[i].vclass], c);
-        cv[w->ops[i].vq_class] = std::max(cv[w->ops[i].vq_class], c);
-      }
-    }
-    // op o owns the chunks whose first pair it holds: [ceil(base_o / 32), ceil(base_o+1 / 32));
-    // a chunk entry is (chunk, its first pair's op | bit 31 when all its pairs are that op's)
-    auto first_chunk = [&](int i) { return (uint32_t)((w->ops[i].pair_base + 31) / 32); };
+    // the order classify_kernel takes the 32-pair chunks in: costliest ops first (a bucket sort,
+    // stable within a bucket).  Op o owns the chunks whose first pair it holds, [ceil(base_o / 32),
+    // ceil(base_o+1 / 32)); the host places each op's run, the cull launch writes the entries
+    w->h_chunk_dst.resize(n_ops);
+    auto chunks_of = [&](uint64_t base, uint64_t end) { return (uint32_t)((end + 31) / 32 - (base + 31) / 32); };
     uint32_t bucket_n[64] = {0};
-    for (int i = 0; i < n_ops; i++) {
-      const uint32_t c0 = first_chunk(i), c1 = i + 1 < n_ops ? first_chunk(i + 1) : (uint32_t)n_chunks;
-      bucket_n[w->h_op_bucket[i]] += c1 - c0;
+    uint64_t base = 0;
+    for (const OpLite& o : w->lite) {
+      bucket_n[cost_bucket(o.cost)] += chunks_of(base, base + o.n_pairs);
+      base += o.n_pairs;
     }
     uint32_t at = 0;
     for (int b = 63; b >= 0; b--) {
@@ -1866,18 +1926,15 @@ static int build_enqueue_impl(px_world* w, int mode, void* stream) {
       bucket_n[b] = at;
       at += n;
     }
-    for (int i = 0; i < n_ops; i++) {  // each op's chunks, in order, at its bucket's next place
-      const uint32_t c0 = first_chunk(i), c1 = i + 1 < n_ops ? first_chunk(i + 1) : (uint32_t)n_chunks;
-      const uint64_t end = i + 1 < n_ops ? w->ops[i + 1].pair_base : P;  // the op's pairs end here
-      uint32_t* dst = w->h_chunk_op.data() + 2 * (size_t)bucket_n[w->h_op_bucket[i]];
-      for (uint32_t c = c0; c < c1; c++) {
-        *dst++ = c;
-        *dst++ = (uint32_t)i | ((uint64_t)c * 32 + 32 <= end || end >= P ? 0x80000000u : 0u);
-      }
-      bucket_n[w->h_op_bucket[i]] += c1 - c0;
+    base = 0;
+    for (int i = 0; i < n_ops; i++) {
+      const OpLite& o = w->lite[i];
+      uint32_t& next = bucket_n[cost_bucket(o.cost)];
+      w->h_chunk_dst[i] = next;
+      next += chunks_of(base, base + o.n_pairs);
+      base += o.n_pairs;
     }
-    ups.clear();
-    ups.push_back({w->chunk_op.p, w->h_chunk_op.data(), 8 * n_chunks});
+    ups.push_back({w->chunk_dst.p, w->h_chunk_dst.data(), 4 * (size_t)n_ops});
     // the sub-block and voxel passes take the classes costliest first
     int order[VCLASSES];
     for (int k = 0; k < VCLASSES; k++) order[k] = k;
@@ -1889,10 +1946,26 @@ static int build_enqueue_impl(px_world* w, int mode, void* stream) {
       std::stable_sort(vorder + 32 * g, vorder + 32 * g + 32, [&](int x, int y) { return cv[x] > cv[y]; });
     for (int k = 0; k < VQ_CLASSES; k++) w->vclass_order[k] = (uint8_t)vorder[k];
     w->vq_nonempty = 0;
-    for (int i = 0; i < n_ops; i++)
-      if (w->ops[i].bx0 <= w->ops[i].bx1) w->vq_nonempty |= 1u << (w->ops[i].vq_class / 32);
-    if ((rc = issue_uploads(w, ups, s))) return rc;
+    for (int k = 0; k < VQ_CLASSES; k++)
+      if (vper[k]) w->vq_nonempty |= 1u << (k / 32);
   }
+  // the build's counters and flags start at zero
+  ups.push_back({w->res.p, nullptr, sizeof(BuildResult)});
+  ups.push_back({w->work_counter.p, nullptr, 16});
+  ups.push_back({w->chunk_counter.p, nullptr, 1024});
+  ups.push_back({w->evt.p, nullptr, P});
+  ups.push_back({w->bmark.p, nullptr, 4 * ((w->ncells + 31) / 32)});
+  ups.push_back({w->replay_tmp.p, nullptr, replay_clear_bytes(P)});  // the replay's tickets and look-back flags
+  ups.push_back({w->tree.p, nullptr, tree_clear_bytes(E_max), 0x7f});  // min-tree levels 1 and 2, above every depth
+  if ((rc = issue_uploads(w, ups, s))) return rc;  // the op tables
+
+  BuildResult* res = (BuildResult*)w->res.p;
+  launch_cull((const uint2*)w->d_boxes.p, n_ops, w->TX, w->TY, w->TZ, (uint32_t*)w->tile_cnt.p,
+              (uint32_t*)w->tile_off.p, (uint32_t*)w->tile_ops.p, (uint2*)w->tile_boxes.p,
+              (uint32_t*)w->chunk_counter.p + CULL_COUNTER, w->cull_sorted,
+              {(const OpDev*)w->d_ops.p, upload ? (const uint32_t*)w->chunk_dst.p : nullptr, (uint2*)w->chunk_op.p,
+               (uint32_t)n_chunks, P},
+              s);
   FoldArgs fa{};
   fa.chunk_order = (const uint2*)w->chunk_op.p;
   for (int k = 0; k < VCLASSES; k++) fa.class_order[k] = w->class_order[k];
@@ -1910,14 +1983,6 @@ static int build_enqueue_impl(px_world* w, int mode, void* stream) {
                                                           // [2] paint pushed, [4..136] voxel, [160..193] pairs,
                                                           // [CULL_COUNTER] tile-list entries
   {  // per-class regions: the class's pairs (sub-block pass), 8 sub-blocks per pair (voxel pass)
-    uint64_t per[VCLASSES] = {0}, vper[VQ_CLASSES] = {0};
-    for (int i = 0; i < n_ops; i++) {
-      const OpDev& o = w->ops[i];
-      if (o.bx0 > o.bx1) continue;
-      const uint64_t np = (uint64_t)o.nx * o.ny * (uint64_t)(o.bz1 - o.bz0 + 1);
-      per[o.vclass & (VCLASSES - 1)] += np;
-      vper[o.vq_class] += np;
-    }
     uint64_t at = 0;
     for (int k = 0; k < VCLASSES; k++) {
       fa.pq_base[k] = (uint32_t)at;
@@ -2145,6 +2210,9 @@ static int build_finish_impl(px_world* w) {
   w->ops_applied += w->ops.size();
   w->last_ops.swap(w->ops);
   w->last_boxes.swap(w->boxes);
+  w->last_lite.swap(w->lite);
+  w->lite.clear();
+  w->cull_ready = false;
   w->last_code.swap(w->code);
   w->last_params.swap(w->params);
   w->last_code32.swap(w->code32);
@@ -2203,6 +2271,8 @@ static int world_reset_impl(px_world* w, int requeue_last_ops, void* stream) {
     if (!w->ops.empty()) return fail(w, PX_E_INVALID_ARG, "ops are already queued");
     w->ops = w->last_ops;
     w->boxes = w->last_boxes;
+    w->lite = w->last_lite;
+    w->cull_ready = false;
     w->code = w->last_code;
     w->params = w->last_params;
     w->code32 = w->last_code32;
@@ -2495,7 +2565,7 @@ static int batch_create_impl(px_world* const* worlds, size_t n, int mode, uint32
     w->derived_valid = saved[i].derived_valid;
     w->free_valid = saved[i].free_valid;
     w->pairs_per_block = saved[i].ppb;
-    w->ops.clear(); w->boxes.clear(); w->code.clear(); w->params.clear();
+    w->ops.clear(); w->lite.clear(); w->boxes.clear(); w->code.clear(); w->params.clear();
     w->code32.clear(); w->p32.clear(); w->bases.clear();
     w->q.clear();
   }

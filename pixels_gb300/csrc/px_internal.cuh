@@ -276,8 +276,18 @@ constexpr uint32_t TAG_STAGED = 0x40000000u;
 // (cull_sorted_kernel, up to CULL_SORTED_MAX_OPS ops); else the union boxes of 32
 // consecutive ops
 constexpr int CULL_SORTED_MAX_OPS = 47 * 1024;  // 8 warps x ops / 8 bytes of shared memory: 47 KiB
+// The same launch writes the classify pass's chunk order (dst set): op o's chunks, whose first
+// pair it holds, from entry dst[o] on.
+struct ChunkFill {
+  const OpDev* ops;
+  const uint32_t* dst;      // per op; nullptr: the order is there already
+  uint2* order;             // FoldArgs::chunk_order
+  uint32_t n_chunks;
+  unsigned long long n_pairs;
+};
 void launch_cull(const uint2* boxes, int n_ops, int TX, int TY, int TZ, uint32_t* tile_cnt, uint32_t* tile_off,
-                 uint32_t* tile_ops, uint2* tile_boxes, uint32_t* counter, bool sorted, cudaStream_t s);
+                 uint32_t* tile_ops, uint2* tile_boxes, uint32_t* counter, bool sorted, const ChunkFill& fill,
+                 cudaStream_t s);
 // max_blocks > 0 caps the persistent grids (builds sharing the GPU)
 // The evaluation passes (classify .. paint) go on s; the apply pass on s_apply,
 // after eval_done is recorded on s (s_apply == s: one stream, no event).
