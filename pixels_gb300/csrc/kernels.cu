@@ -140,7 +140,7 @@ __device__ __forceinline__ bool box_overlaps_tile(uint2 b, int tx, int ty, int t
 // after its first n_tile_blocks.
 __device__ __forceinline__ void fill_chunks(const ChunkFill& f, int n_ops, int block) {
   const int i = block * 8 + (int)(threadIdx.x >> 5);
-  if (i >= n_ops) return;
+  if (i >= n_ops || !f.dst) return;
   const unsigned long long base = f.ops[i].pair_base, end = i + 1 < n_ops ? f.ops[i + 1].pair_base : f.n_pairs;
   const uint32_t c0 = (uint32_t)((base + 31) / 32), c1 = (uint32_t)((end + 31) / 32);
   uint2* dst = f.order + f.dst[i];
@@ -318,13 +318,95 @@ __global__ void __launch_bounds__(256) cull_sorted_kernel(const uint2* __restric
   }
 }
 
+// The same lists for the few tiles that a short op list touches: one warp per (op, tile)
+// pair, which leaves the tile to its first op's warp.  n_pairs pairs; a tile no op
+// touches keeps no list (nothing asks for one).  256 strokes on a map of 105,600 tiles: a
+// warp per tile 41 us, 11 so; one stroke 19 us, and 3.
+__global__ void __launch_bounds__(256) cull_few_kernel(const uint2* __restrict__ boxes, int n_ops, int TX, int TY,
+                                                       uint32_t n_pairs, uint32_t* tile_cnt, uint32_t* tile_off,
+                                                       uint32_t* tile_ops, uint2* tile_boxes, uint32_t* counter,
+                                                       int n_tile_blocks, ChunkFill fill) {
+  pdl_prologue();
+  if ((int)blockIdx.x >= n_tile_blocks) {
+    fill_chunks(fill, n_ops, (int)blockIdx.x - n_tile_blocks);
+    return;
+  }
+  __shared__ uint32_t s_cnt[8], s_base;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t* __restrict__ first = reinterpret_cast<const uint32_t*>(boxes + n_ops);
+  const uint32_t p = blockIdx.x * 8 + warp;
+  uint32_t cnt = 0, word = 0;  // lane g: the ops of group g (32 consecutive ones) that touch the tile
+  int tx = 0, ty = 0, tz = 0;
+  if (p < n_pairs) {
+    // the pair's op: the last one whose first pair is at or below p (32 entries per step)
+    int lo = 0;
+    for (int len = n_ops; len > 1;) {
+      const int step = (len + 31) / 32, k = lane * step;
+      const uint32_t m = __ballot_sync(FULLMASK, k < len && __ldg(first + lo + k) <= p);
+      const int c = __popc(m) - 1;
+      lo += c * step;
+      len = min(step, len - c * step);
+    }
+    const uint2 b = __ldg(boxes + lo);
+    const int x0 = (int)(b.x & 1023u) >> 2, y0 = (int)((b.x >> 10) & 1023u) >> 2, z0 = (int)((b.x >> 20) & 1023u) >> 2;
+    const int nx = ((int)(b.y & 1023u) >> 2) - x0 + 1, ny = ((int)((b.y >> 10) & 1023u) >> 2) - y0 + 1;
+    const int r = (int)(p - __ldg(first + lo));
+    tz = z0 + r / (nx * ny);
+    ty = y0 + r / nx % ny;
+    tx = x0 + r % nx;
+    const int n_groups = (n_ops + 31) / 32;
+    bool owner = true;
+    for (int g = 0; g < n_groups && owner; g++) {
+      const int i = g * 32 + lane;
+      const uint32_t m = __ballot_sync(FULLMASK, i < n_ops && box_overlaps_tile(__ldg(boxes + i), tx, ty, tz));
+      if (m && !cnt) owner = g * 32 + __ffs(m) - 1 == lo;  // the tile's first op
+      if (lane == g) word = m;
+      cnt += __popc(m);
+    }
+    if (!owner) cnt = 0;
+  }
+  if (lane == 0) s_cnt[warp] = cnt;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t sum = 0;
+    for (int k = 0; k < 8; k++) sum += s_cnt[k];
+    s_base = sum ? atomicAdd(counter, sum) : 0u;
+  }
+  __syncthreads();
+  if (!cnt) return;
+  uint32_t pos = s_base;
+  for (int k = 0; k < warp; k++) pos += s_cnt[k];
+  if (lane == 0) {
+    const int tile = tx + TX * (ty + TY * tz);
+    tile_cnt[tile] = cnt;
+    tile_off[tile] = pos;
+  }
+  const uint32_t c = __popc(word);
+  uint32_t incl = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(FULLMASK, incl, o);
+    if (lane >= o) incl += t;
+  }
+  uint32_t at = pos + incl - c;
+  for (uint32_t m = word; m; m &= m - 1) {  // the ops in order: lane g's after those of the groups before it
+    const uint32_t i = (uint32_t)lane * 32u + (uint32_t)(__ffs(m) - 1);
+    tile_ops[at] = i;
+    tile_boxes[at] = __ldg(boxes + i);
+    at++;
+  }
+}
+
 void launch_cull(const uint2* boxes, int n_ops, int TX, int TY, int TZ, uint32_t* tile_cnt, uint32_t* tile_off,
-                 uint32_t* tile_ops, uint2* tile_boxes, uint32_t* counter, bool sorted, const ChunkFill& fill,
-                 cudaStream_t s) {
-  const int n_tiles = TX * TY * TZ, n_tile_blocks = (n_tiles + 7) / 8;
+                 uint32_t* tile_ops, uint2* tile_boxes, uint32_t* counter, int how, uint32_t n_tile_pairs,
+                 const ChunkFill& fill, cudaStream_t s) {
+  const int n_tiles = TX * TY * TZ, n_tile_blocks = ((how == CULL_FEW ? (int)n_tile_pairs : n_tiles) + 7) / 8;
   const int W = (n_ops + 31) / 32;
-  const dim3 grid(n_tile_blocks + (fill.dst ? (n_ops + 7) / 8 : 0));
-  if (sorted)
+  const dim3 grid(std::max(1, n_tile_blocks + (fill.dst ? (n_ops + 7) / 8 : 0)));
+  if (how == CULL_FEW)
+    launch_pdl(cull_few_kernel, grid, dim3(256), 0, s, boxes, n_ops, TX, TY, n_tile_pairs, tile_cnt, tile_off, tile_ops,
+               tile_boxes, counter, n_tile_blocks, fill);
+  else if (how == CULL_SORTED)
     launch_pdl(cull_sorted_kernel, grid, dim3(256), (size_t)8 * W * 4, s, boxes, n_ops, TX, TY, TZ, W, tile_cnt, tile_off,
                tile_ops, tile_boxes, counter, n_tile_blocks, fill);
   else

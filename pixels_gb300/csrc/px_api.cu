@@ -142,7 +142,8 @@ struct px_world {
 
   // per-build device scratch
   DevBuf d_ops, d_boxes, d_code, d_params, d_code32, d_p32, d_bases;
-  bool cull_sorted = false;
+  int cull_how = CULL_SEQ;
+  uint32_t cull_pairs = 0;      // CULL_FEW: (op, tile) pairs
   DevBuf tile_cnt, tile_off, tile_ops, tile_boxes;
   DevBuf evt, fsrc, pos, etype, ew, depth, tree, replay_tmp;
   DevBuf staging, stage_cell, stage_src, touched;
@@ -1376,11 +1377,30 @@ class HostPool {
 // every 32 ops of the culling order, then that order, two per entry, where it is not the op
 // order: along a Morton curve of the boxes' centres (in 4-brick tiles), taken where its groups
 // cover less than half the tiles the op order's do -- scattered ops (cull_sorted_kernel's bit
-// set costs more on compact scenes).
+// set costs more on compact scenes).  Where the ops touch few of the world's tiles -- edits on a
+// resident map -- neither: their first (op, tile) pairs (cull_few_kernel).
 void cull_tables(px_world* w, int n_ops) {
   const int n_groups = (n_ops + 31) / 32;
   w->h_boxes.resize((size_t)n_ops + n_groups + (n_ops + 1) / 2);
   const uint2* B = w->h_boxes.data();
+  if (n_ops && n_ops <= CULL_FEW_MAX_OPS) {
+    uint64_t pairs = 0;
+    uint2* first = w->h_boxes.data() + n_ops;
+    for (int i = 0; i < n_ops; i++) {
+      (i & 1 ? first[i >> 1].y : first[i >> 1].x) = (uint32_t)pairs;
+      if (B[i].x >> 30) continue;
+      uint64_t t = 1;
+      for (int a = 0; a < 30; a += 10) t *= ((B[i].y >> a) & 1023u) / 4 - ((B[i].x >> a) & 1023u) / 4 + 1;
+      pairs += t;
+      if (2 * pairs >= w->ntiles) break;
+    }
+    if (2 * pairs < w->ntiles) {
+      w->cull_how = CULL_FEW;
+      w->cull_pairs = (uint32_t)pairs;
+      w->n_cull = (size_t)n_ops + (n_ops + 1) / 2;
+      return;
+    }
+  }
   // the union boxes of 32 ops of an order (none: the op order), and the tiles they cover in all
   // (the group tests a tile passes grow with it)
   auto group_boxes = [&](const uint32_t* ord, uint2* gb) {
@@ -1405,7 +1425,7 @@ void cull_tables(px_world* w, int n_ops) {
   };
   uint2* const groups = w->h_boxes.data() + n_ops;
   const uint64_t vol_seq = group_boxes(nullptr, groups);
-  w->cull_sorted = false;
+  w->cull_how = CULL_SEQ;
   w->n_cull = (size_t)n_ops + n_groups;
   if (n_ops > CULL_SORTED_MAX_OPS || n_groups <= 1) return;
   auto spread = [](uint32_t v) {  // 8 bits -> every third bit
@@ -1442,7 +1462,7 @@ void cull_tables(px_world* w, int n_ops) {
   }
   w->h_groups.resize(n_groups);
   if (2 * group_boxes(ord, w->h_groups.data()) >= vol_seq) return;
-  w->cull_sorted = true;
+  w->cull_how = CULL_SORTED;
   std::memcpy(groups, w->h_groups.data(), sizeof(uint2) * n_groups);
   for (int k = 0; k < n_ops; k += 2) w->h_boxes[w->n_cull++] = make_uint2(ord[k], k + 1 < n_ops ? ord[k + 1] : 0u);
 }
@@ -1962,7 +1982,7 @@ static int build_enqueue_impl(px_world* w, int mode, void* stream) {
   BuildResult* res = (BuildResult*)w->res.p;
   launch_cull((const uint2*)w->d_boxes.p, n_ops, w->TX, w->TY, w->TZ, (uint32_t*)w->tile_cnt.p,
               (uint32_t*)w->tile_off.p, (uint32_t*)w->tile_ops.p, (uint2*)w->tile_boxes.p,
-              (uint32_t*)w->chunk_counter.p + CULL_COUNTER, w->cull_sorted,
+              (uint32_t*)w->chunk_counter.p + CULL_COUNTER, w->cull_how, w->cull_pairs,
               {(const OpDev*)w->d_ops.p, upload ? (const uint32_t*)w->chunk_dst.p : nullptr, (uint2*)w->chunk_op.p,
                (uint32_t)n_chunks, P},
               s);

@@ -271,10 +271,13 @@ struct FoldArgs {
 constexpr uint32_t TAG_STAGED = 0x40000000u;
 
 // Host-side launch wrappers (kernels.cu)
-// counter: a zeroed word (the tile lists' reservation count).  sorted: boxes holds
-// the op boxes, the union boxes of 32 ops in the order after them, then that order
-// (cull_sorted_kernel, up to CULL_SORTED_MAX_OPS ops); else the union boxes of 32
-// consecutive ops
+// counter: a zeroed word (the tile lists' reservation count).  boxes holds the op boxes and,
+// by how, CULL_SEQ: the union boxes of 32 consecutive ops; CULL_SORTED: the union boxes of
+// 32 ops of an order, then that order, two per entry (up to CULL_SORTED_MAX_OPS ops);
+// CULL_FEW: the ops' first (op, tile) pairs, two per entry (up to CULL_FEW_MAX_OPS ops,
+// n_tile_pairs pairs in all)
+enum { CULL_SEQ, CULL_SORTED, CULL_FEW };
+constexpr int CULL_FEW_MAX_OPS = 1024;  // a ballot word per lane
 constexpr int CULL_SORTED_MAX_OPS = 47 * 1024;  // 8 warps x ops / 8 bytes of shared memory: 47 KiB
 // The same launch writes the classify pass's chunk order (dst set): op o's chunks, whose first
 // pair it holds, from entry dst[o] on.
@@ -286,8 +289,8 @@ struct ChunkFill {
   unsigned long long n_pairs;
 };
 void launch_cull(const uint2* boxes, int n_ops, int TX, int TY, int TZ, uint32_t* tile_cnt, uint32_t* tile_off,
-                 uint32_t* tile_ops, uint2* tile_boxes, uint32_t* counter, bool sorted, const ChunkFill& fill,
-                 cudaStream_t s);
+                 uint32_t* tile_ops, uint2* tile_boxes, uint32_t* counter, int how, uint32_t n_tile_pairs,
+                 const ChunkFill& fill, cudaStream_t s);
 // max_blocks > 0 caps the persistent grids (builds sharing the GPU)
 // The evaluation passes (classify .. paint) go on s; the apply pass on s_apply,
 // after eval_done is recorded on s (s_apply == s: one stream, no event).
