@@ -46,14 +46,24 @@ namespace px {
 #ifndef PX_FOLD_MINB
 #define PX_FOLD_MINB 3
 #endif
-// items per ticket of the lean voxel kernels, at most, and tickets per warp, at least.  Sum of
-// these kernels, penthouse at 80 / 256 edits at 160 / synthetic: 1 item 165 / 182 / 620 us,
-// 4 items 92 / 73 / 284, 8 items 98 / 72 / 289, 16 items (2 tickets) 106 / 74 / 317
+// Work per ticket, at most: items of the lean voxel kernels, passes of four pairs of the
+// sub-block pass, chunks of the classify pass; every warp still takes PX_TICKETS tickets.
+// One counter serves a grid, at some 0.65 ns an atomic.  Sums of the lean voxel kernels, penthouse
+// at 80 / 256 edits at 160 / synthetic: 1 item 165 / 182 / 620 us, 4 items 92 / 73 / 284, 8
+// items 98 / 72 / 289, 16 items (2 tickets) 106 / 74 / 317.  Penthouse at 128, sub-block pass:
+// 1 pass 135 us, 2 112, 4 111 (at 80: 54, 54, 58), classify:
+// 1 chunk 49, 2 47.  More bricks per ticket in the apply pass: 119 -> 159 us (heavy neighbours)
+#ifndef PX_TICKETS
+#define PX_TICKETS 4u
+#endif
 #ifndef PX_VOXEL_TICKET
 #define PX_VOXEL_TICKET 4u
 #endif
-#ifndef PX_VOXEL_TICKETS
-#define PX_VOXEL_TICKETS 4u
+#ifndef PX_SUB_TICKET
+#define PX_SUB_TICKET 2u
+#endif
+#ifndef PX_CLASSIFY_TICKET
+#define PX_CLASSIFY_TICKET 2u
 #endif
 // the apply pass takes four bricks per warp at a time where it has at least this many for every
 // warp.  Whole passes: the penthouse at 80 voxels per metre (40 bricks per warp) 587 us with
@@ -466,6 +476,12 @@ struct NextTicket {
   __device__ __forceinline__ uint32_t get() const { return __shfl_sync(FULLMASK, raw, 0); }
 };
 
+// Work units of `per` items a warp takes per ticket, at most `most`, so that every warp still
+// takes PX_TICKETS tickets of n items.
+__device__ __forceinline__ uint32_t tickets(uint32_t n, uint32_t per, uint32_t most) {
+  return max(1u, min(most, n / (per * PX_TICKETS * gridDim.x * (blockDim.x >> 5))));
+}
+
 // Decisions of apply() from a float32 interval (thresholds certified on the host):
 // brick/sub-block: 0 = outside (skip), 1 = partial, 2 = full, 3 = undecided.
 __device__ __forceinline__ int classify32(Iv d, const float* thr, int base) {
@@ -636,10 +652,7 @@ __device__ __forceinline__ void classify_finish(const FoldArgs& a, bool valid, u
     const uint32_t wm = __ballot_sync(FULLMASK, first && heavy == (e == 0));
     if (!wm) continue;
     uint32_t base = 0;
-    if (lane == 0) {
-      base = atomicAdd(a.work_counter + 1 + e, (uint32_t)__popc(wm));
-      atomicAdd(&a.res->n_work, (uint32_t)__popc(wm));
-    }
+    if (lane == 0) base = atomicAdd(a.work_counter + 1 + e, (uint32_t)__popc(wm));
     base = __shfl_sync(FULLMASK, base, 0) + __popc(wm & ((1u << lane) - 1u));
     if (first && heavy == (e == 0))
       a.work[e ? (uint32_t)a.touched_cap - base : base] = (uint32_t)bx | ((uint32_t)by << 10) | ((uint32_t)bz << 20);
@@ -697,12 +710,15 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_CLASSIFY_MINB : PX_CLASSIF
   uint32_t st_local = 0;
   const unsigned long long P = a.n_pairs;
   const uint32_t n_chunks = (uint32_t)((P + 31) / 32);
+  const uint32_t B = tickets(n_chunks, 1u, PX_CLASSIFY_TICKET);
   NextTicket tk;
-  tk.issue(a.chunk_counter, 1u, lane);
+  tk.issue(a.chunk_counter, B, lane);
   for (;;) {
-    const uint32_t take = tk.get();
-    if (take >= n_chunks) break;
-    tk.issue(a.chunk_counter, 1u, lane);
+    const uint32_t first = tk.get();
+    if (first >= n_chunks) break;
+    tk.issue(a.chunk_counter, B, lane);
+#pragma unroll 1
+    for (uint32_t take = first; take < min(first + B, n_chunks); take++) {
     const uint2 ce = __ldg(a.chunk_order + take);
     const uint32_t chunk = ce.x;
     const unsigned long long p = (unsigned long long)chunk * 32 + lane;
@@ -759,6 +775,7 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_CLASSIFY_MINB : PX_CLASSIF
       }
     }
     classify_finish<MODE>(a, valid, o, O, p, bx, by, bz, cls, lane, st_local);
+    }
   }
   uint32_t nb = n_brick, stw = st_local;
 #pragma unroll
@@ -853,30 +870,34 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_SUB_MINB : PX_CLASSIFY64_M
     if (lane >= o) incl += t;
   }
   const uint32_t n_items = __shfl_sync(FULLMASK, incl, 31);
+  const uint32_t at0 = (lane < VCLASSES ? a.pq_base[my_cls] : 0u) - (incl - own);  // queue position of item `it`: at0 + it
   const int g = lane >> 3, s = lane & 7;
+  const uint32_t B = tickets(n_items, 4u, PX_SUB_TICKET);  // passes per ticket
   NextTicket tk;
-  tk.issue(&a.pitem_counter[0], 4u, lane);
+  tk.issue(&a.pitem_counter[0], 4u * B, lane);
   for (;;) {
-    const uint32_t base = tk.get();
-    if (base >= n_items) break;
-    tk.issue(&a.pitem_counter[0], 4u, lane);
-    // the class and queue position of each of the pass's four items
-    uint32_t my_k = 0, my_first = 0;
+    const uint32_t first = tk.get();
+    if (first >= n_items) break;
+    tk.issue(&a.pitem_counter[0], 4u * B, lane);
+#pragma unroll 1
+    for (uint32_t base = first; base < min(first + 4u * B, n_items); base += 4u) {
+    // the queue position of each of the pass's four items, by its class
+    const uint32_t it = base + (uint32_t)g;
+    const bool have = it < n_items;
+    uint32_t at = it;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       const int kq = __popc(__ballot_sync(FULLMASK, lane < VCLASSES && incl <= base + q));
-      const uint32_t fq = __shfl_sync(FULLMASK, incl - own, kq & 31);
-      if (g == q) { my_k = (uint32_t)kq; my_first = fq; }
+      const uint32_t aq = __shfl_sync(FULLMASK, at0, kq & 31);
+      if (g == q) at += aq;
     }
-    const uint32_t it = base + (uint32_t)g;
-    const bool have = it < n_items;
     uint32_t oo = 0;
     unsigned long long pp = 0;
     int pbx = 0, pby = 0, pbz = 0, scls = PC_SKIP;
     bool boxr = false;
     Iv dc = {-INFINITY, INFINITY};  // enclosure of the sub-block centre's value
     if (have) {
-      const uint2 item = __ldg(a.pitems + a.pq_base[a.class_order[my_k]] + (it - my_first));
+      const uint2 item = __ldg(a.pitems + at);
       oo = item.x;
       pp = item.y;
       const OpDev* Q = a.ops + oo;
@@ -909,6 +930,7 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_SUB_MINB : PX_CLASSIFY64_M
     code16 |= __shfl_xor_sync(FULLMASK, code16, 4);
     if (s == 0 && have) a.psub[pp] = (uint16_t)code16;
     sub_finish<MODE>(a, have, oo, pp, pbx, pby, pbz, s, scls, dc, boxr, lane, st_local);
+    }
   }
   uint32_t stw = st_local;
 #pragma unroll
@@ -1098,10 +1120,7 @@ __global__ void __launch_bounds__(256, G == VQ_WIDE ? PX_VWIDE_MINB : G == VQ_AF
   // distance classes of the two voxels (OpDev::lip: axes at 1.5 voxels from the centre)
   const int kxy = (lx == 0 || lx == 3) + (lyv == 0 || lyv == 3);
   const int kc[2] = {kxy + (lz == 0), kxy + (lz == 1)};
-  // items per ticket: one counter serves the whole grid, and with a ticket per item its
-  // atomics, some 0.65 ns each, were the kernel's bound (1.5 items per ns whatever the
-  // shapes); few where the items are few, so that the warps end together
-  const uint32_t B = max(1u, min(PX_VOXEL_TICKET, n_items / (PX_VOXEL_TICKETS * gridDim.x * (blockDim.x >> 5))));
+  const uint32_t B = tickets(n_items, 1u, PX_VOXEL_TICKET);  // items per ticket
   NextTicket tk;
   tk.issue(taken, B, lane);
   for (;;) {

@@ -155,7 +155,6 @@ struct BuildResult {
   uint32_t n_holes;      // after the build
   uint32_t stage_count;  // bricks that end as pool bricks and were touched (staging slots wanted)
   uint32_t touched_count;  // bricks whose grid entry the build rewrites
-  uint32_t n_work;       // bricks with at least one (op, brick) pair that is not skipped
   uint32_t n_fresh;
   uint32_t max_pool_index;
   BuildCounters c;
