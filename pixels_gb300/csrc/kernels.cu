@@ -2237,11 +2237,7 @@ void launch_replay(const ReplayArgs& a, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 // finalize: staging -> pool at the replayed indices, grid entries
 
-#ifndef PX_FIN_BRICKS
-#define PX_FIN_BRICKS 8
-#endif
-constexpr int FIN_BRICKS = PX_FIN_BRICKS;  // touched bricks per warp pass of finalize (at most 32)
-static_assert(FIN_BRICKS >= 1 && FIN_BRICKS <= 32, "one brick per lane");
+constexpr int FIN_BRICKS = 8;  // staged bricks per warp pass of finalize, at most (one per lane)
 
 __global__ void __launch_bounds__(256) finalize_kernel(FinalizeArgs a) {
   __shared__ uint8_t op_s[256];
@@ -2267,34 +2263,37 @@ __global__ void __launch_bounds__(256) finalize_kernel(FinalizeArgs a) {
   // the holes after the build: their pushes' event indices become pool indices
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x, nh = a.res->n_holes; k < nh; k += gridDim.x * blockDim.x)
     a.holes_out[k] = (uint32_t)(__ldcg(a.ew + a.holes_out[k]) & 0xffffffffull);
+  // the touched bricks that end uniform: their grid entries
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, n = a.res->touched_count; t < n; t += gridDim.x * blockDim.x) {
+    const uint2 e = a.touched[t];
+    if (!(e.y & TAG_STAGED) || (e.y & UNIFORM)) a.grid[e.x] = e.y;
+  }
   const int lane = threadIdx.x & 31;
-  const uint32_t n = a.res->touched_count;
-  // FIN_BRICKS touched bricks per warp pass: each of the first lanes resolves one
-  // brick's pool index (a chain of dependent loads), then the warp copies the
-  // staged bricks four at a time (eight 16-byte loads in flight per lane).  Few
-  // bricks per pass keep many warps' chains and copies in flight at once.
+  const uint32_t n = a.res->stage_count;
+  // per staged bricks per warp pass: each of the first lanes resolves one brick's pool
+  // index (a chain of dependent loads), then the warp copies the bricks four at a
+  // time (eight 16-byte loads in flight per lane).  Up to FIN_BRICKS, fewer where
+  // that would leave warps without any: with 8 / 4 / 2 / 16 everywhere, penthouse at 128
+  // voxels per metre 72 / 79 / 112 / 75 us, at 80 23 / 24 / 30 / 24, at 20 10 / 7 / 6 / 16,
+  // twelve scenes 156 / 116 / 104 / 232 in all; over the touched bricks, a quarter of
+  // them staged, 8 per pass, 100, 31, 10 and 145.
   const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * FIN_BRICKS; base < n;
-       base += n_warps * FIN_BRICKS) {
-    const uint32_t t = base + lane;
-    uint32_t cell = 0, slot = 0, idx = 0;
+  uint32_t per = 1;
+  while (per < (uint32_t)FIN_BRICKS && n > per * n_warps) per *= 2;
+  for (uint32_t base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per; base < n; base += n_warps * per) {
+    const uint32_t slot = base + lane;
+    uint32_t cell = 0, idx = 0;
     bool staged = false;
-    if (lane < FIN_BRICKS && t < n) {
-      const uint2 e = a.touched[t];
-      cell = e.x;
-      if (!(e.y & TAG_STAGED) || (e.y & UNIFORM)) {
-        a.grid[e.x] = e.y;
+    if (lane < per && slot < n) {
+      const long long src = a.stage_src[slot];
+      cell = a.stage_cell[slot];
+      if (src >= 0) {
+        const unsigned long long w = a.ew[H + a.pos[src]];
+        if (!(w & KNOWN)) atomicOr(&a.res->status, (uint32_t)ST_CHAIN);
+        else { idx = (uint32_t)(w & 0xffffffffull); staged = true; }
       } else {
-        slot = e.y & 0x3fffffffu;
-        const long long src = a.stage_src[slot];
-        if (src >= 0) {
-          const unsigned long long w = a.ew[H + a.pos[src]];
-          if (!(w & KNOWN)) atomicOr(&a.res->status, (uint32_t)ST_CHAIN);
-          else { idx = (uint32_t)(w & 0xffffffffull); staged = true; }
-        } else {
-          idx = (uint32_t)(-(src + 1));
-          staged = true;
-        }
+        idx = (uint32_t)(-(src + 1));
+        staged = true;
       }
     }
     uint32_t mx = staged ? idx : 0u;
@@ -2363,9 +2362,9 @@ __global__ void __launch_bounds__(256) finalize_kernel(FinalizeArgs a) {
 void launch_finalize(const FinalizeArgs& a, uint32_t touched_cap, cudaStream_t s) {
   int dev = 0, n_sms = 152;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
-  // a grid-stride loop over the touched bricks (their count is known on the device
-  // only): at most four blocks per SM, fewer when the bound is small
-  const size_t b = ((size_t)touched_cap + 8 * FIN_BRICKS - 1) / (8 * FIN_BRICKS);
+  // grid-stride loops over the touched and the staged bricks (their counts are known on the
+  // device only): at most four blocks per SM, fewer when the bound is small
+  const size_t b = ((size_t)touched_cap + 7) / 8;
   const int blocks = (int)std::max<size_t>(1, std::min<size_t>(b, (size_t)n_sms * 4));
   launch_pdl(finalize_kernel, dim3(blocks), dim3(256), 0, s, a);
 }
