@@ -31,11 +31,14 @@ namespace px {
 #define FULLMASK 0xffffffffu
 
 // CTAs per SM the two build kernels are compiled for (register budget)
-#ifndef PX_CLASSIFY_MINB
-#define PX_CLASSIFY_MINB 3
-#endif
-#ifndef PX_SUB_MINB
-#define PX_SUB_MINB PX_CLASSIFY_MINB
+// The mixed form's classify and sub-block passes, compiled for two CTAs per SM (128 registers, no
+// spills) and for three (80 registers, spills around the rare interpreter): two where a build
+// has the GPU to itself and at most this many (op, brick) pairs.  Both passes, two / three:
+// 256 edits at 160 voxels per metre (0.25 M pairs) 61 / 74 us, penthouse at 20 (0.03 M) 37 / 42,
+// at 80 (0.4 M) 79 / 82, synthetic (1.0 M) 153 / 150, penthouse at 128 (1.2 M) 178 / 167; twelve
+// scenes side by side 1,181 / 1,160 us in all
+#ifndef PX_TWO_CTA_PAIRS
+#define PX_TWO_CTA_PAIRS (1u << 19)
 #endif
 #ifndef PX_VOXEL_MINB
 #define PX_VOXEL_MINB 3
@@ -701,8 +704,8 @@ __device__ __forceinline__ void classify_finish(const FoldArgs& a, bool valid, u
 //   sub-blocks: 4 partial pairs x 8 sub-blocks per pass;
 // partial sub-blocks go to a queue that voxel_kernel drains one at a time
 // (64 voxels on 32 lanes), which keeps the heavy voxel work evenly spread.
-template <int MODE>
-__global__ void __launch_bounds__(256, MODE == 1 ? PX_CLASSIFY_MINB : PX_CLASSIFY64_MINB) classify_kernel(FoldArgs a) {
+template <int MODE, int MINB>
+__global__ void __launch_bounds__(256, MINB) classify_kernel(FoldArgs a) {
   pdl_prologue();
   const int lane = threadIdx.x & 31;
   LaneStats ls = {a.res};
@@ -854,8 +857,8 @@ __device__ __forceinline__ void sub_finish(const FoldArgs& a, bool have, uint32_
 // warp pass (8 lanes each, one sub-block per lane), pairs taken in shape-class
 // order like the voxel work.  Writes the pair's 2-bit sub-block classes, the
 // voxel masks of lone boxes (per-axis runs), and queues the partial sub-blocks.
-template <int MODE>
-__global__ void __launch_bounds__(256, MODE == 1 ? PX_SUB_MINB : PX_CLASSIFY64_MINB) sub_kernel(FoldArgs a) {
+template <int MODE, int MINB>
+__global__ void __launch_bounds__(256, MINB) sub_kernel(FoldArgs a) {
   pdl_prologue();
   const int lane = threadIdx.x & 31;
   LaneStats ls = {a.res};
@@ -1736,8 +1739,13 @@ void launch_fold(const FoldArgs& a, int mode, int n_sms, cudaStream_t s, cudaEve
                  cudaStream_t s_apply, cudaEvent_t eval_done) {
   auto grid = [&](int per_sm) { return max_blocks > 0 && max_blocks < n_sms * per_sm ? max_blocks : n_sms * per_sm; };
   if (mode == 1) {
-    launch_pdl(classify_kernel<1>, dim3(grid(PX_CLASSIFY_MINB)), dim3(256), 0, s, a);
-    launch_pdl(sub_kernel<1>, dim3(grid(PX_SUB_MINB)), dim3(256), 0, s, a);
+    if (max_blocks <= 0 && a.n_pairs <= PX_TWO_CTA_PAIRS) {
+      launch_pdl(classify_kernel<1, 2>, dim3(grid(2)), dim3(256), 0, s, a);
+      launch_pdl(sub_kernel<1, 2>, dim3(grid(2)), dim3(256), 0, s, a);
+    } else {
+      launch_pdl(classify_kernel<1, 3>, dim3(grid(3)), dim3(256), 0, s, a);
+      launch_pdl(sub_kernel<1, 3>, dim3(grid(3)), dim3(256), 0, s, a);
+    }
     if (a.vq_nonempty & (1u << VQ_NARROW)) {
       if (a.validate) launch_pdl(voxel_lean_kernel<true, VQ_NARROW>, dim3(grid(PX_VSIMPLE_MINB)), dim3(256), 0, s, a);
       else launch_pdl(voxel_lean_kernel<false, VQ_NARROW>, dim3(grid(PX_VSIMPLE_MINB)), dim3(256), 0, s, a);
@@ -1753,8 +1761,8 @@ void launch_fold(const FoldArgs& a, int mode, int n_sms, cudaStream_t s, cudaEve
     if (a.vq_nonempty & (1u << VQ_GENERIC))
       launch_pdl(voxel_kernel<1, VQ_GENERIC, VQ_GENERIC>, dim3(grid(PX_VOXEL_MINB)), dim3(256), 0, s, a);
   } else {
-    launch_pdl(classify_kernel<0>, dim3(grid(PX_CLASSIFY64_MINB)), dim3(256), 0, s, a);
-    launch_pdl(sub_kernel<0>, dim3(grid(PX_CLASSIFY64_MINB)), dim3(256), 0, s, a);
+    launch_pdl(classify_kernel<0, PX_CLASSIFY64_MINB>, dim3(grid(PX_CLASSIFY64_MINB)), dim3(256), 0, s, a);
+    launch_pdl(sub_kernel<0, PX_CLASSIFY64_MINB>, dim3(grid(PX_CLASSIFY64_MINB)), dim3(256), 0, s, a);
     launch_pdl(voxel_kernel<0, VQ_NARROW, VQ_GENERIC>, dim3(grid(PX_CLASSIFY64_MINB)), dim3(256), 0, s, a);
   }
   // the mixed form's paint pass also resolves the lean voxel kernels' rescue list
