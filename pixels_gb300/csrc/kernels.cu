@@ -1323,9 +1323,14 @@ __global__ void __launch_bounds__(256, PX_PAINT_MINB) paint_kernel(FoldArgs a) {
   // float64 paints (the front of the queue) first, then the certified float32 ones
   const uint32_t n_front = min(__ldg(a.paint_item_counter), a.paint_items_cap);
   const uint32_t n_items = n_front + min(__ldg(a.paint_item_counter + 1), a.paint_items_cap - n_front);
+  // two items per ticket only where there are many: an item of a float64 paint takes tens of
+  // microseconds, and a second one behind it is the pass's tail (penthouse at 128 voxels per
+  // metre, two always / two from eight per warp on: 132 / 97 us; such an item shared by two or
+  // four warps changed nothing)
+  const uint32_t batch = n_items >= 8u * gridDim.x * (blockDim.x >> 5) ? 2u : 1u;
   WorkBatch wb;
   for (;;) {
-    const uint32_t it = wb.next(a.paint_counter, 2, lane);
+    const uint32_t it = wb.next(a.paint_counter, batch, lane);
     if (it >= n_items) break;
     const uint2 item = __ldg(a.paint_items + (it < n_front ? it : a.paint_items_cap - 1 - (it - n_front)));
     // a float64 item (the front) is half a sub-block: voxel rows r = bit 31 of its op field;
