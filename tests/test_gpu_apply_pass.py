@@ -11,7 +11,7 @@ import pytest
 
 from pixels_gb300 import config
 from pixels_gb300.ir import Program
-from pixels_gb300.paints import noise
+from pixels_gb300.paints import noise, tufted
 from pixels_gb300.shapes import box, capsule, rotateY, roundBox, sphere
 from pixels_gb300.world import MODE_FP64, MODE_MIXED, VoxelWorld
 
@@ -61,6 +61,34 @@ def test_crowded_bricks(built_lib, mode, vpm, dims, n_ops, cover):
     np.testing.assert_array_equal(grid, o.grid)
     assert w.poolUsed == o.pool_used
     np.testing.assert_array_equal(w.freeBricks(), o.free_holes)
+    live = np.nonzero((o.grid != 0) & ((o.grid & 0x80000000) == 0))[0]
+    idx = o.grid[live].astype(np.int64) - 1
+    np.testing.assert_array_equal(w.pool.reshape(-1, 512)[idx], o.pool.reshape(-1, 512)[idx])
+    w.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [MODE_FP64, MODE_MIXED])
+def test_paints_past_the_slot_budget(built_lib, mode):
+    """A painted op over 65^3 bricks has more (op, brick) pairs than there are paint slots
+    (262,144): its paints are called by the apply pass, the costly kind keeps its slots."""
+    vpm, dims = 20.0, (520, 520, 520)
+    prog = Program()
+    with config.using(vpm):
+        prog.add_op(0, sphere((9.0, 9.0, 9.0), 2.5), 0x0305)
+        prog.add_op(0, capsule((0.5, 0.5, 0.5), (25.5, 25.5, 25.5), 0.4), noise(77, 31.0, 1.5, 2.5, 0.75, 0.1, 0x0107, 9))
+        prog.add_op(2, capsule((25.5, 0.5, 0.5), (0.5, 25.5, 25.5), 0.6), noise(5, 12.0, 2.5, 0.5, 3.0, -0.1, 0x0211, 0x0312))
+        prog.add_op(0, roundBox((12.0, 12.0, 11.0), (1.0, 0.6, 0.8), 0.1), tufted(11.0, 11.4, 21))
+        prog.add_op(1, sphere((12.6, 12.2, 11.2), 0.7), 0)
+    o = pyoracle.OracleWorld(prog.to_bytes(), vpm, dims, threads=8)
+    assert o.stats["paint_evals"] > 0
+    w = VoxelWorld(*dims, vpm=vpm, mode=mode)
+    w._pending = prog
+    w.build()
+    assert w.stats()["pairs"] > 2 * 262144
+    grid = w.grid
+    np.testing.assert_array_equal(grid, o.grid)
+    assert w.poolUsed == o.pool_used
     live = np.nonzero((o.grid != 0) & ((o.grid & 0x80000000) == 0))[0]
     idx = o.grid[live].astype(np.int64) - 1
     np.testing.assert_array_equal(w.pool.reshape(-1, 512)[idx], o.pool.reshape(-1, 512)[idx])
