@@ -102,6 +102,33 @@ __device__ __forceinline__ void pdl_prologue() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+__device__ __forceinline__ unsigned long long device_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
+// The end of a build's last kernel, by every thread of every block: the block that finishes last
+// copies the result to the host's copy (pinned memory), so that the build ends with this
+// kernel instead of a copy behind it (7 us of a build; the times of its passes come from the
+// device clock for the same reason: an event between two kernels costs their overlap, 4 us each).
+__device__ __forceinline__ void publish_result(BuildResult* res, BuildResult* host) {
+  if (!host) return;
+  __shared__ bool s_last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(&res->done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(res);
+  volatile uint32_t* dst = reinterpret_cast<volatile uint32_t*>(host);
+  for (uint32_t i = threadIdx.x; i < sizeof(BuildResult) / 4; i += blockDim.x) dst[i] = __ldcg(src + i);
+  __threadfence_system();
+}
+
 // The staging area lives between the apply pass and finalize only: its stores
 // ask L2 to keep the lines (evict_last), and finalize, once it has read a staged
 // brick, drops its lines from L2 without writing them back (discard.global.L2),
@@ -707,6 +734,7 @@ __device__ __forceinline__ void classify_finish(const FoldArgs& a, bool valid, u
 template <int MODE, int MINB>
 __global__ void __launch_bounds__(256, MINB) classify_kernel(FoldArgs a) {
   pdl_prologue();
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.res->t_classify = device_ns();
   const int lane = threadIdx.x & 31;
   LaneStats ls = {a.res};
   uint32_t n_brick = 0;
@@ -1441,6 +1469,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_al
 template <bool INLINE>
 __global__ void __launch_bounds__(256, PX_FOLD_MINB) fold_kernel(FoldArgs a) {
   pdl_prologue();
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.res->t_apply = device_ns();
   __shared__ __align__(16) unsigned long long spm[8][32][8];  // voxel masks of the looked-up partial pairs
   __shared__ __align__(16) uint32_t spv[8][BRICK_VOXELS];  // paint values of the next painted pair
   const int lane = threadIdx.x & 31;
@@ -1740,7 +1769,7 @@ __global__ void __launch_bounds__(256, PX_FOLD_MINB) fold_kernel(FoldArgs a) {
   }
 }
 
-void launch_fold(const FoldArgs& a, int mode, int n_sms, cudaStream_t s, cudaEvent_t mid, int max_blocks,
+void launch_fold(const FoldArgs& a, int mode, int n_sms, cudaStream_t s, int max_blocks,
                  cudaStream_t s_apply, cudaEvent_t eval_done) {
   auto grid = [&](int per_sm) { return max_blocks > 0 && max_blocks < n_sms * per_sm ? max_blocks : n_sms * per_sm; };
   if (mode == 1) {
@@ -1773,7 +1802,6 @@ void launch_fold(const FoldArgs& a, int mode, int n_sms, cudaStream_t s, cudaEve
   // the mixed form's paint pass also resolves the lean voxel kernels' rescue list
   if (mode == 1) launch_pdl(paint_kernel<1>, dim3(grid(4)), dim3(256), 0, s, a);
   else if (a.n_paint_slots) launch_pdl(paint_kernel<0>, dim3(grid(4)), dim3(256), 0, s, a);
-  if (mid) cudaEventRecord(mid, s);
   if (s_apply != s) {  // the apply pass waits for these passes on its own stream
     cudaEventRecord(eval_done, s);
     cudaStreamWaitEvent(s_apply, eval_done, 0);
@@ -1960,6 +1988,7 @@ __global__ void __launch_bounds__(RP_THREADS) event_scan_kernel(ReplayArgs a) {
   int32_t* const L2 = a.tl.n >= 2 ? a.tree + a.tl.off[1] : nullptr;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
+    a.res->t_replay = device_ns();
     a.res->h_before = H;
     a.res->u_before = U0;
     if (P == 0) { a.res->n_events = H; a.res->n_fresh = 0; }
@@ -2252,11 +2281,7 @@ void launch_replay(const ReplayArgs& a, cudaStream_t s) {
 
 constexpr int FIN_BRICKS = 8;  // staged bricks per warp pass of finalize, at most (one per lane)
 
-__global__ void __launch_bounds__(256) finalize_kernel(FinalizeArgs a) {
-  __shared__ uint8_t op_s[256];
-  op_s[threadIdx.x] = a.opaque[threadIdx.x];  // 256 threads
-  pdl_prologue();
-  __syncthreads();
+__device__ __forceinline__ void finalize_build(const FinalizeArgs& a, const uint8_t* op_s) {
   // commit only a complete build (every staging slot written, every pool index within
   // the pool) that follows committed builds; the first thread records the outcome
   const bool after_failure = __ldcg(&a.state->poisoned) != 0;
@@ -2372,6 +2397,15 @@ __global__ void __launch_bounds__(256) finalize_kernel(FinalizeArgs a) {
   }
 }
 
+__global__ void __launch_bounds__(256) finalize_kernel(FinalizeArgs a) {
+  __shared__ uint8_t op_s[256];
+  op_s[threadIdx.x] = a.opaque[threadIdx.x];  // 256 threads
+  pdl_prologue();
+  __syncthreads();
+  finalize_build(a, op_s);
+  publish_result(a.res, a.host);
+}
+
 void launch_finalize(const FinalizeArgs& a, uint32_t touched_cap, cudaStream_t s) {
   int dev = 0, n_sms = 152;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
@@ -2385,8 +2419,7 @@ void launch_finalize(const FinalizeArgs& a, uint32_t touched_cap, cudaStream_t s
 // ---------------------------------------------------------------------------
 // derive: super-grid counts and density (GpuWorld.ts:90-101, VoxelWorld.ts:159-170)
 
-__global__ void __launch_bounds__(256) derive_kernel(DeriveArgs a) {
-  pdl_prologue();
+__device__ __forceinline__ void derive_world(const DeriveArgs& a) {
   // a build that committed nothing leaves the world (and its derived buffers) as they were
   if (a.res && (a.res->status & (ST_NO_COMMIT | ST_POOL_OVERFLOW))) return;
   const uint32_t* __restrict__ grid = a.grid;
@@ -2463,6 +2496,12 @@ __global__ void __launch_bounds__(256) derive_kernel(DeriveArgs a) {
   if (used > cap || len > a.free_cap) return;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (uint64_t)gridDim.x * blockDim.x)
     a.free_list[i] = i < n_holes ? __ldg(a.holes + i) : (uint32_t)(cap - 1 - (i - n_holes));
+}
+
+__global__ void __launch_bounds__(256) derive_kernel(DeriveArgs a) {
+  pdl_prologue();
+  derive_world(a);
+  publish_result(a.res, a.host);
 }
 
 // A build's op-table uploads (read straight from the host arrays: pageable

@@ -185,7 +185,7 @@ struct px_world {
   // in-flight build
   bool in_flight = false;
   cudaStream_t stream = nullptr;
-  cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_fold0 = nullptr, ev_fold1 = nullptr, ev_mid = nullptr;
+  cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t ev_eval = nullptr;   // evaluation passes done (the apply stream waits for it)
   cudaEvent_t ev_done = nullptr;   // the build's result block is on the host
   cudaStream_t apply_stream = nullptr;  // pipelined builds: the apply pass's stream (nullptr: the build's)
@@ -839,9 +839,6 @@ static int world_create_impl(int dx, int dy, int dz, double vpm, uint32_t initia
   }
   cudaEventCreate(&w->ev0);
   cudaEventCreate(&w->ev1);
-  cudaEventCreate(&w->ev_fold0);
-  cudaEventCreate(&w->ev_fold1);
-  cudaEventCreate(&w->ev_mid);
   cudaEventCreateWithFlags(&w->ev_eval, cudaEventDisableTiming);
   cudaEventCreateWithFlags(&w->ev_done, cudaEventDisableTiming);
   // material tables (VoxelWorld.ts:159-170,190-196): filled by px_set_tables or the defaults
@@ -898,9 +895,6 @@ void px_world_destroy(px_world* w) {
   if (w->h_res) cudaFreeHost(w->h_res);
   if (w->ev0) cudaEventDestroy(w->ev0);
   if (w->ev1) cudaEventDestroy(w->ev1);
-  if (w->ev_fold0) cudaEventDestroy(w->ev_fold0);
-  if (w->ev_fold1) cudaEventDestroy(w->ev_fold1);
-  if (w->ev_mid) cudaEventDestroy(w->ev_mid);
   if (w->ev_eval) cudaEventDestroy(w->ev_eval);
   if (w->ev_done) cudaEventDestroy(w->ev_done);
   delete w;
@@ -1570,9 +1564,6 @@ px_world* twin_create(px_world* w, uint64_t P, uint32_t max_ops, int* rc) {
   }
   cudaEventCreate(&t->ev0);
   cudaEventCreate(&t->ev1);
-  cudaEventCreate(&t->ev_fold0);
-  cudaEventCreate(&t->ev_fold1);
-  cudaEventCreate(&t->ev_mid);
   cudaEventCreateWithFlags(&t->ev_eval, cudaEventDisableTiming);
   cudaEventCreateWithFlags(&t->ev_done, cudaEventDisableTiming);
   *rc = reserve_build_scratch(t, P, max_ops);  // its own scratch; the shared buffers are already sized
@@ -1818,6 +1809,7 @@ static int enqueue_build_derive(px_world* w, cudaStream_t s, const uint32_t* hol
   // counts kept by finalize, unless the material tables changed since: then recount
   da.pcount = w->pcount_valid ? w->d_pcount : nullptr;
   da.pcount_out = w->pcount_valid ? nullptr : w->d_pcount;
+  da.host = w->h_res;
   w->pcount_refresh = !w->pcount_valid;
   launch_derive(da, s);
   return PX_OK;
@@ -2061,10 +2053,8 @@ static int build_enqueue_impl(px_world* w, int mode, void* stream) {
   fa.res = res;
   int max_blocks = 0;  // persistent grids sized to the build (batched builds share the GPU)
   if (w->pairs_per_block) max_blocks = (int)std::max<uint64_t>(1, (P + w->pairs_per_block - 1) / w->pairs_per_block);
-  if (!w->capturing) CU(cudaEventRecord(w->ev_fold0, s));
-  launch_fold(fa, mode, w->n_sms, s, w->capturing ? nullptr : w->ev_mid, max_blocks, sa, w->ev_eval);
+  launch_fold(fa, mode, w->n_sms, s, max_blocks, sa, w->ev_eval);
   s = sa;  // the rest of the build follows the apply pass
-  if (!w->capturing) CU(cudaEventRecord(w->ev_fold1, s));
 
   ReplayArgs ra{};
   ra.P = P; ra.E_max = E_max; ra.H_max = H_max; ra.state = w->d_state;
@@ -2097,12 +2087,12 @@ static int build_enqueue_impl(px_world* w, int mode, void* stream) {
   fn.res = res;
   fn.opaque = (const uint8_t*)w->opaque.p;
   fn.pcount = w->d_pcount;
+  fn.host = w->derive_max ? nullptr : w->h_res;  // the build's last kernel hands its result to the host
   launch_finalize(fn, (uint32_t)touched_bound, s);
   if (w->derive_max && (rc = enqueue_build_derive(w, s, (const uint32_t*)holes_out.p))) return rc;
   CU(cudaGetLastError());
   w->stats.kernel_launches = (uint32_t)(launch_count() - launches0);
   if (!w->capturing) CU(cudaEventRecord(w->ev1, s));
-  CU(cudaMemcpyAsync(w->h_res, res, sizeof(BuildResult), cudaMemcpyDeviceToHost, s));
   if (!w->capturing) CU(cudaEventRecord(w->ev_done, s));
   w->in_flight = true;
   w->last_P = P;
@@ -2153,13 +2143,10 @@ static int build_finish_impl(px_world* w) {
   CU(cudaEventSynchronize(w->ev_done));  // the result block (later work on the stream may still run)
   w->uploads_pending = false;
   const BuildResult& r = *w->h_res;
-  float ms = 0.f, fold_ms = 0.f;
+  float ms = 0.f;
   cudaEventElapsedTime(&ms, w->ev0, w->ev1);
-  cudaEventElapsedTime(&fold_ms, w->ev_fold0, w->ev_fold1);
-  w->stats.fold_ms = fold_ms;
-  float cls_ms = 0.f;
-  cudaEventElapsedTime(&cls_ms, w->ev_fold0, w->ev_mid);
-  w->stats.classify_ms = cls_ms;
+  w->stats.fold_ms = (float)((double)(r.t_replay - r.t_classify) * 1e-6);
+  w->stats.classify_ms = (float)((double)(r.t_apply - r.t_classify) * 1e-6);
   w->stats.build_ms = ms;
   fill_stats(w, r);
   // transactional retries: nothing was committed
@@ -2197,6 +2184,7 @@ static int build_finish_impl(px_world* w) {
     CU(clear_poison());
     const uint32_t st2 = r.status & ~(uint32_t)ST_POOL_OVERFLOW;
     CU(cudaMemcpyAsync(&dres->status, &st2, 4, cudaMemcpyHostToDevice, w->stream));
+    CU(cudaMemsetAsync(&dres->done, 0, 4, w->stream));
     w->fin.pool32 = w->d_pool32;
     w->fin.pcount = w->d_pcount;
     w->fin.pool_cap = w->pool_cap;
@@ -2206,7 +2194,6 @@ static int build_finish_impl(px_world* w) {
       if ((rc = enqueue_build_derive(w, w->stream, (const uint32_t*)holes_after.p))) { w->retries = 0; return rc; }
     }
     CU(cudaGetLastError());
-    CU(cudaMemcpyAsync(w->h_res, dres, sizeof(BuildResult), cudaMemcpyDeviceToHost, w->stream));
     CU(cudaEventRecord(w->ev_done, w->stream));
     w->in_flight = true;
     rc = px_build_finish(w);

@@ -163,7 +163,9 @@ struct BuildResult {
   uint32_t n_rescue;     // voxels the float32 points left undecided (voxel_lean_kernel), pushed
   uint32_t h_before;     // holes before the build (from the WorldState)
   uint32_t u_before;     // poolUsed before the build
-  uint32_t pad2;
+  uint32_t done;         // blocks of the build's last kernel that have finished (publish_result)
+  // device clock (ns) at the start of the classify pass, the apply pass and the allocator replay
+  unsigned long long t_classify, t_apply, t_replay;
 };
 
 // Pair classification (state independent): class per (op, brick) pair, the 8
@@ -293,7 +295,7 @@ void launch_cull(const uint2* boxes, int n_ops, int TX, int TY, int TZ, uint32_t
 // max_blocks > 0 caps the persistent grids (builds sharing the GPU)
 // The evaluation passes (classify .. paint) go on s; the apply pass on s_apply,
 // after eval_done is recorded on s (s_apply == s: one stream, no event).
-void launch_fold(const FoldArgs& a, int mode, int n_sms, cudaStream_t s, cudaEvent_t mid, int max_blocks,
+void launch_fold(const FoldArgs& a, int mode, int n_sms, cudaStream_t s, int max_blocks,
                  cudaStream_t s_apply, cudaEvent_t eval_done);
 
 
@@ -364,6 +366,7 @@ struct FinalizeArgs {
   // written for every brick the build writes to the pool
   const uint8_t* opaque;
   uint16_t* pcount;
+  BuildResult* host;        // the build's last kernel: the result's copy in pinned host memory (else nullptr)
 };
 void launch_finalize(const FinalizeArgs& a, uint32_t touched_cap, cudaStream_t s);
 
@@ -407,6 +410,7 @@ struct DeriveArgs {
   // written to pcount_out
   const uint16_t* pcount;
   uint16_t* pcount_out;
+  BuildResult* host;        // a build's last step: the result's copy in pinned host memory
 };
 void launch_derive(const DeriveArgs& a, cudaStream_t s);
 // entries the GPU free list of a pool of `pool_cap` bricks can need
