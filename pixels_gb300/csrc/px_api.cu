@@ -2268,8 +2268,16 @@ static int world_reset_impl(px_world* w, int requeue_last_ops, void* stream) {
     CU(cudaStreamSynchronize(w->stream));
     w->uploads_pending = false;
   }
-  CU(cudaMemsetAsync(w->d_grid, 0, w->ncells * 4, (cudaStream_t)stream));
-  CU(cudaMemsetAsync(w->d_state, 0, sizeof(WorldState), (cudaStream_t)stream));
+  {  // one kernel instead of two memsets: 446 -> 442 us a replay of the penthouse at 80 voxels per
+     // metre, 1128 -> 1118 us one of twelve worlds
+    HostUploads hu{};
+    hu.e[0] = {nullptr, w->d_grid, w->ncells * 4, 0u};
+    hu.e[1] = {nullptr, w->d_state, sizeof(WorldState), 0u};
+    hu.n = 2;
+    set_programmatic_launch(false);
+    launch_uploads(hu, (cudaStream_t)stream);
+    CU(cudaGetLastError());
+  }
   w->pool_used = 0;
   w->n_holes = 0;
   w->derived_valid = false;
