@@ -86,6 +86,10 @@ PX_HD double px_round(double x) {
   return r;
 }
 
+// Math.round(n / 512 * 255) of a brick with n opaque voxels: n / 512 and the product are exact in
+// float64, so the rounding (half up) is that of the fraction 255 n / 512 (float64 units are slow here)
+PX_HD unsigned char density_byte(unsigned n) { return (unsigned char)((n * 255u + 256u) >> 9); }
+
 PX_HD double px_hypot2(double a, double b) {
   a = fabs(a);
   b = fabs(b);

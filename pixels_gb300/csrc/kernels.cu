@@ -3,20 +3,26 @@
 // Pipeline of one build (all on one stream, no host round trip):
 //   cull      one warp per 4^3-brick tile scans the op list (ballot) and keeps
 //             the ops whose brick box overlaps the tile, in op order.
-//   fold      persistent warps, one brick at a time: the brick's 512 voxels live
-//             in registers (two voxels per lane per z slice); the warp applies
-//             the brick's ops in order exactly as apply() does (shapes.ts:353-412):
-//             brick classify, 4^3 sub-block classify, boundary voxels, paint,
-//             uniform shortcuts, compaction.  Pool alloc/free events are
-//             recorded per (op, brick) pair; bricks that end non-uniform are
-//             written to a staging area.
+//   classify  every (op, brick) pair: skipped, full or partial (shapes.ts:358-366).
+//   sub       the eight 4^3 sub-blocks of the partial pairs (shapes.ts:382-389).
+//   voxel     the voxel masks of the partial sub-blocks (shapes.ts:390-394), one kernel
+//             per program form.
+//   paint     the paint values of the covered sub-blocks of painted ops, and the
+//             voxels that the voxel kernels left to float64.
+//   fold      the apply pass, persistent warps, one or four bricks per ticket: a brick's
+//             512 voxels live in registers (two voxels per lane per z slice); the
+//             warp applies the brick's ops in order exactly as apply() does
+//             (shapes.ts:353-412) from the results above: uniform shortcuts, masked
+//             writes, compaction.  Pool alloc/free events are recorded per (op,
+//             brick) pair; bricks that end non-uniform are written to a staging area.
 //   replay    parallel replay of the LIFO pool allocator (VoxelWorld.ts:112-127)
 //             over the events in (op, cell) order: clamped depth scan, match
 //             of each pop to its push (previous-smaller-value search on a
 //             32-ary min tree), pointer chasing of recycled indices.
 //   finalize  staging -> pool at the replayed indices (16-byte vector copies),
 //             grid entries.
-//   derive    super-grid counts and density bytes (GpuWorld.ts:90-101).
+//   derive    super-grid counts, density bytes (GpuWorld.ts:90-101) and the free list.
+// The last of them hands the build's result to the host.
 #include <algorithm>
 #include <cstdio>
 #include "px_internal.cuh"
@@ -39,6 +45,9 @@ namespace px {
 // scenes side by side 1,181 / 1,160 us in all
 #ifndef PX_TWO_CTA_PAIRS
 #define PX_TWO_CTA_PAIRS (1u << 19)
+#endif
+#ifndef PX_DERIVE_PER_SM
+#define PX_DERIVE_PER_SM 8
 #endif
 #ifndef PX_UPLOAD_BLOCKS
 #define PX_UPLOAD_BLOCKS 128
@@ -2454,7 +2463,7 @@ __device__ __forceinline__ void derive_world(const DeriveArgs& a) {
         nz += g != 0;
         if (g == 0) density[ci] = 0;
         else if (g & UNIFORM) density[ci] = udens[g & 0xffu];
-        else if (a.pcount) density[ci] = (uint8_t)px_round(((double)__ldg(a.pcount + (g - 1)) / 512.0) * 255.0);
+        else if (a.pcount) density[ci] = density_byte(__ldg(a.pcount + (g - 1)));
         else { is_mixed[h] = true; mixed_g[h] = g; mixed_ci[h] = ci; }
       }
     }
@@ -2477,7 +2486,7 @@ __device__ __forceinline__ void derive_world(const DeriveArgs& a) {
 #pragma unroll
         for (int o = 16; o; o >>= 1) cnt += __shfl_xor_sync(FULLMASK, cnt, o);
         if (lane == 0) {
-          density[ci] = (uint8_t)px_round(((double)cnt / 512.0) * 255.0);
+          density[ci] = density_byte(cnt);
           if (a.pcount_out) a.pcount_out[g - 1] = (uint16_t)cnt;
         }
       }
@@ -2534,10 +2543,16 @@ void launch_uploads(const HostUploads& u, cudaStream_t s) {
   launch_pdl(upload_kernel, dim3((unsigned)blocks, (unsigned)u.n), dim3(256), 0, s, u);
 }
 
+// A warp per super cell, one wave of blocks: every block is counted as it ends
+// (publish_result), so blocks past the wave cost more than their share.  Penthouse at 128
+// voxels per metre, a block per eight super cells / 8 blocks per SM / 4 / 2: 52.6 / 45.6 / 60 / 80 us;
+// at 80: 14.2 / 11.8 / 13.0 / 16.0 us.  The density bytes in integers then took them to 38.3 and 9.9.
 void launch_derive(const DeriveArgs& a, cudaStream_t s) {
   const int n_super = ((a.BX + 3) / 4) * ((a.BY + 3) / 4) * ((a.BZ + 3) / 4);
+  int dev = 0, n_sms = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
   const size_t b = ((size_t)n_super * 32 + 255) / 256;
-  launch_pdl(derive_kernel, dim3((unsigned)(b < 65535 ? b : 65535)), dim3(256), 0, s, a);
+  launch_pdl(derive_kernel, dim3((unsigned)std::min<size_t>(b, (size_t)n_sms * PX_DERIVE_PER_SM)), dim3(256), 0, s, a);
 }
 
 // ---------------------------------------------------------------------------
