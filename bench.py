@@ -338,12 +338,12 @@ def serving_section(args, pyoracle):
 
 # DRAM bytes per build from one ncu capture on the penthouse at vpm=80 (the
 # bench cannot run ncu itself): dram__bytes_read.sum + dram__bytes_write.sum of
-# the evaluation kernels (classify, sub-block, the four voxel kernels, paint,
-# apply) with caches flushed before each kernel, and of all 15 kernels of the
+# the evaluation kernels (classify, sub-block, the three voxel kernels, paint,
+# apply) with caches flushed before each kernel, and of all 14 kernels of the
 # build, flushed before each and left alone (the run's first build)
-EVAL_TRAFFIC_BYTES = 33_314_048
-BUILD_TRAFFIC_COLD_BYTES = 91_652_352
-BUILD_TRAFFIC_WARM_BYTES = 65_374_208
+EVAL_TRAFFIC_BYTES = 34_811_648
+BUILD_TRAFFIC_COLD_BYTES = 92_620_032
+BUILD_TRAFFIC_WARM_BYTES = 69_085_184
 
 
 def hbm_line(cfg, pool_used, ir_bytes, ms, derived_bytes=0):
@@ -696,12 +696,12 @@ def main():
         "roofline": {"bound": "fp32-alu", "achieved": round(achieved, 4), "peak": round(peak32, 2),
                      "unit": "TFLOP/s", "frac": round(achieved / peak32, 5), "traffic": EVAL_TRAFFIC_BYTES,
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the classify, sub-block, "
-                                       "voxel (4), paint and apply kernels of one build of this workload "
+                                       "voxel (3), paint and apply kernels of one build of this workload "
                                        "(one capture, caches flushed before each kernel, --clock-control none)",
                      "build_traffic": {"cold": BUILD_TRAFFIC_COLD_BYTES, "warm": BUILD_TRAFFIC_WARM_BYTES,
-                                       "what": "all 15 kernels of one build: caches flushed before each kernel "
+                                       "what": "all 14 kernels of one build: caches flushed before each kernel "
                                                "(cold), or left alone (warm, the run's first build)"},
-                     "kernel": "classify_kernel + sub_kernel + voxel_lean_kernel x3 + voxel_kernel + paint_kernel "
+                     "kernel": "classify_kernel + sub_kernel + voxel_lean_kernel x3 + paint_kernel "
                                "+ fold_kernel (every SDF and paint evaluation)",
                      "alg_ops_per_launch": int(alg_ops),
                      "fold_ms": round(fold_s * 1e3, 4),
