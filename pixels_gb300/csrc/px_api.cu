@@ -89,6 +89,14 @@ struct SubmitChunk {
   }
 };
 
+// How a cull table is laid out (launch_cull): the form, its (op, tile) pairs (CULL_FEW) and
+// its entries.
+struct CullPlan {
+  int how = CULL_SEQ;
+  uint32_t pairs = 0;
+  size_t n = 0;
+};
+
 // one host-to-device copy of a build's op tables
 struct Upload {
   void* dst;
@@ -127,11 +135,12 @@ struct px_world {
   hvec<uint2> boxes;
   hvec<OpLite> lite, last_lite;
   std::vector<SubmitChunk> chunks;  // conversion workspace of px_submit_ops, kept between lists
-  // the cull kernels' table as uploaded (cull_tables) and its scratch
+  // the cull kernels' table of the queued ops (cull_tables), its layout and its scratch
   hvec<uint2> h_boxes, h_groups;
   hvec<uint32_t> h_sort[4];
-  size_t n_cull = 0;            // its entries
+  CullPlan cull;
   bool cull_ready = false;      // it holds the queued ops
+  CullPlan dev_cull;            // the layout of the table on the device: the last one uploaded
   hvec<uint2> code;
   hvec<double> params;
   hvec<uint32_t> code32, last_code32;   // per instruction: float32 parameter offset
@@ -142,8 +151,6 @@ struct px_world {
 
   // per-build device scratch
   DevBuf d_ops, d_boxes, d_code, d_params, d_code32, d_p32, d_bases;
-  int cull_how = CULL_SEQ;
-  uint32_t cull_pairs = 0;      // CULL_FEW: (op, tile) pairs
   DevBuf tile_cnt, tile_off, tile_ops, tile_boxes;
   DevBuf evt, fsrc, pos, etype, ew, depth, tree, replay_tmp;
   DevBuf staging, stage_cell, stage_src, touched;
@@ -1389,9 +1396,7 @@ void cull_tables(px_world* w, int n_ops) {
       if (2 * pairs >= w->ntiles) break;
     }
     if (2 * pairs < w->ntiles) {
-      w->cull_how = CULL_FEW;
-      w->cull_pairs = (uint32_t)pairs;
-      w->n_cull = (size_t)n_ops + (n_ops + 1) / 2;
+      w->cull = {CULL_FEW, (uint32_t)pairs, (size_t)n_ops + (n_ops + 1) / 2};
       return;
     }
   }
@@ -1419,8 +1424,7 @@ void cull_tables(px_world* w, int n_ops) {
   };
   uint2* const groups = w->h_boxes.data() + n_ops;
   const uint64_t vol_seq = group_boxes(nullptr, groups);
-  w->cull_how = CULL_SEQ;
-  w->n_cull = (size_t)n_ops + n_groups;
+  w->cull = {CULL_SEQ, 0u, (size_t)n_ops + n_groups};
   if (n_ops > CULL_SORTED_MAX_OPS || n_groups <= 1) return;
   auto spread = [](uint32_t v) {  // 8 bits -> every third bit
     v = (v | (v << 8)) & 0x00f00fu;
@@ -1456,9 +1460,9 @@ void cull_tables(px_world* w, int n_ops) {
   }
   w->h_groups.resize(n_groups);
   if (2 * group_boxes(ord, w->h_groups.data()) >= vol_seq) return;
-  w->cull_how = CULL_SORTED;
+  w->cull.how = CULL_SORTED;
   std::memcpy(groups, w->h_groups.data(), sizeof(uint2) * n_groups);
-  for (int k = 0; k < n_ops; k += 2) w->h_boxes[w->n_cull++] = make_uint2(ord[k], k + 1 < n_ops ? ord[k + 1] : 0u);
+  for (int k = 0; k < n_ops; k += 2) w->h_boxes[w->cull.n++] = make_uint2(ord[k], k + 1 < n_ops ? ord[k + 1] : 0u);
 }
 
 // The build scratch that scales with the (op, brick) pairs P, the tile-list
@@ -1902,7 +1906,8 @@ static int build_enqueue_impl(px_world* w, int mode, void* stream) {
       cull_tables(w, n_ops);
       w->cull_ready = true;
     }
-    ups.push_back({w->d_boxes.p, w->h_boxes.data(), sizeof(uint2) * w->n_cull});
+    ups.push_back({w->d_boxes.p, w->h_boxes.data(), sizeof(uint2) * w->cull.n});
+    w->dev_cull = w->cull;  // (a list queued and dropped meanwhile does not touch the resident table's layout)
     ups.push_back({w->d_code.p, w->code.data(), sizeof(uint2) * w->code.size()});
     ups.push_back({w->d_params.p, w->params.data(), sizeof(double) * w->params.size()});
     ups.push_back({w->d_code32.p, w->code32.data(), sizeof(uint32_t) * w->code32.size()});
@@ -1974,7 +1979,7 @@ static int build_enqueue_impl(px_world* w, int mode, void* stream) {
   BuildResult* res = (BuildResult*)w->res.p;
   launch_cull((const uint2*)w->d_boxes.p, n_ops, w->TX, w->TY, w->TZ, (uint32_t*)w->tile_cnt.p,
               (uint32_t*)w->tile_off.p, (uint32_t*)w->tile_ops.p, (uint2*)w->tile_boxes.p,
-              (uint32_t*)w->chunk_counter.p + CULL_COUNTER, w->cull_how, w->cull_pairs,
+              (uint32_t*)w->chunk_counter.p + CULL_COUNTER, w->dev_cull.how, w->dev_cull.pairs,
               {(const OpDev*)w->d_ops.p, upload ? (const uint32_t*)w->chunk_dst.p : nullptr, (uint2*)w->chunk_op.p,
                (uint32_t)n_chunks, P},
               s);
