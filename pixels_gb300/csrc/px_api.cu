@@ -132,6 +132,7 @@ struct px_world {
   hvec<uint2> last_boxes, last_code;
   hvec<double> last_params;
   bool ops_resident = false;   // the device op tables already hold `ops`
+  bool last_resident = false;  // they hold `last_ops` (no table was reallocated or written since)
   hvec<uint2> boxes;
   hvec<OpLite> lite, last_lite;
   std::vector<SubmitChunk> chunks;  // conversion workspace of px_submit_ops, kept between lists
@@ -1465,6 +1466,16 @@ void cull_tables(px_world* w, int n_ops) {
   for (int k = 0; k < n_ops; k += 2) w->h_boxes[w->cull.n++] = make_uint2(ord[k], k + 1 < n_ops ? ord[k + 1] : 0u);
 }
 
+// Sizes of the buffers a resident op list lives in: one that was reallocated (ensure; always to
+// another size) has lost the list.
+struct OpTables {
+  size_t n[9];
+  explicit OpTables(const px_world* w)
+      : n{w->d_ops.bytes, w->d_boxes.bytes, w->d_code.bytes, w->d_params.bytes, w->d_code32.bytes,
+          w->d_p32.bytes, w->d_bases.bytes, w->chunk_op.bytes, w->chunk_dst.bytes} {}
+  bool operator!=(const OpTables& o) const { return std::memcmp(n, o.n, sizeof n) != 0; }
+};
+
 // The build scratch that scales with the (op, brick) pairs P, the tile-list
 // entries, the paint slots, the touched bricks, the allocator events E_max and
 // the staging slots.
@@ -1506,18 +1517,21 @@ namespace px {
 // pool so that such a build's staging guess fits.
 int reserve_build_scratch(px_world* w, uint64_t P, uint32_t max_ops) {
   if (w->in_flight || w->batch_locked) return fail(w, PX_E_INVALID_ARG, "the world is busy");
+  struct Track {  // whatever is allocated below, also by a reservation that fails half way
+    px_world* w;
+    OpTables before;
+    ~Track() {
+      if (OpTables(w) != before) w->ops_resident = w->last_resident = false;
+    }
+  } track{w, OpTables(w)};
   {  // op tables of up to max_ops one-instruction ops with up to 16 parameters and 64 bricks per axis
     const size_t n = max_ops ? max_ops : 1;
-    const void* before[7] = {w->d_ops.p, w->d_boxes.p, w->d_code.p, w->d_params.p, w->d_code32.p, w->d_p32.p, w->d_bases.p};
     int rc0;
     if ((rc0 = ensure(w, w->d_ops, sizeof(OpDev) * n)) || (rc0 = ensure(w, w->d_boxes, sizeof(uint2) * (n + (n + 31) / 32 + (n + 1) / 2))) ||
         (rc0 = ensure(w, w->d_code, sizeof(uint2) * n)) || (rc0 = ensure(w, w->d_params, sizeof(double) * 16 * n)) ||
         (rc0 = ensure(w, w->d_code32, sizeof(uint32_t) * n)) || (rc0 = ensure(w, w->d_p32, sizeof(float2) * 16 * n)) ||
         (rc0 = ensure(w, w->d_bases, sizeof(float2) * 192 * n)) || (rc0 = ensure(w, w->chunk_dst, 4 * n)))
       return rc0;
-    const void* after[7] = {w->d_ops.p, w->d_boxes.p, w->d_code.p, w->d_params.p, w->d_code32.p, w->d_p32.p, w->d_bases.p};
-    for (int k = 0; k < 7; k++)
-      if (after[k] != before[k]) w->ops_resident = false;  // a reallocated table lost its resident copy
   }
   const uint64_t touched_bound = P < w->ncells ? P : w->ncells;
   const size_t E_max = (size_t)w->pool_cap + 2 * P;  // the holes are pool bricks
@@ -1871,24 +1885,19 @@ static int build_enqueue_impl(px_world* w, int mode, void* stream) {
   if ((rc = grow_pool(w, (uint64_t)U0 + stage_cap, U0, s))) return rc;
 
   // scratch (a reallocated op table loses its resident copy)
-  const void* op_bufs_before[9] = {w->d_ops.p, w->d_boxes.p, w->d_code.p, w->d_params.p, w->d_code32.p,
-                                   w->d_p32.p, w->d_bases.p, w->chunk_op.p, w->chunk_dst.p};
-  if ((rc = ensure(w, w->d_ops, sizeof(OpDev) * (size_t)n_ops)) ||
+  const OpTables tables_before(w);
+  const bool no_room =
+      (rc = ensure(w, w->d_ops, sizeof(OpDev) * (size_t)n_ops)) ||
       (rc = ensure(w, w->d_boxes, sizeof(uint2) * ((size_t)n_ops + (n_ops + 31) / 32 + (n_ops + 1) / 2))) ||
       (rc = ensure(w, w->d_code, sizeof(uint2) * w->code.size())) ||
       (rc = ensure(w, w->d_params, sizeof(double) * w->params.size())) ||
       (rc = ensure(w, w->d_code32, sizeof(uint32_t) * w->code32.size())) ||
       (rc = ensure(w, w->d_p32, sizeof(float2) * w->p32.size())) ||
       (rc = ensure(w, w->d_bases, sizeof(float2) * w->bases.size())) || (rc = ensure(w, w->chunk_dst, 4 * (size_t)n_ops)) ||
-      (rc = ensure_pair_scratch(w, P, tile_pairs, n_slots, touched_bound, E_max, stage_cap)))
-    return rc;
+      (rc = ensure_pair_scratch(w, P, tile_pairs, n_slots, touched_bound, E_max, stage_cap));
+  if (OpTables(w) != tables_before) w->ops_resident = w->last_resident = false;
+  if (no_room) return rc;
   const uint32_t H_max = H;
-  {
-    const void* after[9] = {w->d_ops.p, w->d_boxes.p, w->d_code.p, w->d_params.p, w->d_code32.p,
-                            w->d_p32.p, w->d_bases.p, w->chunk_op.p, w->chunk_dst.p};
-    for (int k = 0; k < 9; k++)
-      if (after[k] != op_bufs_before[k]) w->ops_resident = false;
-  }
   DevBuf& holes_in = w->holes_in_a ? w->holes_a : w->holes_b;
   DevBuf& holes_out = w->holes_in_a ? w->holes_b : w->holes_a;
   if ((rc = ensure(w, holes_in, 4 * (size_t)H + 4)) || (rc = ensure(w, holes_out, 4 * E_max + 4))) return rc;
@@ -1900,6 +1909,7 @@ static int build_enqueue_impl(px_world* w, int mode, void* stream) {
   std::vector<Upload>& ups = w->h_uploads;
   ups.clear();
   if (upload) {
+    w->last_resident = false;  // (until this list is the last one built)
     ups.push_back({w->d_ops.p, w->ops.data(), sizeof(OpDev) * (size_t)n_ops});
     if (!w->cull_ready) {  // several lists were queued
       w->h_boxes.assign(w->boxes.begin(), w->boxes.end());
@@ -2220,6 +2230,7 @@ static int build_finish_impl(px_world* w) {
   w->n_holes = r.n_holes;
   w->holes_in_a = !w->holes_in_a;
   w->ops_applied += w->ops.size();
+  w->last_resident = true;
   w->last_ops.swap(w->ops);
   w->last_boxes.swap(w->boxes);
   w->last_lite.swap(w->lite);
@@ -2299,7 +2310,7 @@ static int world_reset_impl(px_world* w, int requeue_last_ops, void* stream) {
     w->p32 = w->last_p32;
     w->bases = w->last_bases;
     w->q = w->last_q;
-    w->ops_resident = true;  // the device tables of the last build still hold them
+    w->ops_resident = w->last_resident;  // the device tables of the last build, unless they were reallocated
   }
   return PX_OK;
 }

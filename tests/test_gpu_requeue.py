@@ -9,7 +9,7 @@ world of the last list.  Whole numbers, equal or wrong.
 import numpy as np
 import pytest
 
-from pixels_gb300 import _lib, config
+from pixels_gb300 import _lib, config, serving
 from pixels_gb300.batch import Batch
 from pixels_gb300.ir import Program
 from pixels_gb300.shapes import box, capsule, sphere
@@ -73,5 +73,28 @@ def test_requeue_after_a_list_that_is_not_built(built_lib, form, between, mode):
     else:
         _lib.world_reset(w._h, True)
         _lib.build(w._h, mode)
+        check(w, o)
+    w.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["rows", "scattered", "few"])
+@pytest.mark.parametrize("n", [0, 5])
+def test_requeue_after_serving_that_builds_nothing(built_lib, form, n):
+    """px_serve_run grows the op tables for its largest step before the first edit; with no
+    edit, or none that fits the pool, nothing is uploaded into them.  The requeued list is not
+    in the grown tables: it has to be uploaded again."""
+    prog = scene(form)
+    o = pyoracle.OracleWorld(prog.to_bytes(), VPM, DIMS, threads=8)
+    w = VoxelWorld(*DIMS, vpm=VPM, mode=MODE_MIXED)
+    w._pending = prog
+    w.build()
+    edits = [(0, (5.0, 5.0, 5.0 + i), (0.0, 0.0, 0.0), 1.0) for i in range(n)]
+    res, order = serving.serve(w, edits, np.zeros(n), max_batch=4096, pool_budget=w.liveBricks)
+    assert len(order) == 0 and (res["status"] == 3).all()
+    check(w, o)
+    for _ in range(2):  # uploaded again, then resident
+        _lib.world_reset(w._h, True)
+        _lib.build(w._h, MODE_MIXED)
         check(w, o)
     w.close()
