@@ -1327,7 +1327,11 @@ __device__ __forceinline__ uint32_t paint_voxel(const FoldArgs& a, const OpDev* 
 // the paint work of the others.  Paint pass of the synthetic scene (7,672 entries, 410 of
 // them left to float64; 129 us without any): two warps per SM 149 us, one 156, four 201,
 // every warp 189 to 211, and float64 at once in two 153; the penthouse at 80 voxels per
-// metre (870 entries, 37 us without): 41, 40, 42, 41 to 44, and 57 us.  A paint item of the
+// metre (870 entries, 37 us without): 41, 40, 42, 41 to 44, and 57 us.  A longer list
+// takes more warps: small grids (builds side by side, a few pairs per block) have few blocks,
+// and a warp's rounds follow each other.  Faces through voxel centres, 60,002 entries, two
+// warps per SM only / as here: one block 9.7 / 2.7 ms a pass, ten blocks 1.9 / 0.30 ms, the
+// whole GPU 187 / 184 us.  A paint item of the
 // same sub-block may read its mask before or after the OR: it then paints the voxel too
 // or leaves it out, and either way stores the same value.
 template <int MODE>
@@ -1338,10 +1342,12 @@ __global__ void __launch_bounds__(256, PX_PAINT_MINB) paint_kernel(FoldArgs a) {
   if (MODE == 1) {
     LaneStats ls = {a.res};
     const uint32_t n_resc = min(__ldcg(&a.res->n_rescue), a.rescue_cap);
-    // one warp of each of half the blocks takes consecutive entries
-    const uint32_t nb = (gridDim.x + 1) / 2, per = (n_resc + nb - 1) / nb;
-    const uint32_t end = threadIdx.x < 32 && blockIdx.x < nb ? min(n_resc, (blockIdx.x + 1) * per) : 0u;
-    for (uint32_t r = blockIdx.x * per + (uint32_t)lane; r < end; r += 32) {
+    // one warp of each of half the blocks takes consecutive entries; a list longer than
+    // 32 for each of these is spread over more warps of more blocks, up to all
+    const uint32_t n_take = min(gridDim.x * (blockDim.x >> 5), max((gridDim.x + 1) / 2, (n_resc + 31) / 32));
+    const uint32_t me = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, per = (n_resc + n_take - 1) / n_take;
+    const uint32_t end = me < n_take ? min(n_resc, (me + 1) * per) : 0u;
+    for (uint32_t r = me * per + (uint32_t)lane; r < end; r += 32) {
       const uint4 ri = __ldcg(a.rescue + r);
       const OpDev* R = a.ops + (ri.x & 0xffffffu);
       const int bit = (int)((ri.x >> 24) & 63u);
