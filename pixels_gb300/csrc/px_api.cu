@@ -690,6 +690,39 @@ static void lean_error(const OpDev& d, const float2* p32, const float2* bases, c
   }
 }
 
+// A Lipschitz constant of the value of a (valid) program, from its parameters.  What the shape
+// constructors make has constant 1, but an op list may hold any parameters: a rotation whose
+// cos^2 + sin^2 is not 1 scales, as may an ellipsoid's factor or a capsule's 1 / |e|^2 that do not
+// fit the rest.  Every primitive is a distance to a set, or such distances of its axes combined
+// by minima, maxima and lengths (constant 1: shapes.ts:40-218); a polygon's sign changes only
+// where its distance is 0; offsets and combinators keep the larger constant.
+double program_lipschitz(const uint32_t* code, uint32_t n, const double* P) {
+  double scale[DEEP_MAX_ROT + 1], L = 1;
+  int r = 0;
+  scale[0] = 1;
+  for (uint32_t i = 0; i < n; i++) {
+    const double* p = P + code[2 * i + 1];
+    double l = 1;
+    switch (code[2 * i] & 0xffu) {
+      case OP_ROT_X: case OP_ROT_Y: case OP_ROT_Z:
+        scale[r + 1] = scale[r] * std::max(1.0, std::sqrt(p[2] * p[2] + p[3] * p[3]));
+        r++;
+        break;
+      case OP_ROT_END: r--; break;
+      case OP_ELLIPSOID:  // (|q / radii| - 1) * factor
+        l = std::fabs(p[6]) / std::min(std::min(std::fabs(p[3]), std::fabs(p[4])), std::fabs(p[5]));
+        break;
+      case OP_CAPSULE:  // q - e clamp(q . e / b): along e, 1 - |e|^2 / b between the clamps
+        l = std::fabs(1 - (p[3] * p[3] + p[4] * p[4] + p[5] * p[5]) / p[6]);
+        break;
+      default: break;
+    }
+    L = std::max(L, scale[r] * std::max(1.0, l));
+    if (!(l <= 1e300)) return std::numeric_limits<double>::infinity();  // (NaN too)
+  }
+  return L <= 1 + 0x1p-44 ? 1.0 : L;  // (the roundings of 16 nested rotations and of this)
+}
+
 // Validate one op's SDF bytecode: opcodes, parameter ranges, finite values,
 // stack and rotation depths.  `deep` is set when the program needs more than
 // the register evaluators hold (it then runs on the deep float64 evaluator).
@@ -1180,9 +1213,12 @@ int convert_ops(const px_world* w, const IrOp* iops, size_t i0, size_t i1, const
       d.thr[T_M] = ru32(M);
       // Lipschitz decisions of voxels from their sub-block centre's value: a voxel
       // centre lies sqrt(n1 + 9 n3) / 2 voxels from the centre (n3 axes at offset
-      // 1.5, the others at 0.5), plus the float64 rounding of both points
+      // 1.5, the others at 0.5), plus the float64 rounding of both points.  A program that
+      // stretches distances beyond MAX_LIPSCHITZ takes none: every voxel in float64
+      const double lip_program = program_lipschitz(code + 2 * (size_t)o.code_begin, o.code_len, P);
+      if (!(lip_program <= MAX_LIPSCHITZ)) d.flags |= OPF_FP64_ONLY;
       {
-        const double L = std::max(1.0, o.slack) * (1 + 0x1p-40);
+        const double L = std::max(lip_program, o.slack) * (1 + 0x1p-40);
         const double dist[4] = {std::sqrt(3.0) / 2, std::sqrt(11.0) / 2, std::sqrt(19.0) / 2, std::sqrt(27.0) / 2};
         for (int k = 0; k < 4; k++) d.lip[k] = ru32(L * (dist[k] * vs + 0x1p-40) + M);
       }

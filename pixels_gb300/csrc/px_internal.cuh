@@ -46,6 +46,9 @@ constexpr uint8_t OPF_FROM_IR = OPF_CONTAINS | OPF_HAS_SLACK | OPF_PAINT_FRAME; 
 // inputs and the reference's float64 result (valid for |values| <= 2^10 m).
 constexpr double MIXED_MARGIN = 0x1p-30;
 constexpr double MIXED_MAX_COORD = 1024.0;
+// the largest Lipschitz constant of a program (1 for the shape constructors') within that margin:
+// it scales coordinates of 2^10 m, some 20 roundings of 2^-53 each, to 2^-34 m
+constexpr double MAX_LIPSCHITZ = 16.0;
 
 // per-op float32 thresholds of the mixed mode (certified comparisons)
 enum { T_BSK_HI, T_BSK_LO, T_BFU_HI, T_BFU_LO, T_SSK_HI, T_SSK_LO, T_SFU_HI, T_SFU_LO, T_V_HI, T_V_LO, T_M, T_COUNT };
@@ -98,7 +101,7 @@ struct alignas(128) OpDev {
 
   // mixed mode: a voxel of a partial sub-block is outside if the sub-block centre's
   // value exceeds lip[k], inside if it is below -lip[k] (k: the voxel's distance class
-  // from the centre; every shape's SDF is Lipschitz with constant <= its slack)
+  // from the centre; the constant is the program's own, program_lipschitz, or the larger slack)
   float lip[4];
   float err[2];                          // error bounds of a lean program's float32 points, per primitive (plus the margin)
   uint32_t vclass;                       // sub-block work class (VCLASSES): first primitive, y-extruded
