@@ -990,10 +990,29 @@ __device__ __forceinline__ int lip_decide(const OpDev* O, Iv dc, int ox, int oy,
   return dc.lo > t ? 0 : (dc.hi < -t ? 1 : 3);
 }
 
+// A voxel the float32 points left undecided ([lo, hi]: its enclosure): float32 intervals,
+// which follow this voxel's magnitudes instead of the op's largest, then float64.  Returns
+// the decision.  Out of line: a few voxels in a build.
+__device__ __noinline__ int rescue_voxel(const FoldArgs& a, const OpDev* R, int bx, int by, int bz, int lx, int ly, int lz,
+                                         Iv dk, LaneStats& ls) {
+  Iv bo[3];
+  brick_bases(a, R, bx, by, bz, bo);
+  bool amb = false;
+  const Iv d = sdf32i(a.code + R->code_off, a.code32 + R->code_off, (int)R->code_len, reinterpret_cast<const Iv*>(a.p32),
+                      iadd(bo[0], koff((float)lx, a.vs_lo, a.vs_hi)), iadd(bo[1], koff((float)ly, a.vs_lo, a.vs_hi)),
+                      iadd(bo[2], koff((float)lz, a.vs_lo, a.vs_hi)), R->thr[T_M], amb);
+  if (!amb && d.lo > R->thr[T_V_HI]) return 0;
+  if (!amb && d.hi <= R->thr[T_V_LO]) return 1;
+  const VoxelF64 f = voxel_f64(a.params, a.vs, 0, a.code + R->code_off, (int)R->code_len, dk, false, 3,
+                               (float)(bx * 8 + lx) + 0.5f, (float)(by * 8 + ly) + 0.5f, (float)(bz * 8 + lz) + 0.5f);
+  ls.rescue(0, amb, f.err);
+  return f.inside;
+}
+
 // Voxel inside-masks of the queued partial sub-blocks: one sub-block per warp
 // pass, 64 voxel SDFs on 32 lanes, two ballots (shapes.ts:390-394), any
-// program (the bytecode interpreters); a voxel its float32 interval cannot
-// decide is evaluated in float64 in line.  Groups G0 .. G1 of the voxel queue, one
+// program (the bytecode interpreters, lean programs' points first); a voxel its
+// float32 interval cannot decide is evaluated in float64 in line.  Groups G0 .. G1 of the voxel queue, one
 // after the other (the mixed form sends the lean programs' groups to
 // voxel_lean_kernel and this kernel the rest; the float64 form every group here).
 template <int MODE, int G0, int G1>
@@ -1036,7 +1055,35 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_VOXEL_MINB : PX_CLASSIFY64
     const uint2* code = a.code + V->code_off;
     const int clen = (int)V->code_len;
     unsigned long long m;
-    if (MODE == 1 && use32 && (V->flags & OPF_Y_SEPARABLE)) {
+    if (MODE == 1 && V->lw[0] && !a.validate) {
+      // a lean program whose float32 points leave more voxels undecided than the rescue list
+      // should hold (LEAN_BOUND .. POINT_BOUND): its points first, the rest in intervals and
+      // float64 here.  Voxel pass of a box of 60 m and a capsule of 30 at 160 voxels per metre:
+      // the interpreter for every voxel 148 and 198 us
+      const int lx = lane & 3, lyv = (lane >> 2) & 3, lz = lane >> 4;  // and lz + 2
+      const int x = sxo + lx, y = syo + lyv, z = szo + lz;
+      const float zp[2] = {coord_f(bo[2].lo, (float)z, a.vs_lo), coord_f(bo[2].lo, (float)(z + 2), a.vs_lo)};
+      float lo[2], hi[2];
+      lean_f<2, 3, true, true>(a, V, coord_f(bo[0].lo, (float)x, a.vs_lo), coord_f(bo[1].lo, (float)y, a.vs_lo), zp, lo, hi);
+      uint32_t bal[2], open = 0, late = 0;  // open: bit q, this lane's voxel q is undecided
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const int lip = lip_decide(V, dcen, lx, lyv, lz + 2 * q);
+        const int inside = lip != 3 ? lip : lo[q] > 0.f ? 0 : hi[q] < 0.f ? 1 : 3;
+        bal[q] = __ballot_sync(FULLMASK, inside == 1);
+        open |= (uint32_t)(inside == 3) << q;
+      }
+      while (__any_sync(FULLMASK, open)) {  // seldom more than once: few are undecided, and few lanes hold two
+        const int q = open & 1u ? 0 : 1;
+        if (open && rescue_voxel(a, V, vbx, vby, vbz, x, y, z + 2 * q, q ? Iv{lo[1], hi[1]} : Iv{lo[0], hi[0]}, ls) == 1)
+          late |= 1u << q;
+        open &= open - 1;
+        __syncwarp();
+      }
+      bal[0] |= __ballot_sync(FULLMASK, late & 1u);
+      bal[1] |= __ballot_sync(FULLMASK, late & 2u);
+      m = (unsigned long long)bal[0] | ((unsigned long long)bal[1] << 32);
+    } else if (MODE == 1 && use32 && (V->flags & OPF_Y_SEPARABLE)) {
       // lane = column (x, z) of the sub-block and a pair of y rows: one pass, the x/z work once
       const int col = lane & 15, yh = lane >> 4;
       const int lx = sxo + (col & 3), lz = szo + (col >> 2), ly0 = syo + 2 * yh;
@@ -1238,25 +1285,6 @@ __global__ void __launch_bounds__(256, G == VQ_WIDE ? PX_VWIDE_MINB : G == VQ_AF
       }
     }
   }
-}
-
-// A voxel the float32 points left undecided ([lo, hi]: its enclosure): float32 intervals,
-// which follow this voxel's magnitudes instead of the op's largest, then float64.  Returns
-// the decision.  Out of line: a few voxels in a build.
-__device__ __noinline__ int rescue_voxel(const FoldArgs& a, const OpDev* R, int bx, int by, int bz, int lx, int ly, int lz,
-                                         Iv dk, LaneStats& ls) {
-  Iv bo[3];
-  brick_bases(a, R, bx, by, bz, bo);
-  bool amb = false;
-  const Iv d = sdf32i(a.code + R->code_off, a.code32 + R->code_off, (int)R->code_len, reinterpret_cast<const Iv*>(a.p32),
-                      iadd(bo[0], koff((float)lx, a.vs_lo, a.vs_hi)), iadd(bo[1], koff((float)ly, a.vs_lo, a.vs_hi)),
-                      iadd(bo[2], koff((float)lz, a.vs_lo, a.vs_hi)), R->thr[T_M], amb);
-  if (!amb && d.lo > R->thr[T_V_HI]) return 0;
-  if (!amb && d.hi <= R->thr[T_V_LO]) return 1;
-  const VoxelF64 f = voxel_f64(a.params, a.vs, 0, a.code + R->code_off, (int)R->code_len, dk, false, 3,
-                               (float)(bx * 8 + lx) + 0.5f, (float)(by * 8 + ly) + 0.5f, (float)(bz * 8 + lz) + 0.5f);
-  ls.rescue(0, amb, f.err);
-  return f.inside;
 }
 
 // One paint call at voxel (x, y, z) of the world, in float64 (the paint kinds

@@ -1242,10 +1242,11 @@ int convert_ops(const px_world* w, const IrOp* iops, size_t i0, size_t i1, const
           ysep = ysep && op_is_y_separable(code[2 * ((size_t)o.code_begin + k)] & 0xffu);
         if (ysep) d.flags |= OPF_Y_SEPARABLE;
         d.vclass = (first_prim & 15u) | (ysep && !(d.flags & OPF_FP64_ONLY) ? 16u : 0u);
-        // a lean program (LP_* forms), where its float32 points decide all but a few voxels: an
-        // error bound of up to 1/128 voxel leaves at most about one in 300 near the surface
-        // undecided (shapes of some 50 m at 80 voxels per metre; larger ones take the
-        // interpreter).  A second primitive may be far away, and its bound larger
+        // a lean program (LP_* forms) of the lean kernels, where its float32 points decide all but
+        // a few voxels: an error bound of up to LEAN_BOUND voxels leaves at most about one in 300
+        // near the surface to the rescue list (shapes of some 50 m at 80 voxels per metre).  A
+        // second primitive may be far away, and its bound larger.  Up to POINT_BOUND voxels the
+        // points still decide most and come first, before the interpreter, in the same kernels
         uint8_t lp[8] = {0};
         const uint32_t* oc = code + 2 * (size_t)o.code_begin;
         if (!(d.flags & (OPF_FP64_ONLY | OPF_DEEP)) && d.bx0 <= d.bx1) lean_program(oc, o.code_len, lp);
@@ -1266,12 +1267,15 @@ int convert_ops(const px_world* w, const IrOp* iops, size_t i0, size_t i1, const
           const int nb[3] = {d.bx1 - d.bx0 + 1, d.by1 - d.by0 + 1, d.bz1 - d.bz0 + 1};
           double E[2];
           lean_error(d, out.p32.data(), out.bases.data() + d.base_off, nb, rd32(vs), ru32(vs), E);
-          if (E[0] <= vs / 128 && E[1] <= vs / 32) {
+          const bool lean = E[0] <= vs * LEAN_BOUND && E[1] <= vs * LEAN_BOUND2;
+          if (lean || std::max(E[0], E[1]) <= vs * POINT_BOUND) {
             d.err[0] = ru32(E[0]);
             d.err[1] = ru32(E[1]);
           } else {
-            for (int k = 0; k < 8; k++) { d.lw[k] = 0; lp[k] = 0; }
+            for (int k = 0; k < 8; k++) d.lw[k] = 0;
           }
+          if (!lean)
+            for (int k = 0; k < 8; k++) lp[k] = 0;
         }
         // the voxel queue's group and class: one primitive under at most one rotation
         // (by primitive and rotation), the other lean forms (by first primitive and

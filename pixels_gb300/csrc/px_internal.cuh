@@ -93,10 +93,10 @@ struct alignas(128) OpDev {
   int32_t bx0, by0, bz0, bx1, by1, bz1;  // brick box (inclusive), from apply()'s voxel range
   int32_t nx, ny;                        // box extent in bricks (x, y)
 
-  // a lean program (LP_* forms; lw[0] == 0: not one), all a kernel needs of it in two
-  // 16-byte loads: form | combinator << 8 | first stage's kind << 16 | second's << 20 |
-  // has an offset << 24; first primitive (opcode | count << 8), its parameters and its
-  // stage's (p32 indices); the second primitive's three; the offset's parameter
+  // a lean program (LP_* forms; lw[0] == 0: not one, or its bound is past POINT_BOUND), all a
+  // kernel needs of it in two 16-byte loads: form | combinator << 8 | first stage's kind << 16 |
+  // second's << 20 | has an offset << 24; first primitive (opcode | count << 8), its parameters and
+  // its stage's (p32 indices); the second primitive's three; the offset's parameter
   uint32_t lw[8];
 
   // mixed mode: a voxel of a partial sub-block is outside if the sub-block centre's
@@ -199,6 +199,13 @@ constexpr int CULL_COUNTER = 200;         // chunk_counter[CULL_COUNTER]: tile-l
 // subtract step, an intersection or a union.
 enum { LP_FORM, LP_COMB, LP_P1, LP_P2, LP_S1, LP_S2, LP_KINDS, LP_OFF };  // lean_program's reading (host)
 enum : uint8_t { LP_NEGMAX = 1, LP_MAX = 2, LP_MIN = 3, LP_NONE = 0xff, LP_AFFINE = 4 };
+// Largest error bounds of a lean program's float32 points, in voxels: of a program of the lean
+// voxel kernels (first primitive, second), and of one whose points the generic voxel kernel tries
+// before the interpreter.  Shapes of 30 to 120 m at 160 voxels per metre, past the first bound,
+// whole passes without / with points: 12-sided prisms 562 / 404 and 580 / 433 us, rotated boxes 325 / 267
+// and 359 / 312, capsules 390 / 319 and 386 / 336; of 400 m a sphere 514 / 408, a cylinder 316 / 339.
+// A last bound of 1/8 keeps the 120 m prism at 595 us, one of 1 takes one of 400 m from 630 to 1,061
+constexpr double LEAN_BOUND = 1.0 / 128, LEAN_BOUND2 = 1.0 / 32, POINT_BOUND = 1.0 / 2;
 // code32 flags of the float32 path: a run of rotations (not all about y) composed
 // into an affine map on its first rotation; its other rotations and all but the
 // first of its ends are skipped
