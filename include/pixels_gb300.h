@@ -162,8 +162,9 @@ int px_snap_anchors(px_world* w, const int32_t* xyz, size_t n, const uint8_t* em
    density of a uniform brick of material id (VoxelWorld.ts:162).  256 bytes each. */
 int px_set_material_tables(px_world* w, const uint8_t* opaque256, const uint8_t* uniform_density256);
 
-/* Validation mode for the mixed form (testing aid, slow): every float32
-   evaluation is also done in float64 and checked against its enclosure;
+/* Validation mode (testing aid, slow): every float32 evaluation of the mixed form is
+   also done in float64 and checked against its enclosure, and in both forms every
+   voxel that a sub-block's centre would settle is evaluated and compared;
    stats.violations counts failures (must stay 0). */
 int px_set_validation(px_world* w, int on);
 

@@ -1287,6 +1287,71 @@ __global__ void __launch_bounds__(256, G == VQ_WIDE ? PX_VWIDE_MINB : G == VQ_AF
   }
 }
 
+// Validation mode, a lean program's float32 point at a brick's centre (what 1), a sub-block's (2) or
+// a voxel's (0), at offsets k from the brick's first voxel centre: does the float64 value d lie
+// outside its enclosure, or decide otherwise?
+__device__ __forceinline__ bool lean_disagrees(const FoldArgs& a, const OpDev* O, const float (&b)[3], float kx, float ky,
+                                               float kz, double d, int what) {
+  const float z[1] = {coord_f(b[2], kz, a.vs_lo)};
+  float lo[1], hi[1];
+  lean_f<1, 3, true, true>(a, O, coord_f(b[0], kx, a.vs_lo), coord_f(b[1], ky, a.vs_lo), z, lo, hi);
+  if (!(lo[0] == lo[0] && hi[0] == hi[0])) return false;  // undecided
+  if (!(lo[0] <= d && d <= hi[0])) return true;
+  if (what == 0) return d > 0.0 ? hi[0] < 0.f : lo[0] > 0.f;
+  const int c = classify32({lo[0], hi[0]}, O->thr, what == 1 ? T_BSK_HI : T_SSK_HI);
+  return c != 3 && c != classify64(d, what == 1 ? O->bhd : O->shd);
+}
+
+// Validation mode: what the passes above take instead of an evaluation, against float64, per
+// (op, brick) pair: the points of lean programs at the brick's centre, the sub-blocks' and the boundary
+// voxels, and the voxels that a sub-block centre settles (lip_decide; from the float64 centre, the
+// tightest enclosure).  A warp per pair; only counts violations.
+template <int MODE>
+__global__ void __launch_bounds__(256) validate_kernel(FoldArgs a) {
+  pdl_prologue();
+  const int lane = threadIdx.x & 31;
+  LaneStats ls = {a.res};
+  const unsigned long long n_warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
+  for (unsigned long long p = (unsigned long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); p < a.n_pairs; p += n_warps) {
+    uint32_t o = 0;  // the pair's op: the last one whose first pair is at or below p
+    for (uint32_t end = a.n_ops; end - o > 1;) {
+      const uint32_t mid = o + (end - o) / 2;
+      if (a.ops[mid].pair_base <= p) o = mid;
+      else end = mid;
+    }
+    const OpDev* O = a.ops + o;
+    if (O->flags & OPF_FP64_ONLY) continue;  // evaluated everywhere
+    const bool lean = MODE == 1 && O->lw[0];
+    int bx, by, bz;
+    brick_of_pair(O, p, bx, by, bz);
+    float b[3] = {0.f, 0.f, 0.f};
+    if (lean) brick_bases_f(a, O, bx, by, bz, b);
+    auto at = [&](float x, float y, float z) {  // in voxels from the brick's corner
+      return sdf64_at(a.code + O->code_off, (int)O->code_len, a.params, a.vs, (float)(bx * 8) + x, (float)(by * 8) + y,
+                      (float)(bz * 8) + z);
+    };
+    if (lean && lean_disagrees(a, O, b, 3.5f, 3.5f, 3.5f, at(4.f, 4.f, 4.f), 1) && lane == 0) ls.viol();
+    if (a.pcode[p] != PC_PARTIAL) continue;
+    const uint32_t sc = a.psub[p];
+#pragma unroll 1
+    for (int s = 0; s < 8; s++) {
+      const int x0 = (s & 1) * 4, y0 = ((s >> 1) & 1) * 4, z0 = (s >> 2) * 4;
+      const double dc = at(x0 + 2.f, y0 + 2.f, z0 + 2.f);
+      if (lean && lean_disagrees(a, O, b, x0 + 1.5f, y0 + 1.5f, z0 + 1.5f, dc, 2) && lane == 0) ls.viol();
+      if (((sc >> (2 * s)) & 3u) != PC_PARTIAL) continue;
+      const Iv c = {__double2float_rd(dc - MIXED_MARGIN), __double2float_ru(dc + MIXED_MARGIN)};
+#pragma unroll 1
+      for (int e = lane; e < 64; e += 32) {
+        const int x = x0 + (e & 3), y = y0 + ((e >> 2) & 3), z = z0 + (e >> 4);
+        const double d = at(x + 0.5f, y + 0.5f, z + 0.5f);
+        const int lip = lip_decide(O, c, e & 3, (e >> 2) & 3, e >> 4);
+        if (lip == (d > 0.0 ? 1 : 0)) ls.viol();
+        if (lean && lean_disagrees(a, O, b, (float)x, (float)y, (float)z, d, 0)) ls.viol();
+      }
+    }
+  }
+}
+
 // One paint call at voxel (x, y, z) of the world, in float64 (the paint kinds
 // that paint_kernel does not evaluate ahead).  Out of line, so that the apply
 // loop holds no float64 values.  Returns the value (a u16 for these kinds) with
@@ -1845,6 +1910,7 @@ void launch_fold(const FoldArgs& a, int mode, int n_sms, cudaStream_t s, int max
     launch_pdl(sub_kernel<0, PX_CLASSIFY64_MINB>, dim3(grid(PX_CLASSIFY64_MINB)), dim3(256), 0, s, a);
     launch_pdl(voxel_kernel<0, VQ_NARROW, VQ_GENERIC>, dim3(grid(PX_CLASSIFY64_MINB)), dim3(256), 0, s, a);
   }
+  if (a.validate) launch_pdl(mode == 1 ? validate_kernel<1> : validate_kernel<0>, dim3(grid(4)), dim3(256), 0, s, a);
   // the mixed form's paint pass also resolves the lean voxel kernels' rescue list
   if (mode == 1) launch_pdl(paint_kernel<1>, dim3(grid(4)), dim3(256), 0, s, a);
   else if (a.n_paint_slots) launch_pdl(paint_kernel<0>, dim3(grid(4)), dim3(256), 0, s, a);
