@@ -140,8 +140,8 @@ int px_set_derive_on_build(px_world* w, uint32_t max_bricks);
    current; make it before any stream capture on that device, and do not call
    it on a device reset (cudaDeviceReset) since that first call.  grid, pool
    and super_counts must be 4-byte aligned (else PX_E_INVALID_ARG, no GPU
-   work).  All calls share the area, so calls that overlap in time race:
-   serialise them.  Returns after the work on `stream` has finished;
+   work).  All calls on a device share its area, so calls on one device that
+   overlap in time race: serialise them.  Returns after the work on `stream` has finished;
    PX_E_INVALID_ARG also when the grid names a pool brick >= n_pool_bricks
    (that cell's density is written as 0). */
 #define PX_NOALLOC_MAX_POOL_BRICKS 1048576u

@@ -18,12 +18,13 @@
 // PX_E_TOO_LARGE before any GPU work.
 //
 // Status: a cell that names a brick beyond the pool is reported through a word
-// of host memory that the kernel can write (a page of this library's own data,
-// registered on first use): it stores the call's number there, so nothing is
-// cleared before the kernels and nothing copied back after them.
+// of host memory that the kernel can write (one per device, in a page of this
+// library's own data, registered on first use and for the rest of the process): it
+// stores the call's number there, so nothing is cleared before the kernels and nothing
+// copied back after them.
 //
 // Set-up: the first call on each device, with that device current, looks up
-// the array's device address (cudaGetSymbolAddress) and the status page's, and
+// the array's device address (cudaGetSymbolAddress) and the status word's, and
 // keeps them for later calls on that device.  Make the first call on a device
 // before any stream capture is begun on it.  The kept addresses belong to the
 // device's current context: after cudaDeviceReset (which unloads the library's
@@ -35,9 +36,10 @@
 // those three addresses must be multiples of 4 bytes (a uint16 pool that starts at
 // an odd element is refused with PX_E_INVALID_ARG before any GPU work).
 //
-// Every call shares the array and the status page: calls that overlap in time
-// (from several host threads, or on several streams) race on them and may return
-// wrong results.  Callers serialise them.  The counts are written for every pool
+// Every call on a device shares its array and status word: calls on one device that
+// overlap in time (from several host threads, or on several streams) race on them and
+// may return wrong results.  Callers serialise them.  Calls on different devices share
+// nothing.  The counts are written for every pool
 // brick before they are read, so they need no clearing.
 #include <cuda_runtime.h>
 
@@ -172,11 +174,15 @@ __global__ void __launch_bounds__(256) noalloc_cells_kernel(const uint32_t* __re
 }
 
 std::mutex g_setup_mu;
-alignas(4096) uint32_t g_status_page[1024];  // word 0: the number of the last call that met a bad cell
+constexpr int STATUS_STRIDE = 16;  // words: a line of 64 bytes per device
+// word STATUS_STRIDE d: the number of the last call on device d that met a bad cell
+alignas(4096) uint32_t g_status_page[MAX_DEVICES * STATUS_STRIDE];
+static_assert(sizeof g_status_page % 4096 == 0, "whole pages are registered");
 bool g_registered = false;
 struct Addresses {
   uint16_t* scratch;
-  uint32_t* status;
+  uint32_t* status;           // the device's word, as the device sees it
+  volatile uint32_t* report;  // and as the host does
 } g_addr[MAX_DEVICES];
 std::atomic<uint32_t> g_calls{0};
 
@@ -191,18 +197,19 @@ int addresses_for_current_device(Addresses* out) {
   std::lock_guard<std::mutex> g(g_setup_mu);
   if (!g_addr[dev].scratch) {
     void *p = nullptr, *q = nullptr;
+    uint32_t* const word = g_status_page + dev * STATUS_STRIDE;
     if (!g_registered && cudaHostRegister(g_status_page, sizeof g_status_page,
                                           cudaHostRegisterMapped | cudaHostRegisterPortable) != cudaSuccess) {
       cudaGetLastError();
       return PX_E_CUDA;
     }
     g_registered = true;
-    if (cudaHostGetDevicePointer(&q, g_status_page, 0) != cudaSuccess || !q ||
+    if (cudaHostGetDevicePointer(&q, word, 0) != cudaSuccess || !q ||
         cudaGetSymbolAddress(&p, g_derive_scratch) != cudaSuccess || !p) {
       cudaGetLastError();
       return PX_E_CUDA;
     }
-    g_addr[dev] = {(uint16_t*)p, (uint32_t*)q};
+    g_addr[dev] = {(uint16_t*)p, (uint32_t*)q, word};
   }
   *out = g_addr[dev];
   return PX_OK;
@@ -255,5 +262,5 @@ extern "C" int px_derive_noalloc(const uint32_t* grid, const uint16_t* pool, int
     cudaGetLastError();
     return PX_E_CUDA;
   }
-  return *(volatile uint32_t*)g_status_page == call ? PX_E_INVALID_ARG : PX_OK;
+  return *at.report == call ? PX_E_INVALID_ARG : PX_OK;
 }
