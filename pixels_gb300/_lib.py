@@ -149,8 +149,8 @@ def world_destroy(h):
 
 
 def submit_ops(h, ir: bytes):
-    if not isinstance(ir, bytes):  # read in place when immutable
-        ir = bytes(ir)
+    if not isinstance(ir, bytes):  # read in place: immutable bytes only
+        raise TypeError(f"an op list is bytes, not {type(ir).__name__}")
     _check(h, load().px_submit_ops(h, ir, len(ir)))
 
 
