@@ -10,6 +10,7 @@
 #include <atomic>
 #include <condition_variable>
 #include <functional>
+#include <exception>
 #include <limits>
 #include <mutex>
 #include <thread>
@@ -1327,7 +1328,8 @@ class HostPool {
   }
   int size() const { return (int)workers_.size() + 1; }
   // run f(k) for k in [0, n) on the pool and the calling thread; returns once every f(k)
-  // has, without waiting for workers that woke too late to take one
+  // has, without waiting for workers that woke too late to take one.  What an f(k) threw (a
+  // failed allocation) is thrown here then, the first one caught
   void run(int n, const std::function<void(int)>& f) {
     if (n <= 1 || workers_.empty()) {
       for (int k = 0; k < n; k++) f(k);
@@ -1353,6 +1355,13 @@ class HostPool {
         done_cv_.wait(g, [&] { return done_.load(std::memory_order_acquire) == (uint32_t)n; });
         break;
       }
+    }
+    if (failed_.load(std::memory_order_relaxed)) {  // (ordered by done_)
+      std::exception_ptr e;
+      std::lock_guard<std::mutex> g(mu_);
+      std::swap(e, error_);
+      failed_.store(false, std::memory_order_relaxed);
+      std::rethrow_exception(e);
     }
   }
 
@@ -1381,7 +1390,13 @@ class HostPool {
         continue;  // the next job began meanwhile
       }
       if (!ticket_.compare_exchange_weak(t, t + 1, std::memory_order_acq_rel)) continue;
-      (*f)((int)k);
+      try {
+        (*f)((int)k);
+      } catch (...) {
+        std::lock_guard<std::mutex> g(mu_);
+        if (!error_) error_ = std::current_exception();
+        failed_.store(true, std::memory_order_relaxed);
+      }
       if (done_.fetch_add(1, std::memory_order_acq_rel) + 1 == n) {
         std::lock_guard<std::mutex> g(mu_);
         done_cv_.notify_one();
@@ -1413,6 +1428,8 @@ class HostPool {
   Job job_[2];
   std::atomic<uint64_t> ticket_{0};  // generation << 32 | next index
   std::atomic<uint32_t> done_{0};    // indices of the current job that have returned
+  std::atomic<bool> failed_{false};
+  std::exception_ptr error_;         // under mu_: what the first of them to fail threw
 };
 
 // The cull kernels' table from the op boxes in h_boxes[0 .. n_ops): after them the union box of
@@ -1505,6 +1522,28 @@ void cull_tables(px_world* w, int n_ops) {
   std::memcpy(groups, w->h_groups.data(), sizeof(uint2) * n_groups);
   for (int k = 0; k < n_ops; k += 2) w->h_boxes[w->cull.n++] = make_uint2(ord[k], k + 1 < n_ops ? ord[k + 1] : 0u);
 }
+
+// Puts a world's queue back as it was found unless what was queued is kept: a failed host
+// allocation half way leaves arrays of different lengths.
+struct QueueUndo {
+  px_world* w;
+  size_t ops, code, p32, bases, params, painted64, painted32;
+  uint64_t pairs, tile_pairs;
+  bool keep = false;
+  explicit QueueUndo(px_world* w_)
+      : w(w_), ops(w->ops.size()), code(w->code.size()), p32(w->p32.size()), bases(w->bases.size()), params(w->params.size()),
+        painted64(w->q.painted64.size()), painted32(w->q.painted32.size()), pairs(w->q.pairs), tile_pairs(w->q.tile_pairs) {}
+  ~QueueUndo() {
+    if (keep) return;
+    w->ops.resize(ops); w->lite.resize(ops); w->boxes.resize(ops);
+    w->code.resize(code); w->code32.resize(code);
+    w->p32.resize(p32); w->bases.resize(bases); w->params.resize(params);
+    w->q.painted64.resize(painted64); w->q.painted32.resize(painted32);
+    w->q.pairs = pairs;
+    w->q.tile_pairs = tile_pairs;
+    w->cull_ready = false;
+  }
+};
 
 // Sizes of the buffers a resident op list lives in: one that was reallocated (ensure; always to
 // another size) has lost the list.
@@ -1735,6 +1774,7 @@ static int submit_ops_impl(px_world* w, const void* ir, size_t bytes) {
     uint64_t pairs;
   };
   std::vector<Place> at(n_chunks);
+  QueueUndo undo(w);
   Place end = {w->code.size(), w->p32.size(), w->bases.size(), w->ops.size(), param_base + n_params, w->q.pairs};
   for (int k = 0; k < n_chunks; k++) {
     const SubmitChunk& c = chunks[k];
@@ -1806,6 +1846,7 @@ static int submit_ops_impl(px_world* w, const void* ir, size_t bytes) {
     for (int k = 0; k < 3; k++) merge(k);
   }
   w->cull_ready = first_list;
+  undo.keep = true;
   return PX_OK;
 }
 
@@ -2340,6 +2381,7 @@ static int world_reset_impl(px_world* w, int requeue_last_ops, void* stream) {
   w->free_valid = false;
   if (requeue_last_ops) {
     if (!w->ops.empty()) return fail(w, PX_E_INVALID_ARG, "ops are already queued");
+    QueueUndo undo(w);
     w->ops = w->last_ops;
     w->boxes = w->last_boxes;
     w->lite = w->last_lite;
@@ -2350,6 +2392,7 @@ static int world_reset_impl(px_world* w, int requeue_last_ops, void* stream) {
     w->p32 = w->last_p32;
     w->bases = w->last_bases;
     w->q = w->last_q;
+    undo.keep = true;
     w->ops_resident = w->last_resident;  // the device tables of the last build, unless they were reallocated
   }
   return PX_OK;
