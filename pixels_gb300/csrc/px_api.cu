@@ -88,7 +88,16 @@ struct SubmitChunk {
     rc = PX_OK;
     err.clear();
   }
+  size_t bytes() const {  // the room its arrays hold
+    return ops.capacity() * sizeof(OpDev) + lite.capacity() * sizeof(OpLite) + (boxes.capacity() + code.capacity()) * sizeof(uint2) +
+           xparams.capacity() * sizeof(double) + (bases.capacity() + p32.capacity()) * sizeof(float2) +
+           (code32.capacity() + xfix.capacity() + painted64.capacity() + painted32.capacity()) * sizeof(uint32_t);
+  }
 };
+// The most conversion workspace a world keeps from one list to the next, about a second copy of its
+// op tables (4,096 primitives: 4 MB); a longer list's is given back (the conversion takes
+// longer than its page faults), as is a batched world's, which queues nothing.
+constexpr size_t KEEP_CHUNK_BYTES = 16u << 20;
 
 // How a cull table is laid out (launch_cull): the form, its (op, tile) pairs (CULL_FEW) and
 // its entries.
@@ -1847,6 +1856,9 @@ static int submit_ops_impl(px_world* w, const void* ir, size_t bytes) {
   }
   w->cull_ready = first_list;
   undo.keep = true;
+  size_t held = 0;
+  for (const SubmitChunk& c : chunks) held += c.bytes();
+  if (held > KEEP_CHUNK_BYTES) std::vector<SubmitChunk>().swap(chunks);
   return PX_OK;
 }
 
@@ -2682,6 +2694,7 @@ static int batch_create_impl(px_world* const* worlds, size_t n, int mode, uint32
     w->ops.clear(); w->lite.clear(); w->boxes.clear(); w->code.clear(); w->params.clear();
     w->code32.clear(); w->p32.clear(); w->bases.clear();
     w->q.clear();
+    std::vector<SubmitChunk>().swap(w->chunks);
   }
   if (rc == PX_OK && ce != cudaSuccess) rc = batch_fail(b, PX_E_CUDA, "capture: %s", cudaGetErrorString(ce));
   if (rc == PX_OK && cudaGraphInstantiate(&b->exec, b->graph, 0) != cudaSuccess)
