@@ -767,23 +767,30 @@ __global__ void __launch_bounds__(256, MINB) classify_kernel(FoldArgs a) {
     const unsigned long long p = (unsigned long long)chunk * 32 + lane;
     const bool valid = p < P;
     uint32_t o = ce.y & 0x7fffffffu;
-    if (!(ce.y >> 31)) {  // the chunk spans several ops (at most 32 start in it; warp-uniform)
-      // lane j holds the first pair of op o + 1 + j; a lane's op is o plus the number of
-      // those at or below its pair (sorted: a binary search over the lanes, by shuffles)
-      const unsigned long long pb =
-          o + 1 + (uint32_t)lane < a.n_ops ? __ldg(&a.ops[o + 1 + lane].pair_base) : ~0ull;
-      // (33 possible counts: six halvings; every lane shuffles each time, from lane <= 31)
-      uint32_t lo = 0, hi = 32;
+    if (!(ce.y >> 31)) {  // the chunk spans several ops (warp-uniform)
+      // lane j holds the first pair of op base + 1 + j; a lane's op is base plus the number of
+      // those at or below its pair (sorted: a binary search over the lanes, by shuffles), or
+      // among the next 32: a chunk has pairs of 32 ops at most, but ops without any may lie between
+      bool open = true;
+#pragma unroll 1
+      for (uint32_t base = o;; base += 32) {
+        const unsigned long long pb =
+            base + 1 + (uint32_t)lane < a.n_ops ? __ldg(&a.ops[base + 1 + lane].pair_base) : ~0ull;
+        // (33 possible counts: six halvings; every lane shuffles each time, from lane <= 31)
+        uint32_t lo = 0, hi = 32;
 #pragma unroll
-      for (int k = 0; k < 6; k++) {
-        const uint32_t mid = min((lo + hi) >> 1, 31u);
-        const unsigned long long v = __shfl_sync(FULLMASK, pb, (int)mid);
-        if (lo < hi) {
-          if (v <= p) lo = mid + 1;
-          else hi = mid;
+        for (int k = 0; k < 6; k++) {
+          const uint32_t mid = min((lo + hi) >> 1, 31u);
+          const unsigned long long v = __shfl_sync(FULLMASK, pb, (int)mid);
+          if (lo < hi) {
+            if (v <= p) lo = mid + 1;
+            else hi = mid;
+          }
         }
+        if (open) o = base + lo;
+        open = open && valid && lo == 32;
+        if (!__any_sync(FULLMASK, open)) break;
       }
-      o += lo;
     }
     const OpDev* O = a.ops + o;
     int bx = 0, by = 0, bz = 0, cls = PC_SKIP;
