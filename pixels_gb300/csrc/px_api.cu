@@ -1627,8 +1627,23 @@ int reserve_build_scratch(px_world* w, uint64_t P, uint32_t max_ops) {
   int rc = grow_pool(w, (uint64_t)w->pool_used + stage_cap, w->pool_used, nullptr);
   if (rc) return rc;
   if ((rc = ensure_pair_scratch(w, P, P, 0, touched_bound, E_max, stage_cap))) return rc;
-  if ((rc = ensure(w, w->holes_a, 4 * E_max + 4))) return rc;
-  return ensure(w, w->holes_b, 4 * E_max + 4);
+  // the free lists: the current one holds the world's holes, which move with it
+  DevBuf& now = w->holes_in_a ? w->holes_a : w->holes_b;
+  DevBuf& next = w->holes_in_a ? w->holes_b : w->holes_a;
+  if (now.bytes < 4 * E_max + 4 && !now.borrowed && w->n_holes) {
+    DevBuf grown;
+    if ((rc = ensure(w, grown, 4 * E_max + 4))) return rc;
+    if (cudaMemcpyAsync(grown.p, now.p, 4 * (size_t)w->n_holes, cudaMemcpyDeviceToDevice, nullptr) != cudaSuccess ||
+        cudaStreamSynchronize(nullptr) != cudaSuccess) {
+      cudaGetLastError();
+      release(grown);
+      return fail(w, PX_E_CUDA, "the free list could not be copied");
+    }
+    release(now);
+    now = grown;
+  }
+  if ((rc = ensure(w, now, 4 * E_max + 4))) return rc;
+  return ensure(w, next, 4 * E_max + 4);
 }
 uint64_t build_stage_slots(const px_world* w, uint64_t P) { return stage_slots(w, P); }
 
