@@ -209,8 +209,10 @@ typedef struct px_edit_result {
    (shapes.ts:423-426).  Before the first edit the pool is reserved to
    min(pool_budget_bricks, max(used + 98304, 2 used)) bricks (GpuWorld.ts:57).
    applied_order (n entries, may be NULL) receives the edit indices in the
-   order applied.  Blocks until every edit is applied or rejected; a step that
-   fails (PX_E_QUEUE_OVERFLOW) ends the run with the world as it was before it. */
+   order applied.  Blocks until every edit is applied or rejected.  A step whose
+   work lists run out of room is built again alone with larger ones (the steps
+   queued behind it wait again); a step that still fails ends the run with the
+   world as it was before it and no ops queued. */
 int px_serve_run(px_world* w, const px_edit* edits, const double* arrival_s, size_t n, uint32_t max_batch,
                  uint64_t pool_budget_bricks, int mode, void* stream, px_edit_result* results,
                  uint64_t* applied_order, size_t* n_applied);

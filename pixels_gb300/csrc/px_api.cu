@@ -1651,6 +1651,23 @@ uint64_t build_stage_slots(const px_world* w, uint64_t P) { return stage_slots(w
 #define PIPELINE_PAIRS_PER_BLOCK 64
 #endif
 
+static void borrow(DevBuf& dst, const DevBuf& src) {
+  dst = src;
+  dst.borrowed = true;
+}
+// What a build of the world may have replaced or moved on: its pool, free lists, allocator state
+// and the sizes that failed builds asked for.
+static void twin_share(px_world* t, const px_world* w) {
+  t->d_pool32 = w->d_pool32; t->d_pcount = w->d_pcount;
+  t->pool_cap = w->pool_cap;
+  t->pool_used = w->pool_used; t->n_holes = w->n_holes; t->holes_in_a = w->holes_in_a;
+  t->pcount_valid = w->pcount_valid;
+  t->rescue_cap = w->rescue_cap;
+  t->stage_hint = w->stage_hint;
+  borrow(t->holes_a, w->holes_a);
+  borrow(t->holes_b, w->holes_b);
+}
+
 px_world* twin_create(px_world* w, uint64_t P, uint32_t max_ops, int* rc) {
   *rc = PX_OK;
   px_world* t = new px_world();
@@ -1662,18 +1679,11 @@ px_world* twin_create(px_world* w, uint64_t P, uint32_t max_ops, int* rc) {
   t->vq_nonempty = w->vq_nonempty;
   t->host_reads = w->host_reads;
   t->validate = w->validate;
-  t->rescue_cap = w->rescue_cap;
-  t->stage_hint = w->stage_hint;
   t->pairs_per_block = PIPELINE_PAIRS_PER_BLOCK;
   // the shared world: grid, pool, opaque counts, device state, free lists, material tables
   t->shares_state = true;
-  t->d_grid = w->d_grid; t->d_pool32 = w->d_pool32; t->d_pcount = w->d_pcount; t->d_state = w->d_state;
-  t->pool_cap = w->pool_cap;
-  t->pool_used = w->pool_used; t->n_holes = w->n_holes; t->holes_in_a = w->holes_in_a;
-  t->pcount_valid = w->pcount_valid;
-  auto borrow = [](DevBuf& dst, const DevBuf& src) { dst = src; dst.borrowed = true; };
-  borrow(t->holes_a, w->holes_a);
-  borrow(t->holes_b, w->holes_b);
+  t->d_grid = w->d_grid; t->d_state = w->d_state;
+  twin_share(t, w);
   borrow(t->opaque, w->opaque);
   borrow(t->axis32, w->axis32);
   borrow(t->udens, w->udens);
@@ -1731,6 +1741,28 @@ void pipeline_end(px_world* w, const PipelineState& st, uint64_t ops, cudaStream
   w->free_valid = false;
   cudaMemsetAsync(&w->d_state->poisoned, 0, 4, s);  // a failed build left the world as it was
   cudaStreamSynchronize(s);
+}
+
+static void drop_queue(px_world* w) {
+  w->ops.clear(); w->lite.clear(); w->boxes.clear(); w->code.clear(); w->params.clear();
+  w->code32.clear(); w->p32.clear(); w->bases.clear();
+  w->q.clear();
+  w->cull_ready = false;
+}
+
+int pipeline_clear(px_world* w, px_world* twin, cudaStream_t s) {
+  drop_queue(w);
+  drop_queue(twin);
+  CU(cudaMemsetAsync(&w->d_state->poisoned, 0, 4, s));
+  CU(cudaStreamSynchronize(s));
+  return PX_OK;
+}
+
+int pipeline_resume(px_world* w, px_world* twin, uint64_t P, uint32_t max_ops) {
+  int rc = reserve_build_scratch(w, P, max_ops);
+  if (rc) return rc;
+  twin_share(twin, w);
+  return reserve_build_scratch(twin, P, max_ops);
 }
 
 bool build_done(px_world* w) { return !w->in_flight || cudaEventQuery(w->ev_done) == cudaSuccess; }
@@ -2706,9 +2738,7 @@ static int batch_create_impl(px_world* const* worlds, size_t n, int mode, uint32
     w->derived_valid = saved[i].derived_valid;
     w->free_valid = saved[i].free_valid;
     w->pairs_per_block = saved[i].ppb;
-    w->ops.clear(); w->lite.clear(); w->boxes.clear(); w->code.clear(); w->params.clear();
-    w->code32.clear(); w->p32.clear(); w->bases.clear();
-    w->q.clear();
+    drop_queue(w);
     std::vector<SubmitChunk>().swap(w->chunks);
   }
   if (rc == PX_OK && ce != cudaSuccess) rc = batch_fail(b, PX_E_CUDA, "capture: %s", cudaGetErrorString(ce));

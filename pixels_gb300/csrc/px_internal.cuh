@@ -454,8 +454,8 @@ uint64_t build_stage_slots(const px_world* w, uint64_t P);
 // order their apply passes are queued on the apply stream.
 px_world* twin_create(px_world* w, uint64_t P, uint32_t max_ops, int* rc);
 void twin_destroy(px_world* t);
-// Queue settings of a pipelined world: the apply pass on `apply` (NULL: the
-// build's stream), no retries, and the host's view of the shared allocator
+// Queue settings of a pipelined world: the apply pass on `apply` and no retries (NULL: the
+// build's stream, retries as in any build), and the host's view of the shared allocator
 // state before the build (holes parity, bounds of poolUsed and the hole count).
 void pipeline_set(px_world* w, cudaStream_t apply, bool holes_in_a, uint32_t pool_used_bound, uint32_t n_holes_bound);
 // The committed allocator state a pipeline starts from (and ends with).
@@ -470,6 +470,12 @@ PipelineState pipeline_begin(px_world* w);
 // counts `ops` more ops applied, clears a poisoned device state and restores
 // derive on build.
 void pipeline_end(px_world* w, const PipelineState& st, uint64_t ops, cudaStream_t s);
+// After a pipelined step failed and no build is in flight: the device state takes builds again, and
+// neither world has ops queued.
+int pipeline_clear(px_world* w, px_world* twin, cudaStream_t s);
+// After a build of `w` alone between pipelined ones: its grown pool, free lists and hints are the
+// twin's too, and both have the scratch of their largest step.
+int pipeline_resume(px_world* w, px_world* twin, uint64_t P, uint32_t max_ops);
 // The build's result block is on the host (px_build_finish would not wait).
 bool build_done(px_world* w);
 // Device times (ms since `base`) of the last finished build's first and last kernels.

@@ -189,6 +189,7 @@ static int serve_run_impl(px_world* w, const px_edit* edits, const double* arriv
     double start;
     uint32_t id;
     size_t n_ops;
+    size_t begin;         // the place of its first edit in arrival order
   };
   std::vector<Step> flight;  // at most two steps in flight, oldest first
   size_t next = 0, applied = 0;
@@ -201,32 +202,75 @@ static int serve_run_impl(px_world* w, const px_edit* edits, const double* arriv
   std::vector<double> params;
   std::vector<unsigned char> ir;
 
+  // the op list of some edits, in order, in `ir`
+  auto encode = [&](const std::vector<size_t>& which) {
+    ops.clear();
+    code.clear();
+    params.clear();
+    for (size_t i : which) encode_carve(edits[i], vs, ops, code, params);
+    ir.assign(32 + ops.size() * sizeof(IrOp) + code.size() * 4 + params.size() * 8, 0);
+    uint32_t hdr[8] = {0x52495850u, 1u, (uint32_t)ops.size(), (uint32_t)(code.size() / 2), (uint32_t)params.size(), 0, 0, 0};
+    std::memcpy(ir.data(), hdr, 32);
+    std::memcpy(ir.data() + 32, ops.data(), ops.size() * sizeof(IrOp));
+    std::memcpy(ir.data() + 32 + ops.size() * sizeof(IrOp), code.data(), code.size() * 4);
+    std::memcpy(ir.data() + 32 + ops.size() * sizeof(IrOp) + code.size() * 4, params.data(), params.size() * 8);
+  };
+
+  // A step that failed: its buffers (staging slots, rescue list) were too small, which a
+  // pipelined build cannot mend as later ones are queued behind it.  Those commit nothing; their
+  // edits wait again, and the step is built alone, with the retries of any build.
+  auto build_alone = [&](const Step& stp) {
+    while (!flight.empty()) {
+      px_build_finish(W[flight.back().world]);
+      next = flight.back().begin;
+      flight.pop_back();
+    }
+    int arc = pipeline_clear(w, twin, s_eval);
+    if (arc != PX_OK) return arc;
+    encode(stp.edits);
+    pipeline_set(w, nullptr, committed.holes_in_a, committed.pool_used, committed.n_holes);
+    arc = px_submit_ops(w, ir.data(), ir.size());
+    if (arc == PX_OK) arc = px_build(w, mode, s_eval);
+    parity = committed.holes_in_a != (arc == PX_OK);  // the other holes buffer, if this step wrote it
+    return arc;
+  };
+
   auto finish_oldest = [&]() {
     Step stp = std::move(flight.front());
     flight.erase(flight.begin());
     px_world* x = W[stp.world];
-    const int brc = px_build_finish(x);
+    int brc = px_build_finish(x), after = PX_OK;
+    if (brc == PX_E_QUEUE_OVERFLOW && rc == PX_OK) {
+      x = w;
+      brc = build_alone(stp);
+      if (brc == PX_OK) {  // the step is committed, whether or not the next ones can be queued
+        after = pipeline_resume(w, twin, pair_budget, max_batch);
+        px_stats ws;
+        px_get_stats(w, &ws);
+        pool_cap = ws.pool_capacity;
+      }
+    }
     const double done = secs(t0, clock_t_::now());
     double d0 = -1, d1 = -1;
     build_times(x, base, &d0, &d1);
-    if (brc == PX_OK && rc == PX_OK) {
+    const bool ok = brc == PX_OK;  // committed, also where a later step could not be queued
+    if (ok) {
       px_stats xs;
       px_get_stats(x, &xs);
       committed.pool_used = xs.pool_used;
       committed.n_holes = xs.n_holes;
       committed.holes_in_a = !committed.holes_in_a;  // the step wrote the other holes buffer
       ops_done += stp.n_ops;
-    } else if (rc == PX_OK) {
-      rc = brc;  // later queued steps commit nothing (the device state is poisoned)
     }
+    if (rc == PX_OK) rc = ok ? after : brc;  // (steps queued behind a failed one commit nothing)
     for (size_t i : stp.edits) {
       results[i].start_s = stp.start;
       results[i].done_s = done;
       results[i].dev_start_ms = d0;
       results[i].dev_end_ms = d1;
       results[i].batch = stp.id;
-      results[i].status = (uint32_t)(rc == PX_OK ? PX_OK : PX_E_QUEUE_OVERFLOW);
-      if (rc == PX_OK) {
+      results[i].status = (uint32_t)(ok ? PX_OK : PX_E_QUEUE_OVERFLOW);
+      if (ok) {
         if (applied_order) applied_order[applied] = i;
         applied++;
       }
@@ -259,12 +303,14 @@ static int serve_run_impl(px_world* w, const px_edit* edits, const double* arriv
     const uint64_t live = (uint64_t)committed.pool_used - committed.n_holes;
     const uint64_t used_bound = (uint64_t)committed.pool_used + in_flight;
     std::vector<size_t> batch;
-    ops.clear();
-    code.clear();
-    params.clear();
     uint64_t bound = 0;
+    size_t begin = next;
     while (next < avail && batch.size() < max_batch) {
       const size_t i = order[next];
+      if (results[i].status != PX_OK) {  // rejected before the step behind it had to wait again
+        next++;
+        continue;
+      }
       const uint64_t b = brick_bound(edits[i], vs, dims[0], dims[1], dims[2]);
       const bool fits = live + in_flight + bound + b <= pool_budget_bricks &&
                         used_bound + build_stage_slots(w, bound + b) <= pool_cap && bound + b <= pair_budget;
@@ -278,8 +324,8 @@ static int serve_run_impl(px_world* w, const px_edit* edits, const double* arriv
         break;  // wait for the next step (or for the step in flight to commit)
       }
       bound += b;
+      if (batch.empty()) begin = next;
       batch.push_back(i);
-      encode_carve(edits[i], vs, ops, code, params);
       next++;
     }
     if (batch.empty()) {
@@ -287,12 +333,7 @@ static int serve_run_impl(px_world* w, const px_edit* edits, const double* arriv
       continue;
     }
     const double start = secs(t0, clock_t_::now());
-    ir.assign(32 + ops.size() * sizeof(IrOp) + code.size() * 4 + params.size() * 8, 0);
-    uint32_t hdr[8] = {0x52495850u, 1u, (uint32_t)ops.size(), (uint32_t)(code.size() / 2), (uint32_t)params.size(), 0, 0, 0};
-    std::memcpy(ir.data(), hdr, 32);
-    std::memcpy(ir.data() + 32, ops.data(), ops.size() * sizeof(IrOp));
-    std::memcpy(ir.data() + 32 + ops.size() * sizeof(IrOp), code.data(), code.size() * 4);
-    std::memcpy(ir.data() + 32 + ops.size() * sizeof(IrOp) + code.size() * 4, params.data(), params.size() * 8);
+    encode(batch);
     const int wi = (int)(batch_id & 1u);
     px_world* x = W[wi];
     pipeline_set(x, s_apply, parity, (uint32_t)std::min<uint64_t>(used_bound, pool_cap),
@@ -308,12 +349,13 @@ static int serve_run_impl(px_world* w, const px_edit* edits, const double* arriv
       continue;
     }
     parity = !parity;
-    flight.push_back(Step{std::move(batch), bound, wi, start, batch_id, ops.size()});
+    flight.push_back(Step{std::move(batch), bound, wi, start, batch_id, ops.size(), begin});
     batch_id++;
   }
   stop.store(true);
   producer.join();
   cudaStreamSynchronize(s_apply);
+  if (rc != PX_OK) pipeline_clear(w, twin, s_eval);  // (a failed step's ops are not the next build's)
   pipeline_end(w, committed, ops_done, s_eval);
   twin_destroy(twin);
   cudaStreamDestroy(s_apply);
