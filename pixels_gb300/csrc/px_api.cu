@@ -1716,7 +1716,7 @@ void pipeline_set(px_world* w, cudaStream_t apply, bool holes_in_a, uint32_t poo
 }
 
 PipelineState pipeline_begin(px_world* w) {
-  PipelineState st{w->pool_used, w->n_holes, w->holes_in_a, w->derive_max, w->pairs_per_block};
+  PipelineState st{w->pool_used, w->n_holes, w->holes_in_a, w->derive_max, w->pairs_per_block, w->ops_applied};
   w->derive_max = 0;
   // two builds share the GPU: persistent grids sized to each build's pairs
   // (a few edits need a few blocks, not the whole GPU)
@@ -1733,7 +1733,7 @@ void pipeline_end(px_world* w, const PipelineState& st, uint64_t ops, cudaStream
   w->holes_in_a = st.holes_in_a;
   w->derive_max = st.derive_max;
   w->pairs_per_block = st.pairs_per_block;
-  w->ops_applied += ops;
+  w->ops_applied = st.ops_applied + ops;
   w->stats.ops_applied = w->ops_applied;
   w->stats.pool_used = st.pool_used;
   w->stats.n_holes = st.n_holes;

@@ -464,6 +464,7 @@ struct PipelineState {
   bool holes_in_a;
   uint32_t derive_max;  // the world's derive-on-build setting, off while pipelined
   uint32_t pairs_per_block;  // the world's persistent-grid sizing, restored after the pipeline
+  uint64_t ops_applied;      // before the pipeline (the builds on the world itself count their own)
 };
 PipelineState pipeline_begin(px_world* w);
 // After the last pipelined build: the world takes over the committed state,
