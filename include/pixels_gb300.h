@@ -191,7 +191,7 @@ typedef struct px_edit {
 } px_edit;
 typedef struct px_edit_result {
   uint64_t id;         /* index into the edits array */
-  uint32_t status;     /* PX_OK, or PX_E_OOM when the edit cannot fit the pool budget */
+  uint32_t status;     /* PX_OK: applied; PX_E_OOM: cannot fit the pool budget; else why the run ended before it */
   uint32_t batch;      /* build step that applied it */
   double arrival_s, start_s, done_s;  /* seconds since the run started */
   double dev_start_ms, dev_end_ms;    /* its build step's first and last kernel on the device,

@@ -355,7 +355,11 @@ static int serve_run_impl(px_world* w, const px_edit* edits, const double* arriv
   stop.store(true);
   producer.join();
   cudaStreamSynchronize(s_apply);
-  if (rc != PX_OK) pipeline_clear(w, twin, s_eval);  // (a failed step's ops are not the next build's)
+  if (rc != PX_OK) {
+    pipeline_clear(w, twin, s_eval);  // (a failed step's ops are not the next build's)
+    for (; next < n; next++)  // edits that no step took
+      if (results[order[next]].status == PX_OK) results[order[next]].status = (uint32_t)rc;
+  }
   pipeline_end(w, committed, ops_done, s_eval);
   twin_destroy(twin);
   cudaStreamDestroy(s_apply);

@@ -46,3 +46,28 @@ def test_ops_applied_counts_each_edit_once(built_lib, n, max_batch):
     w.build()
     assert w.stats()["ops_applied"] == total + 1
     w.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("max_batch", [4, 100])
+def test_a_run_that_fails_reports_every_edit(built_lib, max_batch):
+    """A mode that no build takes: the first step cannot be queued.  No edit is reported as
+    applied, and none is left queued for the world's next build."""
+    w = world()
+    before, used = w.grid.copy(), w.poolUsed
+    n = 20
+    es = (_lib.Edit * n)()
+    for e, (shape, a, b, r) in zip(es, edits(n)):
+        e.shape, e.r = shape, r
+        e.a[:], e.b[:] = a, b
+    res, order, applied = (_lib.EditResult * n)(), (ctypes.c_uint64 * n)(), ctypes.c_size_t()
+    rc = _lib.load().px_serve_run(w._h, es, (ctypes.c_double * n)(), n, max_batch, 1 << 40, 7, None, res, order,
+                                  ctypes.byref(applied))
+    assert rc == 1 and applied.value == 0  # PX_E_INVALID_ARG
+    assert all(r.status != 0 for r in res)
+    w.build()
+    np.testing.assert_array_equal(w.grid, before)
+    assert w.poolUsed == used
+    serving.serve(w, edits(n), np.zeros(n), max_batch=max_batch)  # and the world serves
+    assert w.stats()["ops_applied"] == 2 + n
+    w.close()
