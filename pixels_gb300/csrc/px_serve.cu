@@ -169,7 +169,8 @@ static int serve_run_impl(px_world* w, const px_edit* edits, const double* arriv
   std::atomic<size_t> released{0};
   std::atomic<bool> stop{false};
   const auto t0 = clock_t_::now();
-  std::thread producer([&] {
+  std::thread producer;
+  auto release = [&] {
     for (size_t k = 0; k < n; k++) {
       const double t = arrival_s[order[k]];
       std::this_thread::sleep_until(t0 + std::chrono::duration_cast<clock_t_::duration>(std::chrono::duration<double>(t)));
@@ -180,7 +181,7 @@ static int serve_run_impl(px_world* w, const px_edit* edits, const double* arriv
       }
       cv.notify_one();
     }
-  });
+  };
 
   struct Step {
     std::vector<size_t> edits;
@@ -242,8 +243,12 @@ static int serve_run_impl(px_world* w, const px_edit* edits, const double* arriv
     int brc = px_build_finish(x), after = PX_OK;
     if (brc == PX_E_QUEUE_OVERFLOW && rc == PX_OK) {
       x = w;
-      brc = build_alone(stp);
-      if (brc == PX_OK) {  // the step is committed, whether or not the next ones can be queued
+      try {
+        brc = build_alone(stp);
+      } catch (const std::bad_alloc&) {
+        brc = PX_E_OOM;
+      }
+      if (brc == PX_OK && next < n) {  // the step is committed, whether or not the next ones can be queued
         after = pipeline_resume(w, twin, pair_budget, max_batch);
         px_stats ws;
         px_get_stats(w, &ws);
@@ -277,83 +282,99 @@ static int serve_run_impl(px_world* w, const px_edit* edits, const double* arriv
     }
   };
 
-  while ((next < n && rc == PX_OK) || !flight.empty()) {
-    if (flight.size() == 2 || rc != PX_OK) {  // both world objects busy (or draining after a failure)
-      finish_oldest();
-      continue;
-    }
-    if (flight.empty() && released.load() <= next && next < n) {  // idle: sleep until a request arrives
-      std::unique_lock<std::mutex> g(mu);
-      cv.wait(g, [&] { return released.load() > next; });
-    }
-    const size_t avail = released.load();
-    if (next >= n) {
-      finish_oldest();
-      continue;
-    }
-    if (avail <= next) {  // nothing new: the step in flight finishes unless a request arrives first
-      if (build_done(W[flight.front().world])) finish_oldest();
-      else std::this_thread::yield();
-      continue;
-    }
-    // admit in arrival order while the free pool holds the worst case of this
-    // step and of the step still in flight
-    uint64_t in_flight = 0;
-    for (const Step& f : flight) in_flight += f.bound;
-    const uint64_t live = (uint64_t)committed.pool_used - committed.n_holes;
-    const uint64_t used_bound = (uint64_t)committed.pool_used + in_flight;
-    std::vector<size_t> batch;
-    uint64_t bound = 0;
-    size_t begin = next;
-    while (next < avail && batch.size() < max_batch) {
-      const size_t i = order[next];
-      if (results[i].status != PX_OK) {  // rejected before the step behind it had to wait again
-        next++;
+  // A host allocation that fails (or a producer that cannot be started) ends the run like a step that
+  // cannot be queued: the steps in flight finish, the edits of the one being formed were not applied.
+  size_t forming = n;  // the place of its first edit (n: none is)
+  try {
+    flight.reserve(2);
+    producer = std::thread(release);
+    while ((next < n && rc == PX_OK) || !flight.empty()) {
+      forming = n;
+      if (flight.size() == 2 || rc != PX_OK) {  // both world objects busy (or draining after a failure)
+        finish_oldest();
         continue;
       }
-      const uint64_t b = brick_bound(edits[i], vs, dims[0], dims[1], dims[2]);
-      const bool fits = live + in_flight + bound + b <= pool_budget_bricks &&
-                        used_bound + build_stage_slots(w, bound + b) <= pool_cap && bound + b <= pair_budget;
-      if (!fits) {
-        if (batch.empty() && flight.empty()) {  // cannot fit even alone on an idle world: reject
-          results[i].status = PX_E_OOM;
-          results[i].done_s = secs(t0, clock_t_::now());
+      if (flight.empty() && released.load() <= next && next < n) {  // idle: sleep until a request arrives
+        std::unique_lock<std::mutex> g(mu);
+        cv.wait(g, [&] { return released.load() > next; });
+      }
+      const size_t avail = released.load();
+      if (next >= n) {
+        finish_oldest();
+        continue;
+      }
+      if (avail <= next) {  // nothing new: the step in flight finishes unless a request arrives first
+        if (build_done(W[flight.front().world])) finish_oldest();
+        else std::this_thread::yield();
+        continue;
+      }
+      // admit in arrival order while the free pool holds the worst case of this
+      // step and of the step still in flight
+      uint64_t in_flight = 0;
+      for (const Step& f : flight) in_flight += f.bound;
+      const uint64_t live = (uint64_t)committed.pool_used - committed.n_holes;
+      const uint64_t used_bound = (uint64_t)committed.pool_used + in_flight;
+      std::vector<size_t> batch;
+      uint64_t bound = 0;
+      size_t begin = forming = next;
+      while (next < avail && batch.size() < max_batch) {
+        const size_t i = order[next];
+        if (results[i].status != PX_OK) {  // rejected before the step behind it had to wait again
           next++;
           continue;
         }
-        break;  // wait for the next step (or for the step in flight to commit)
+        const uint64_t b = brick_bound(edits[i], vs, dims[0], dims[1], dims[2]);
+        const bool fits = live + in_flight + bound + b <= pool_budget_bricks &&
+                          used_bound + build_stage_slots(w, bound + b) <= pool_cap && bound + b <= pair_budget;
+        if (!fits) {
+          if (batch.empty() && flight.empty()) {  // cannot fit even alone on an idle world: reject
+            results[i].status = PX_E_OOM;
+            results[i].done_s = secs(t0, clock_t_::now());
+            next++;
+            continue;
+          }
+          break;  // wait for the next step (or for the step in flight to commit)
+        }
+        bound += b;
+        if (batch.empty()) begin = next;
+        batch.push_back(i);
+        next++;
       }
-      bound += b;
-      if (batch.empty()) begin = next;
-      batch.push_back(i);
-      next++;
-    }
-    if (batch.empty()) {
-      if (!flight.empty()) finish_oldest();
-      continue;
-    }
-    const double start = secs(t0, clock_t_::now());
-    encode(batch);
-    const int wi = (int)(batch_id & 1u);
-    px_world* x = W[wi];
-    pipeline_set(x, s_apply, parity, (uint32_t)std::min<uint64_t>(used_bound, pool_cap),
-                 (uint32_t)std::min<uint64_t>((uint64_t)committed.n_holes + in_flight, pool_cap));
-    int erc = px_submit_ops(x, ir.data(), ir.size());
-    if (erc == PX_OK) erc = px_build_enqueue(x, mode, s_eval);
-    if (erc != PX_OK) {
-      rc = erc;
-      for (size_t i : batch) {
-        results[i].status = (uint32_t)erc;
-        results[i].done_s = secs(t0, clock_t_::now());
+      if (batch.empty()) {
+        if (!flight.empty()) finish_oldest();
+        continue;
       }
-      continue;
+      const double start = secs(t0, clock_t_::now());
+      encode(batch);
+      const int wi = (int)(batch_id & 1u);
+      px_world* x = W[wi];
+      pipeline_set(x, s_apply, parity, (uint32_t)std::min<uint64_t>(used_bound, pool_cap),
+                   (uint32_t)std::min<uint64_t>((uint64_t)committed.n_holes + in_flight, pool_cap));
+      int erc = px_submit_ops(x, ir.data(), ir.size());
+      if (erc == PX_OK) erc = px_build_enqueue(x, mode, s_eval);
+      if (erc != PX_OK) {
+        rc = erc;
+        for (size_t i : batch) {
+          results[i].status = (uint32_t)erc;
+          results[i].done_s = secs(t0, clock_t_::now());
+        }
+        continue;
+      }
+      parity = !parity;
+      flight.push_back(Step{std::move(batch), bound, wi, start, batch_id, ops.size(), begin});
+      batch_id++;
+      forming = n;
     }
-    parity = !parity;
-    flight.push_back(Step{std::move(batch), bound, wi, start, batch_id, ops.size(), begin});
-    batch_id++;
+  } catch (const std::bad_alloc&) {
+    rc = rc == PX_OK ? PX_E_OOM : rc;
+    next = std::min(next, forming);
+  } catch (...) {
+    rc = rc == PX_OK ? PX_E_CUDA : rc;
+    next = std::min(next, forming);
   }
+  while (!flight.empty()) finish_oldest();
   stop.store(true);
-  producer.join();
+  if (producer.joinable()) producer.join();
   cudaStreamSynchronize(s_apply);
   if (rc != PX_OK) {
     pipeline_clear(w, twin, s_eval);  // (a failed step's ops are not the next build's)
