@@ -100,8 +100,8 @@ namespace px {
 #define PX_VAFF_MINB 3
 #endif
 
-// kernel launches issued by the host wrappers (reported per build)
-static unsigned long long g_launches = 0;
+// kernel launches issued by the host wrappers (reported per build, which one thread enqueues)
+static thread_local unsigned long long g_launches = 0;
 unsigned long long launch_count() { return g_launches; }
 
 // Programmatic dependent launch: the kernels of a build are launched so that
