@@ -997,29 +997,10 @@ __device__ __forceinline__ int lip_decide(const OpDev* O, Iv dc, int ox, int oy,
   return dc.lo > t ? 0 : (dc.hi < -t ? 1 : 3);
 }
 
-// A voxel the float32 points left undecided ([lo, hi]: its enclosure): float32 intervals,
-// which follow this voxel's magnitudes instead of the op's largest, then float64.  Returns
-// the decision.  Out of line: a few voxels in a build.
-__device__ __noinline__ int rescue_voxel(const FoldArgs& a, const OpDev* R, int bx, int by, int bz, int lx, int ly, int lz,
-                                         Iv dk, LaneStats& ls) {
-  Iv bo[3];
-  brick_bases(a, R, bx, by, bz, bo);
-  bool amb = false;
-  const Iv d = sdf32i(a.code + R->code_off, a.code32 + R->code_off, (int)R->code_len, reinterpret_cast<const Iv*>(a.p32),
-                      iadd(bo[0], koff((float)lx, a.vs_lo, a.vs_hi)), iadd(bo[1], koff((float)ly, a.vs_lo, a.vs_hi)),
-                      iadd(bo[2], koff((float)lz, a.vs_lo, a.vs_hi)), R->thr[T_M], amb);
-  if (!amb && d.lo > R->thr[T_V_HI]) return 0;
-  if (!amb && d.hi <= R->thr[T_V_LO]) return 1;
-  const VoxelF64 f = voxel_f64(a.params, a.vs, 0, a.code + R->code_off, (int)R->code_len, dk, false, 3,
-                               (float)(bx * 8 + lx) + 0.5f, (float)(by * 8 + ly) + 0.5f, (float)(bz * 8 + lz) + 0.5f);
-  ls.rescue(0, amb, f.err);
-  return f.inside;
-}
-
 // Voxel inside-masks of the queued partial sub-blocks: one sub-block per warp
 // pass, 64 voxel SDFs on 32 lanes, two ballots (shapes.ts:390-394), any
-// program (the bytecode interpreters, lean programs' points first); a voxel its
-// float32 interval cannot decide is evaluated in float64 in line.  Groups G0 .. G1 of the voxel queue, one
+// program (the bytecode interpreters); a voxel its float32 interval cannot
+// decide is evaluated in float64 in line.  Groups G0 .. G1 of the voxel queue, one
 // after the other (the mixed form sends the lean programs' groups to
 // voxel_lean_kernel and this kernel the rest; the float64 form every group here).
 template <int MODE, int G0, int G1>
@@ -1030,6 +1011,7 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_VOXEL_MINB : PX_CLASSIFY64
   LaneStats ls = {a.res};
 #pragma unroll 1
   for (int g = G0; g <= G1; g++) {
+  if (G0 != G1 && !((a.vq_nonempty >> g) & 1u)) continue;
   uint32_t* const taken = &a.vitem_counter[VQ_TAKEN + g];
   // the group's classes' item counts in the order they are taken, as an inclusive prefix over lanes
   const int my_cls = a.vclass_order[32 * g + lane];
@@ -1054,7 +1036,7 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_VOXEL_MINB : PX_CLASSIFY64
     const OpDev* V = a.ops + (item.x & 0xffffffu);
     const int ss = (int)(item.x >> 24);
     const int vbx = (int)(item.y & 1023u), vby = (int)((item.y >> 10) & 1023u), vbz = (int)(item.y >> 20);
-    const unsigned long long vp = pair_of_brick(V, vbx, vby, vbz);
+    const uint32_t vp = pair_of_brick(V, vbx, vby, vbz);
     const bool use32 = MODE == 1 && !(V->flags & OPF_FP64_ONLY);
     Iv bo[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
     if (use32) brick_bases(a, V, vbx, vby, vbz, bo);
@@ -1062,35 +1044,7 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_VOXEL_MINB : PX_CLASSIFY64
     const uint2* code = a.code + V->code_off;
     const int clen = (int)V->code_len;
     unsigned long long m;
-    if (MODE == 1 && V->lw[0] && !a.validate) {
-      // a lean program whose float32 points leave more voxels undecided than the rescue list
-      // should hold (LEAN_BOUND .. POINT_BOUND): its points first, the rest in intervals and
-      // float64 here.  Voxel pass of a box of 60 m and a capsule of 30 at 160 voxels per metre:
-      // the interpreter for every voxel 148 and 198 us
-      const int lx = lane & 3, lyv = (lane >> 2) & 3, lz = lane >> 4;  // and lz + 2
-      const int x = sxo + lx, y = syo + lyv, z = szo + lz;
-      const float zp[2] = {coord_f(bo[2].lo, (float)z, a.vs_lo), coord_f(bo[2].lo, (float)(z + 2), a.vs_lo)};
-      float lo[2], hi[2];
-      lean_f<2, 3, true, true>(a, V, coord_f(bo[0].lo, (float)x, a.vs_lo), coord_f(bo[1].lo, (float)y, a.vs_lo), zp, lo, hi);
-      uint32_t bal[2], open = 0, late = 0;  // open: bit q, this lane's voxel q is undecided
-#pragma unroll
-      for (int q = 0; q < 2; q++) {
-        const int lip = lip_decide(V, dcen, lx, lyv, lz + 2 * q);
-        const int inside = lip != 3 ? lip : lo[q] > 0.f ? 0 : hi[q] < 0.f ? 1 : 3;
-        bal[q] = __ballot_sync(FULLMASK, inside == 1);
-        open |= (uint32_t)(inside == 3) << q;
-      }
-      while (__any_sync(FULLMASK, open)) {  // seldom more than once: few are undecided, and few lanes hold two
-        const int q = open & 1u ? 0 : 1;
-        if (open && rescue_voxel(a, V, vbx, vby, vbz, x, y, z + 2 * q, q ? Iv{lo[1], hi[1]} : Iv{lo[0], hi[0]}, ls) == 1)
-          late |= 1u << q;
-        open &= open - 1;
-        __syncwarp();
-      }
-      bal[0] |= __ballot_sync(FULLMASK, late & 1u);
-      bal[1] |= __ballot_sync(FULLMASK, late & 2u);
-      m = (unsigned long long)bal[0] | ((unsigned long long)bal[1] << 32);
-    } else if (MODE == 1 && use32 && (V->flags & OPF_Y_SEPARABLE)) {
+    if (MODE == 1 && use32 && (V->flags & OPF_Y_SEPARABLE)) {
       // lane = column (x, z) of the sub-block and a pair of y rows: one pass, the x/z work once
       const int col = lane & 15, yh = lane >> 4;
       const int lx = sxo + (col & 3), lz = szo + (col >> 2), ly0 = syo + 2 * yh;
@@ -1176,9 +1130,28 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_VOXEL_MINB : PX_CLASSIFY64
     // a lone box's sub-block is queued only in validation mode: check its runs
     if ((V->flags & OPF_BOX_RANGES) && lane == 0 && box_mask(V, vbx * 8 + sxo, vby * 8 + syo, vbz * 8 + szo) != m)
       ls.viol();
-    if (lane == 0) a.pmask[vp * 8 + ss] = m;
+    if (lane == 0) a.pmask[(size_t)vp * 8 + ss] = m;
   }
   }
+}
+
+// A voxel the float32 points left undecided ([lo, hi]: its enclosure): float32 intervals,
+// which follow this voxel's magnitudes instead of the op's largest, then float64.  Returns
+// the decision.  Out of line: a few voxels in a build.
+__device__ __noinline__ int rescue_voxel(const FoldArgs& a, const OpDev* R, int bx, int by, int bz, int lx, int ly, int lz,
+                                         Iv dk, LaneStats& ls) {
+  Iv bo[3];
+  brick_bases(a, R, bx, by, bz, bo);
+  bool amb = false;
+  const Iv d = sdf32i(a.code + R->code_off, a.code32 + R->code_off, (int)R->code_len, reinterpret_cast<const Iv*>(a.p32),
+                      iadd(bo[0], koff((float)lx, a.vs_lo, a.vs_hi)), iadd(bo[1], koff((float)ly, a.vs_lo, a.vs_hi)),
+                      iadd(bo[2], koff((float)lz, a.vs_lo, a.vs_hi)), R->thr[T_M], amb);
+  if (!amb && d.lo > R->thr[T_V_HI]) return 0;
+  if (!amb && d.hi <= R->thr[T_V_LO]) return 1;
+  const VoxelF64 f = voxel_f64(a.params, a.vs, 0, a.code + R->code_off, (int)R->code_len, dk, false, 3,
+                               (float)(bx * 8 + lx) + 0.5f, (float)(by * 8 + ly) + 0.5f, (float)(bz * 8 + lz) + 0.5f);
+  ls.rescue(0, amb, f.err);
+  return f.inside;
 }
 
 // Voxel inside-masks of the queued partial sub-blocks of the lean programs --
@@ -1194,9 +1167,11 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_VOXEL_MINB : PX_CLASSIFY64
 // (no call in this kernel: every value live across one would be saved to local
 // memory).
 // G: the group of the voxel queue (VQ_NARROW, VQ_AFFINE or VQ_WIDE), each
-// compiled with only its forms' live values.
+// compiled with only its forms' live values.  VQ_POINT: programs whose points leave more voxels
+// undecided than the rescue list should hold (LEAN_BOUND .. POINT_BOUND); these are evaluated
+// in intervals and float64 in line.
 template <bool VALIDATE, int G>
-__global__ void __launch_bounds__(256, G == VQ_WIDE ? PX_VWIDE_MINB : G == VQ_AFFINE ? PX_VAFF_MINB : PX_VSIMPLE_MINB)
+__global__ void __launch_bounds__(256, G >= VQ_WIDE ? PX_VWIDE_MINB : G == VQ_AFFINE ? PX_VAFF_MINB : PX_VSIMPLE_MINB)
     voxel_lean_kernel(FoldArgs a) {
   pdl_prologue();
   const int lane = threadIdx.x & 31;
@@ -1248,7 +1223,7 @@ __global__ void __launch_bounds__(256, G == VQ_WIDE ? PX_VWIDE_MINB : G == VQ_AF
       const int x = (ss & 1) * 4 + lx, y = ((ss >> 1) & 1) * 4 + lyv, z = ((ss >> 2) & 1) * 4 + lz;
       const float zp[2] = {coord_f(bo[2], (float)z, a.vs_lo), coord_f(bo[2], (float)(z + 2), a.vs_lo)};
       float lo[2], hi[2];
-      lean_f<2, G == VQ_WIDE ? 3 : 1, G != VQ_AFFINE, G != VQ_NARROW>(a, V, coord_f(bo[0], (float)x, a.vs_lo),
+      lean_f<2, G >= VQ_WIDE ? 3 : 1, G != VQ_AFFINE, G != VQ_NARROW>(a, V, coord_f(bo[0], (float)x, a.vs_lo),
                                                                       coord_f(bo[1], (float)y, a.vs_lo), zp, lo, hi);
       uint32_t bal[2], resc[2];
 #pragma unroll
@@ -1269,6 +1244,18 @@ __global__ void __launch_bounds__(256, G == VQ_WIDE ? PX_VWIDE_MINB : G == VQ_AF
         bal[q] = __ballot_sync(FULLMASK, inside == 1);
         resc[q] = __ballot_sync(FULLMASK, inside == 3);  // resolved by paint_kernel; outside until then
       }
+      if constexpr (!VALIDATE && G == VQ_POINT) {  // or here
+        uint32_t open = ((resc[0] >> lane) & 1u) | (((resc[1] >> lane) & 1u) << 1), late = 0;
+        while (__any_sync(FULLMASK, open)) {  // seldom more than once: few are undecided, and few lanes hold two
+          const int q = open & 1u ? 0 : 1;
+          if (open && rescue_voxel(a, V, vbx, vby, vbz, x, y, z + 2 * q, q ? Iv{lo[1], hi[1]} : Iv{lo[0], hi[0]}, ls) == 1)
+            late |= 1u << q;
+          open &= open - 1;
+          __syncwarp();
+        }
+        bal[0] |= __ballot_sync(FULLMASK, late & 1u);
+        bal[1] |= __ballot_sync(FULLMASK, late & 2u);
+      }
       const uint32_t pair = pair_of_brick(V, vbx, vby, vbz);
       const unsigned long long m = (unsigned long long)bal[0] | ((unsigned long long)bal[1] << 32);
       // a lone box's sub-block is queued only in validation mode: check its runs
@@ -1276,7 +1263,7 @@ __global__ void __launch_bounds__(256, G == VQ_WIDE ? PX_VWIDE_MINB : G == VQ_AF
           box_mask(V, vbx * 8 + (ss & 1) * 4, vby * 8 + ((ss >> 1) & 1) * 4, vbz * 8 + ((ss >> 2) & 1) * 4) != m)
         ls.viol();
       if (lane == 0) a.pmask[(size_t)pair * 8 + ss] = m;
-      if (!VALIDATE && (resc[0] | resc[1])) {  // undecided voxels to the rescue list, one atomic per warp
+      if (!VALIDATE && G != VQ_POINT && (resc[0] | resc[1])) {  // undecided voxels to the rescue list, one atomic per warp
         uint32_t base = 0;
         if (lane == 0) base = atomicAdd(&a.res->n_rescue, (uint32_t)(__popc(resc[0]) + __popc(resc[1])));
         base = __shfl_sync(FULLMASK, base, 0);
@@ -1909,6 +1896,10 @@ void launch_fold(const FoldArgs& a, int mode, int n_sms, cudaStream_t s, int max
     if (a.vq_nonempty & (1u << VQ_WIDE)) {
       if (a.validate) launch_pdl(voxel_lean_kernel<true, VQ_WIDE>, dim3(grid(PX_VWIDE_MINB)), dim3(256), 0, s, a);
       else launch_pdl(voxel_lean_kernel<false, VQ_WIDE>, dim3(grid(PX_VWIDE_MINB)), dim3(256), 0, s, a);
+    }
+    if (a.vq_nonempty & (1u << VQ_POINT)) {
+      if (a.validate) launch_pdl(voxel_lean_kernel<true, VQ_POINT>, dim3(grid(PX_VWIDE_MINB)), dim3(256), 0, s, a);
+      else launch_pdl(voxel_lean_kernel<false, VQ_POINT>, dim3(grid(PX_VWIDE_MINB)), dim3(256), 0, s, a);
     }
     if (a.vq_nonempty & (1u << VQ_GENERIC))
       launch_pdl(voxel_kernel<1, VQ_GENERIC, VQ_GENERIC>, dim3(grid(PX_VOXEL_MINB)), dim3(256), 0, s, a);

@@ -1252,11 +1252,11 @@ int convert_ops(const px_world* w, const IrOp* iops, size_t i0, size_t i1, const
           ysep = ysep && op_is_y_separable(code[2 * ((size_t)o.code_begin + k)] & 0xffu);
         if (ysep) d.flags |= OPF_Y_SEPARABLE;
         d.vclass = (first_prim & 15u) | (ysep && !(d.flags & OPF_FP64_ONLY) ? 16u : 0u);
-        // a lean program (LP_* forms) of the lean kernels, where its float32 points decide all but
-        // a few voxels: an error bound of up to LEAN_BOUND voxels leaves at most about one in 300
-        // near the surface to the rescue list (shapes of some 50 m at 80 voxels per metre).  A
-        // second primitive may be far away, and its bound larger.  Up to POINT_BOUND voxels the
-        // points still decide most and come first, before the interpreter, in the same kernels
+        // a lean program (LP_* forms), where its float32 points decide all but a few voxels: an
+        // error bound of up to LEAN_BOUND voxels leaves at most about one in 300 near the surface
+        // to the rescue list (shapes of some 50 m at 80 voxels per metre).  A second primitive may be
+        // far away, and its bound larger.  Up to POINT_BOUND voxels the points still decide most and
+        // come before the interpreter (VQ_POINT)
         uint8_t lp[8] = {0};
         const uint32_t* oc = code + 2 * (size_t)o.code_begin;
         if (!(d.flags & (OPF_FP64_ONLY | OPF_DEEP)) && d.bx0 <= d.bx1) lean_program(oc, o.code_len, lp);
@@ -1289,11 +1289,12 @@ int convert_ops(const px_world* w, const IrOp* iops, size_t i0, size_t i1, const
         }
         // the voxel queue's group and class: one primitive under at most one rotation
         // (by primitive and rotation), the other lean forms (by first primitive and
-        // form), the interpreter's programs (by sub-block class)
+        // form), those of larger error, the interpreter's programs (by sub-block class)
         const uint32_t p1op = d.lw[1] & 15u, k1 = lp[LP_KINDS] & 15u;
         if (lp[LP_FORM] == 1 && k1 != LP_AFFINE) d.vq_class = 32u * VQ_NARROW + (p1op | (k1 ? 16u : 0u));
         else if (lp[LP_FORM] == 1) d.vq_class = 32u * VQ_AFFINE + p1op;
         else if (lp[LP_FORM]) d.vq_class = 32u * VQ_WIDE + (p1op | (lp[LP_FORM] == 3 ? 16u : 0u));
+        else if (d.lw[0]) d.vq_class = 32u * VQ_POINT + (p1op | ((d.lw[0] >> 16) & 15u ? 16u : 0u));
         else d.vq_class = 32u * VQ_GENERIC + d.vclass;
       }
       d.paint_slot = NO_SLOT;
@@ -2146,9 +2147,7 @@ static int build_enqueue_impl(px_world* w, int mode, void* stream) {
   fa.chunk_counter = (uint32_t*)w->chunk_counter.p;
   fa.vitems = (uint4*)w->vitems.p;
   fa.vitems_cap = (uint32_t)(8 * P < 0xffffffffull ? 8 * P : 0xffffffffull);
-  fa.vitem_counter = (uint32_t*)w->chunk_counter.p + 4;   // counters: [0] chunks, [1] paint taken,
-                                                          // [2] paint pushed, [4..136] voxel, [160..193] pairs,
-                                                          // [CULL_COUNTER] tile-list entries
+  fa.vitem_counter = (uint32_t*)w->chunk_counter.p + VITEM_COUNTER;   // [0]: chunks, [1]: paint taken, [2], [3]: paint pushed
   {  // per-class regions: the class's pairs (sub-block pass), 8 sub-blocks per pair (voxel pass)
     uint64_t at = 0;
     for (int k = 0; k < VCLASSES; k++) {
@@ -2164,7 +2163,7 @@ static int build_enqueue_impl(px_world* w, int mode, void* stream) {
     }
   }
   fa.pitems = (uint2*)w->pitems.p;
-  fa.pitem_counter = (uint32_t*)w->chunk_counter.p + 160;
+  fa.pitem_counter = (uint32_t*)w->chunk_counter.p + PITEM_COUNTER;
   fa.rescue = (uint4*)w->rescue.p;
   fa.rescue_cap = w->rescue_cap;
   fa.paint_counter = (uint32_t*)w->chunk_counter.p + 1;

@@ -179,16 +179,21 @@ enum : uint8_t { PC_SKIP = 0, PC_PARTIAL = 1, PC_FULL = 2 };
 // (its first primitive, and whether it runs the y-extruded evaluation), so
 // that warps draining a queue at the same time run the same code.
 constexpr int VCLASSES = 32;
-// The voxel queue has four groups of 32 classes, each drained by its own
+// The voxel queue has five groups of 32 classes, each drained by its own
 // kernel: VQ_NARROW, lean programs of one primitive under at most one rotation
 // (by primitive and rotation), VQ_AFFINE, one primitive under a composed run of
 // rotations (by primitive), VQ_WIDE, the two-primitive lean programs (by first
-// primitive and form), and VQ_GENERIC, every other program (by sub-block class),
-// drained by the interpreter kernel.
-enum { VQ_NARROW = 0, VQ_AFFINE = 1, VQ_WIDE = 2, VQ_GENERIC = 3 };
-constexpr int VQ_CLASSES = 128;
+// primitive and form), VQ_POINT, lean programs of any form whose error bound is
+// past LEAN_BOUND (by first primitive and rotation), and VQ_GENERIC, every other
+// program (by sub-block class), drained by the interpreter kernel.
+enum { VQ_NARROW = 0, VQ_AFFINE = 1, VQ_WIDE = 2, VQ_POINT = 3, VQ_GENERIC = 4 };
+constexpr int VQ_CLASSES = 160;
 constexpr int VQ_TAKEN = 1 + VQ_CLASSES;  // vitem_counter[VQ_TAKEN + group]: items the group's kernel took
-constexpr int CULL_COUNTER = 200;         // chunk_counter[CULL_COUNTER]: tile-list entries reserved by cull_kernel
+// the words of the block of counters (FoldArgs::chunk_counter, 256 words, zeroed per build)
+// (the pair tickets start a 128-byte line of their own: sub-block pass of 512 primitives in float64 143
+// us, 148 behind the voxel classes' counters; the last: tile-list entries reserved by cull)
+constexpr int VITEM_COUNTER = 4, PITEM_COUNTER = 192, CULL_COUNTER = 228;
+static_assert(VITEM_COUNTER + VQ_TAKEN + VQ_CLASSES / 32 <= PITEM_COUNTER && PITEM_COUNTER + 1 + VCLASSES <= CULL_COUNTER, "apart");
 
 // Lean programs (lean_f, sdf32p.cuh), by form:
 //   1  [stage] prim [stage end] [offset]
@@ -199,12 +204,13 @@ constexpr int CULL_COUNTER = 200;         // chunk_counter[CULL_COUNTER]: tile-l
 // subtract step, an intersection or a union.
 enum { LP_FORM, LP_COMB, LP_P1, LP_P2, LP_S1, LP_S2, LP_KINDS, LP_OFF };  // lean_program's reading (host)
 enum : uint8_t { LP_NEGMAX = 1, LP_MAX = 2, LP_MIN = 3, LP_NONE = 0xff, LP_AFFINE = 4 };
-// Largest error bounds of a lean program's float32 points, in voxels: of a program of the lean
-// voxel kernels (first primitive, second), and of one whose points the generic voxel kernel tries
-// before the interpreter.  Shapes of 30 to 120 m at 160 voxels per metre, past the first bound,
-// whole passes without / with points: 12-sided prisms 562 / 404 and 580 / 433 us, rotated boxes 325 / 267
-// and 359 / 312, capsules 390 / 319 and 386 / 336; of 400 m a sphere 514 / 408, a cylinder 316 / 339.
-// A last bound of 1/8 keeps the 120 m prism at 595 us, one of 1 takes one of 400 m from 630 to 1,061
+// Largest error bounds of a lean program's float32 points, in voxels: of a program whose undecided
+// voxels go to the rescue list (first primitive, second), and of one whose points come first but
+// whose undecided voxels are evaluated in line (VQ_POINT).  Shapes of 30 / 120 / 400 m at 160 voxels
+// per metre, past the first bound, whole passes by the interpreter and with points: rotated boxes
+// 325 / 357 / 416 and 243 / 288 / 370 us, capsules 387 / 386 / 625 and 296 / 343 / 644, 12-sided
+// prisms 561 / 580 / 632 and 388 / 423 / 616.  A last bound of 1/8 keeps the prism of 120 m with
+// the interpreter, one of 1 takes the one of 400 m from 630 to 1,061
 constexpr double LEAN_BOUND = 1.0 / 128, LEAN_BOUND2 = 1.0 / 32, POINT_BOUND = 1.0 / 2;
 // code32 flags of the float32 path: a run of rotations (not all about y) composed
 // into an affine map on its first rotation; its other rotations and all but the

@@ -1,8 +1,8 @@
 """Lean programs of any size: which path they take, what they build, what they cost.
 
 A one- or two-primitive program takes the lean voxel kernels while the error bound of its
-float32 points is below 1/128 voxel, tries its points before the interpreter up to half a
-voxel, and the interpreter alone beyond.  The bound grows with the shape, so radii from
+float32 points is below 1/128 voxel, a kernel that evaluates the undecided voxels in line up
+to half a voxel, and the interpreter beyond.  The bound grows with the shape, so radii from
 one to thousands of metres cross both lines; every primitive, rotated, composed and
 combined, must equal the oracle on all of them.
 """
@@ -78,11 +78,12 @@ def timed(ops, dims):
 
 @pytest.mark.gpu
 def test_which_kernels_run(built_lib):
-    """The lean and the generic voxel kernel are launched where a program asks for them: a
-    small and a large shape together take one launch more than either alone."""
-    small, large = sphere((0.2, 0.2, 0.2), 0.1), sphere((0.2, 0.2 - 300.0, 0.2), 300.0)
-    n = {k: timed(s, (64, 64, 64))[0] for k, s in (("small", [small]), ("large", [large]), ("both", [small, large]))}
-    assert n["both"] == n["small"] + 1 == n["large"] + 1, n
+    """Each voxel kernel is launched where a program asks for it: small, large and very large shapes
+    together take one launch more for each further kind."""
+    small, large, vast = (sphere((0.2, 0.2 - r + 0.1, 0.2), r) for r in (0.1, 300.0, 5000.0))
+    n = {k: timed(s, (64, 64, 64))[0] for k, s in (("small", [small]), ("large", [large]), ("vast", [vast]),
+                                                   ("two", [small, large]), ("all", [vast, small, large]))}
+    assert n["small"] == n["large"] == n["vast"] == n["two"] - 1 == n["all"] - 2, n
     # ten metres at this density are still the lean kernels'
     assert timed([small, sphere((0.2, 0.2 - 10.0, 0.2), 10.0)], (64, 64, 64))[0] == n["small"]
 
