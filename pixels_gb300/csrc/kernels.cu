@@ -37,14 +37,20 @@ namespace px {
 #define FULLMASK 0xffffffffu
 
 // CTAs per SM the two build kernels are compiled for (register budget)
-// The mixed form's classify and sub-block passes, compiled for two CTAs per SM (128 registers, no
-// spills) and for three (80 registers, spills around the rare interpreter): two where a build
-// has the GPU to itself and at most this many (op, brick) pairs.  Both passes, two / three:
-// 256 edits at 160 voxels per metre (0.25 M pairs) 61 / 74 us, penthouse at 20 (0.03 M) 37 / 42,
-// at 80 (0.4 M) 79 / 82, synthetic (1.0 M) 153 / 150, penthouse at 128 (1.2 M) 178 / 167; twelve
-// scenes side by side 1,181 / 1,160 us in all
+// The mixed form's classify and sub-block passes, compiled for two CTAs per SM (128 registers; 12
+// bytes spilled in the sub-block pass) and for three (80 registers, spills around the rare
+// interpreter): two where a build has the GPU to itself and at most this many (op, brick) pairs.
+// Both passes, two / three: 256 edits at 160 voxels per metre (0.25 M pairs) 61 / 74 us, penthouse at
+// 20 (0.03 M) 37 / 42, at 80 (0.4 M) 79 / 82, synthetic (1.0 M) 153 / 150, penthouse at 128 (1.2 M)
+// 178 / 167; twelve scenes side by side 1,181 / 1,160 us in all.  A pair of a program that the
+// interpreter evaluates counts as PX_GENERIC_WEIGHT more (long, latency-bound: more warps): whole passes of
+// such scenes, 0.03 M pairs 318 / 323 and 251 / 254 us, 0.06 M 861 / 853, 0.07 M 540 / 536, 0.25 M
+// 1,860 / 1,847
 #ifndef PX_TWO_CTA_PAIRS
 #define PX_TWO_CTA_PAIRS (1u << 19)
+#endif
+#ifndef PX_GENERIC_WEIGHT
+#define PX_GENERIC_WEIGHT 10u
 #endif
 #ifndef PX_DERIVE_PER_SM
 #define PX_DERIVE_PER_SM 8
@@ -1110,8 +1116,10 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_VOXEL_MINB : PX_CLASSIFY64
       m = (unsigned long long)(in[0] | __reduce_or_sync(FULLMASK, lo)) |
           ((unsigned long long)(in[1] | __reduce_or_sync(FULLMASK, hi)) << 32);
     } else {
-      uint32_t bal[2];
-#pragma unroll
+      // one copy of the interpreter for both halves of the sub-block (bound by instruction fetch):
+      // 300 shapes of three to five primitives at 80 voxels per metre 3,779 us a pass with two, 3,212 so
+      uint32_t bal[2] = {0u, 0u};
+#pragma unroll 1
       for (int r = 0; r < 2; r++) {
         const int e = r * 32 + lane;
         const int lx = sxo + (e & 3), lyv = syo + ((e >> 2) & 3), lz = szo + (e >> 4);
@@ -1123,7 +1131,9 @@ __global__ void __launch_bounds__(256, MODE == 1 ? PX_VOXEL_MINB : PX_CLASSIFY64
                                      (float)(vbz * 8 + lz) + 0.5f, 0, ls);
           if (lipd != 3 && inside != lipd) ls.viol();  // validation: the bound disagreed with the evaluation
         }
-        bal[r] = __ballot_sync(FULLMASK, inside == 1);
+        const uint32_t in = __ballot_sync(FULLMASK, inside == 1);
+        if (r) bal[1] = in;
+        else bal[0] = in;
       }
       m = (unsigned long long)bal[0] | ((unsigned long long)bal[1] << 32);
     }
@@ -1874,11 +1884,11 @@ __global__ void __launch_bounds__(256, PX_FOLD_MINB) fold_kernel(FoldArgs a) {
   }
 }
 
-void launch_fold(const FoldArgs& a, int mode, int n_sms, cudaStream_t s, int max_blocks,
+void launch_fold(const FoldArgs& a, int mode, unsigned long long n_generic, int n_sms, cudaStream_t s, int max_blocks,
                  cudaStream_t s_apply, cudaEvent_t eval_done) {
   auto grid = [&](int per_sm) { return max_blocks > 0 && max_blocks < n_sms * per_sm ? max_blocks : n_sms * per_sm; };
   if (mode == 1) {
-    if (max_blocks <= 0 && a.n_pairs <= PX_TWO_CTA_PAIRS) {
+    if (max_blocks <= 0 && a.n_pairs + PX_GENERIC_WEIGHT * n_generic <= PX_TWO_CTA_PAIRS) {
       launch_pdl(classify_kernel<1, 2>, dim3(grid(2)), dim3(256), 0, s, a);
       launch_pdl(sub_kernel<1, 2>, dim3(grid(2)), dim3(256), 0, s, a);
     } else {

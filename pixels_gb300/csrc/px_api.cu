@@ -2207,7 +2207,9 @@ static int build_enqueue_impl(px_world* w, int mode, void* stream) {
   fa.res = res;
   int max_blocks = 0;  // persistent grids sized to the build (batched builds share the GPU)
   if (w->pairs_per_block) max_blocks = (int)std::max<uint64_t>(1, (P + w->pairs_per_block - 1) / w->pairs_per_block);
-  launch_fold(fa, mode, w->n_sms, s, max_blocks, sa, w->ev_eval);
+  uint64_t n_generic = 0;
+  for (int k = 32 * VQ_GENERIC; k < 32 * VQ_GENERIC + 32; k++) n_generic += vper[k];
+  launch_fold(fa, mode, n_generic, w->n_sms, s, max_blocks, sa, w->ev_eval);
   s = sa;  // the rest of the build follows the apply pass
 
   ReplayArgs ra{};

@@ -311,7 +311,8 @@ void launch_cull(const uint2* boxes, int n_ops, int TX, int TY, int TZ, uint32_t
 // max_blocks > 0 caps the persistent grids (builds sharing the GPU)
 // The evaluation passes (classify .. paint) go on s; the apply pass on s_apply,
 // after eval_done is recorded on s (s_apply == s: one stream, no event).
-void launch_fold(const FoldArgs& a, int mode, int n_sms, cudaStream_t s, int max_blocks,
+// n_generic: the (op, brick) pairs of the programs that the interpreter evaluates (VQ_GENERIC)
+void launch_fold(const FoldArgs& a, int mode, unsigned long long n_generic, int n_sms, cudaStream_t s, int max_blocks,
                  cudaStream_t s_apply, cudaEvent_t eval_done);
 
 
