@@ -26,8 +26,9 @@
 namespace px {
 
 // sqrt(v), v >= 0, from the hardware reciprocal square root (maximum relative
-// error 2^-22.9 by the PTX manual): relative error below 2^-22.4 with the
-// product's rounding, 2^-50 absolute below 2^-100
+// error 2^-22.9 by the PTX manual): relative error below 2^-22.3 with the
+// product's rounding, 2^-50 absolute below 2^-100.  (The bounds rely on 8 * 2^-24 for
+// a length, squares and sums included: eb_len.)
 __device__ __forceinline__ float root_f(float v) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaxf(v, 0x1p-100f)));
