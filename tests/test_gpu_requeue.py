@@ -98,3 +98,35 @@ def test_requeue_after_serving_that_builds_nothing(built_lib, form, n):
         _lib.build(w._h, MODE_MIXED)
         check(w, o)
     w.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [MODE_MIXED, MODE_FP64])
+@pytest.mark.parametrize("first,second", [("scattered", "few"), ("few", "scattered"), ("rows", "rows"), ("few", "few")])
+def test_two_lists_queued_and_requeued(built_lib, first, second, mode):
+    """Two lists queued before one build: their cull table is made at the build, and requeued with
+    the tables; then a list of another form, and the two again as one."""
+    parts = [scene(first), scene(second)]
+    whole = Program()
+    for p in parts:
+        code, par = len(whole.code), len(whole.params)
+        whole.ops += [tuple(o[:5]) + (o[5] + code,) + tuple(o[6:]) for o in p.ops]
+        whole.code += [(w0, off + par) for w0, off in p.code]
+        whole.params += p.params
+    o = pyoracle.OracleWorld(whole.to_bytes(), VPM, DIMS, threads=8)
+    w = VoxelWorld(*DIMS, vpm=VPM, mode=mode)
+    for p in parts:
+        _lib.submit_ops(w._h, p.to_bytes())
+    _lib.build(w._h, mode)
+    check(w, o)
+    _lib.world_reset(w._h, True)
+    _lib.build(w._h, mode)
+    check(w, o)
+    _lib.world_reset(w._h)
+    _lib.submit_ops(w._h, scene("few").to_bytes())
+    _lib.build(w._h, mode)
+    _lib.world_reset(w._h)
+    _lib.submit_ops(w._h, whole.to_bytes())
+    _lib.build(w._h, mode)
+    check(w, o)
+    w.close()
